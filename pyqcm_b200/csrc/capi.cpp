@@ -193,6 +193,31 @@ const bool g_parallel_for_set = [] {
   return true;
 }();
 
+// The inter-cluster elements (r, c, R, v) of V(k) on the device, ordered by row
+// (the order of a row's elements kept).
+struct LatticeElements {
+  DevBuf<int> row, col;
+  DevBuf<double> R, v;
+  LatticeElements(int dim, int nel, const int *r, const int *c, const int *Rv, const double *vv, cudaStream_t s) {
+    std::vector<int> first(dim + 1, 0), hc(std::max(nel, 1), 0);
+    std::vector<double> hR(3 * hc.size(), 0.0), hv(2 * hc.size(), 0.0);
+    for (int e = 0; e < nel; ++e) ++first[r[e] + 1];
+    for (int a = 0; a < dim; ++a) first[a + 1] += first[a];
+    std::vector<int> next(first.begin(), first.end() - 1);
+    for (int e = 0; e < nel; ++e) {
+      const int k = next[r[e]]++;
+      hc[k] = c[e];
+      for (int i = 0; i < 3; ++i) hR[3 * k + i] = (double)Rv[3 * e + i];
+      hv[2 * k] = vv[2 * e];
+      hv[2 * k + 1] = vv[2 * e + 1];
+    }
+    row.upload(first, s);
+    col.upload(hc, s);
+    R.upload(hR, s);
+    v.upload(hv, s);
+  }
+};
+
 // Weighted tasks run longest-first (LPT) on the batch thread pool.
 struct Task {
   double cost;
@@ -734,23 +759,13 @@ int qed_sef_integrand_grid(int label, int spin_down, int dim, const double *V0, 
     std::vector<cplx> z(nw);
     for (int i = 0; i < nw; ++i) z[i] = cplx(0.0, w[i]);
     const size_t nn = (size_t)dim * dim;
-    DevBuf<double> dG(2 * nn * nw), dV0(2 * nn), dR(3 * (size_t)std::max(nel, 1)), dv(2 * (size_t)std::max(nel, 1));
-    DevBuf<int> dr(std::max(nel, 1)), dc(std::max(nel, 1));
+    const long nk = (long)nkx * nky * nkz;
+    const int nblk = lattice_blocks(dim, nw, nk);
+    DevBuf<double> dG(2 * nn * nw), dV0(2 * nn), part((size_t)nblk * nw);
     I->green_function_device(z.data(), nw, spin_down != 0, dG.p, W);
     dV0.upload(V0, 2 * nn, W.stream);
-    if (nel) {
-      std::vector<double> Rd(3 * (size_t)nel);
-      for (size_t i = 0; i < Rd.size(); ++i) Rd[i] = (double)R[i];
-      dR.upload(Rd, W.stream);
-      dv.upload(v, 2 * (size_t)nel, W.stream);
-      dr.upload(r, nel, W.stream);
-      dc.upload(c, nel, W.stream);
-    }
-    const long nk = (long)nkx * nky * nkz;
-    const int nblk = (int)((nk + 127) / 128);
-    DevBuf<double> part((size_t)nblk * nw);
-    const int nb = launch_sef_logdet(dim, nw, dG.p, dV0.p, nel, dr.p, dc.p, dR.p, dv.p, nkx, nky, nkz, part.p, W.stream);
-    if (nb != nblk) fail(QED_ERR_INTERNAL, "qed_sef_integrand_grid: block count mismatch");
+    const LatticeElements el(dim, nel, r, c, R, v, W.stream);
+    launch_sef_logdet(dim, nw, dG.p, dV0.p, el.row.p, el.col.p, el.R.p, el.v.p, nkx, nky, nkz, part.p, W.stream);
     std::vector<double> h((size_t)nblk * nw);
     part.download(h.data(), h.size(), W.stream);
     W.sync();
@@ -780,21 +795,13 @@ int qed_cpt_projected_green_function(int label, int spin_down, int dim, const do
     std::vector<cplx> z(nw);
     for (int i = 0; i < nw; ++i) z[i] = cplx(0.0, w[i]);
     const size_t nn = (size_t)dim * dim;
-    DevBuf<double> dG(2 * nn * nw), dV0(2 * nn * nw), dR(3 * (size_t)std::max(nel, 1)),
-        dv(2 * (size_t)std::max(nel, 1)), part((size_t)cpt_partials_size(dim, nw)), dP(2 * nn * nw);
-    DevBuf<int> dr(std::max(nel, 1)), dc(std::max(nel, 1));
+    const int nblk = lattice_blocks(dim, std::min(nw, 65535), (long)nkx * nky * nkz);
+    DevBuf<double> dG(2 * nn * nw), dV0(2 * nn * nw), part(2 * nn * nw * nblk), dP(2 * nn * nw);
     I->green_function_device(z.data(), nw, spin_down != 0, dG.p, W);
     dV0.upload(V0, 2 * nn * nw, W.stream);
-    if (nel) {
-      std::vector<double> Rd(3 * (size_t)nel);
-      for (size_t i = 0; i < Rd.size(); ++i) Rd[i] = (double)R[i];
-      dR.upload(Rd, W.stream);
-      dv.upload(v, 2 * (size_t)nel, W.stream);
-      dr.upload(r, nel, W.stream);
-      dc.upload(c, nel, W.stream);
-    }
-    launch_cpt_projected(dim, nw, dG.p, dV0.p, nel, dr.p, dc.p, dR.p, dv.p, nkx, nky, nkz, offset, part.p, dP.p,
-                         W.stream);
+    const LatticeElements el(dim, nel, r, c, R, v, W.stream);
+    launch_cpt_projected(dim, nw, dG.p, dV0.p, el.row.p, el.col.p, el.R.p, el.v.p, nkx, nky, nkz, offset, part.p,
+                         dP.p, W.stream);
     dP.download(Gproj, 2 * nn * nw, W.stream);
     W.sync();
   });

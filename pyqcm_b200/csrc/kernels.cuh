@@ -161,19 +161,27 @@ void launch_block_hv(const HvOperator &op, int p, const BlockIn &X, const BlockO
 
 // out[0..n) = fixed-order sums of partials with row stride ld
 void launch_finalize_ld(const double *partials, int nblocks, int ld, int n, double *out, cudaStream_t s);
-// log |det(V(k) G(iw) - 1)| on the (w, k) grid, V(k) = V0 + sum_e v_e exp(2 pi i k.R_e)
-// at (r_e, c_e); G: nw column-major n x n complex matrices. Writes, per w, the
-// per-CTA sums partials[w * nblk + b] and returns nblk (n <= 16).
-int launch_sef_logdet(int n, int nw, const double *G, const double *V0, int nel, const int *er, const int *ec,
-                      const double *eR, const double *ev, int nkx, int nky, int nkz, double *partials,
-                      cudaStream_t s);
-// Grid average of G (1 - V(k) G)^{-1} per frequency into Gproj (nw n x n
-// complex, column-major); V0 holds nw k-independent parts of V (one per
-// frequency); k = ((a + off)/nkx, ...). partials: cpt_partials_size(n, nw) doubles.
-void launch_cpt_projected(int n, int nw, const double *G, const double *V0, int nel, const int *er, const int *ec,
+// Lattice sums (lattice.cu). V(k) = V0 + sum_e v_e exp(2 pi i k.R_e) at (r_e, c_e),
+// the elements ordered by row: row[r] .. row[r + 1] are those of row r. G: nw
+// column-major n x n complex matrices, n <= 16.
+// CTAs per frequency, for the sizes of the partial sums below
+int lattice_blocks(int n, int nw, long nk);
+// Integrand of the self-energy functional (lattice_model_instance::SEF_integrand_k,
+// src_qcm/lattice_model_instance.cpp:618-640, summed as in Potthoff_functional's
+// grid path, :520-545) at k = (i/nkx, j/nky, l/nkz): per w, the per-CTA sums of
+// log |det(V(k) G(iw) - 1)| at partials[w * lattice_blocks + b].
+void launch_sef_logdet(int n, int nw, const double *G, const double *V0, const int *row, const int *col,
+                       const double *eR, const double *ev, int nkx, int nky, int nkz, double *partials,
+                       cudaStream_t s);
+// Projected CPT Green function for the CDMFT host
+// (lattice_model_instance::projected_Green_function, src_qcm/CPT.cpp:283-346;
+// set_Gcpt, :76-86): the grid average of G (1 - V(k) G)^{-1} per frequency into
+// Gproj (nw n x n complex, column-major); V0 holds nw k-independent parts of V
+// (one per frequency); k = ((a + off)/nkx, ...). partials: 2 n^2 nw
+// lattice_blocks doubles.
+void launch_cpt_projected(int n, int nw, const double *G, const double *V0, const int *row, const int *col,
                           const double *eR, const double *ev, int nkx, int nky, int nkz, double off,
                           double *partials, double *Gproj, cudaStream_t s);
-int cpt_partials_size(int n, int nw);
 // G = R^T R on the device (p <= 16): R, R^{-1}; *fail = 1 if G is not positive
 // definite or a pivot is below pivot_min; with Rprev, B = R Rprev and B^T
 void launch_block_chol(int p, const double *G, double pivot_min, double *R, double *Rinv, const double *Rprev,
