@@ -2,6 +2,8 @@
 // Hamiltonians, and the error convention (status code + per-thread message).
 #include <algorithm>
 #include <chrono>
+#include <cmath>
+#include <complex>
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
@@ -193,29 +195,41 @@ const bool g_parallel_for_set = [] {
   return true;
 }();
 
-// The inter-cluster elements (r, c, R, v) of V(k) on the device, ordered by row
-// (the order of a row's elements kept).
+// The inter-cluster elements (r, c, R, v) of V(k) on the device as LatticeView
+// wants them: ordered by row (the order of a row's elements kept), the grid's
+// directions by size, R reduced to the grid, the phase of the grid's offset (the
+// same along every direction, in units of a grid step) in v.
 struct LatticeElements {
-  DevBuf<int> row, col;
-  DevBuf<double> R, v;
-  LatticeElements(int dim, int nel, const int *r, const int *c, const int *Rv, const double *vv, cudaStream_t s) {
-    std::vector<int> first(dim + 1, 0), hc(std::max(nel, 1), 0);
-    std::vector<double> hR(3 * hc.size(), 0.0), hv(2 * hc.size(), 0.0);
+  DevBuf<int> row;
+  DevBuf<LatticeElement> el;
+  int nk[3];
+  LatticeElements(int dim, int nel, const int *r, const int *c, const int *R, const double *vv, int nkx, int nky,
+                  int nkz, double off, cudaStream_t s) {
+    const int given[3] = {nkx, nky, nkz};
+    int dir[3] = {0, 1, 2};
+    std::stable_sort(dir, dir + 3, [&](int a, int b) { return given[a] < given[b]; });
+    for (int i = 0; i < 3; ++i) nk[i] = given[dir[i]];
+    std::vector<int> first(dim + 1, 0);
     for (int e = 0; e < nel; ++e) ++first[r[e] + 1];
     for (int a = 0; a < dim; ++a) first[a + 1] += first[a];
     std::vector<int> next(first.begin(), first.end() - 1);
+    std::vector<LatticeElement> h(std::max(nel, 1), LatticeElement{{0.0, 0.0}, {0, 0, 0, 0}});
     for (int e = 0; e < nel; ++e) {
-      const int k = next[r[e]]++;
-      hc[k] = c[e];
-      for (int i = 0; i < 3; ++i) hR[3 * k + i] = (double)Rv[3 * e + i];
-      hv[2 * k] = vv[2 * e];
-      hv[2 * k + 1] = vv[2 * e + 1];
+      int w[3];
+      double turn = 0.0;
+      for (int i = 0; i < 3; ++i) {
+        const long Ri = R[3 * e + dir[i]];
+        w[i] = (int)((Ri % nk[i] + nk[i]) % nk[i]);
+        turn += off * Ri / nk[i];
+      }
+      std::complex<double> x(vv[2 * e], vv[2 * e + 1]);
+      if (off != 0.0) x *= std::polar(1.0, 2.0 * M_PI * turn);
+      h[next[r[e]]++] = LatticeElement{{x.real(), x.imag()}, {c[e], w[0], w[1], w[2]}};
     }
     row.upload(first, s);
-    col.upload(hc, s);
-    R.upload(hR, s);
-    v.upload(hv, s);
+    el.upload(h, s);
   }
+  LatticeView view() const { return {row.p, el.p}; }
 };
 
 // Weighted tasks run longest-first (LPT) on the batch thread pool.
@@ -764,8 +778,8 @@ int qed_sef_integrand_grid(int label, int spin_down, int dim, const double *V0, 
     DevBuf<double> dG(2 * nn * nw), dV0(2 * nn), part((size_t)nblk * nw);
     I->green_function_device(z.data(), nw, spin_down != 0, dG.p, W);
     dV0.upload(V0, 2 * nn, W.stream);
-    const LatticeElements el(dim, nel, r, c, R, v, W.stream);
-    launch_sef_logdet(dim, nw, dG.p, dV0.p, el.row.p, el.col.p, el.R.p, el.v.p, nkx, nky, nkz, part.p, W.stream);
+    const LatticeElements el(dim, nel, r, c, R, v, nkx, nky, nkz, 0.0, W.stream);
+    launch_sef_logdet(dim, nw, dG.p, dV0.p, el.view(), el.nk, part.p, W.stream);
     std::vector<double> h((size_t)nblk * nw);
     part.download(h.data(), h.size(), W.stream);
     W.sync();
@@ -799,9 +813,8 @@ int qed_cpt_projected_green_function(int label, int spin_down, int dim, const do
     DevBuf<double> dG(2 * nn * nw), dV0(2 * nn * nw), part(2 * nn * nw * nblk), dP(2 * nn * nw);
     I->green_function_device(z.data(), nw, spin_down != 0, dG.p, W);
     dV0.upload(V0, 2 * nn * nw, W.stream);
-    const LatticeElements el(dim, nel, r, c, R, v, W.stream);
-    launch_cpt_projected(dim, nw, dG.p, dV0.p, el.row.p, el.col.p, el.R.p, el.v.p, nkx, nky, nkz, offset, part.p,
-                         dP.p, W.stream);
+    const LatticeElements el(dim, nel, r, c, R, v, nkx, nky, nkz, offset, W.stream);
+    launch_cpt_projected(dim, nw, dG.p, dV0.p, el.view(), el.nk, part.p, dP.p, W.stream);
     dP.download(Gproj, 2 * nn * nw, W.stream);
     W.sync();
   });

@@ -161,27 +161,34 @@ void launch_block_hv(const HvOperator &op, int p, const BlockIn &X, const BlockO
 
 // out[0..n) = fixed-order sums of partials with row stride ld
 void launch_finalize_ld(const double *partials, int nblocks, int ld, int n, double *out, cudaStream_t s);
-// Lattice sums (lattice.cu). V(k) = V0 + sum_e v_e exp(2 pi i k.R_e) at (r_e, c_e),
-// the elements ordered by row: row[r] .. row[r + 1] are those of row r. G: nw
-// column-major n x n complex matrices, n <= 16.
+// Lattice sums (lattice.cu). V(k) = V0 + sum_e v_e exp(2 pi i k.R_e) at (r_e, c_e)
+// on the grid k = (i/nk0, j/nk1, l/nk2); an offset of the grid is a factor
+// exp(2 pi i off.R_e) in v_e. The directions may come in any order (the largest
+// last is fastest). The elements (device arrays) are ordered by row: row[r] ..
+// row[r + 1] are those of row r. G: nw column-major n x n complex matrices,
+// n <= 16.
+struct alignas(16) LatticeElement {
+  double2 v;
+  int4 where;  // column, then R reduced to [0, nk) of each direction
+};
+struct LatticeView {
+  const int *row;
+  const LatticeElement *el;
+};
 // CTAs per frequency, for the sizes of the partial sums below
 int lattice_blocks(int n, int nw, long nk);
 // Integrand of the self-energy functional (lattice_model_instance::SEF_integrand_k,
 // src_qcm/lattice_model_instance.cpp:618-640, summed as in Potthoff_functional's
-// grid path, :520-545) at k = (i/nkx, j/nky, l/nkz): per w, the per-CTA sums of
+// grid path, :520-545): per w, the per-CTA sums of
 // log |det(V(k) G(iw) - 1)| at partials[w * lattice_blocks + b].
-void launch_sef_logdet(int n, int nw, const double *G, const double *V0, const int *row, const int *col,
-                       const double *eR, const double *ev, int nkx, int nky, int nkz, double *partials,
+void launch_sef_logdet(int n, int nw, const double *G, const double *V0, const LatticeView &el, const int (&nk3)[3], double *partials,
                        cudaStream_t s);
 // Projected CPT Green function for the CDMFT host
 // (lattice_model_instance::projected_Green_function, src_qcm/CPT.cpp:283-346;
 // set_Gcpt, :76-86): the grid average of G (1 - V(k) G)^{-1} per frequency into
 // Gproj (nw n x n complex, column-major); V0 holds nw k-independent parts of V
-// (one per frequency); k = ((a + off)/nkx, ...). partials: 2 n^2 nw
-// lattice_blocks doubles.
-void launch_cpt_projected(int n, int nw, const double *G, const double *V0, const int *row, const int *col,
-                          const double *eR, const double *ev, int nkx, int nky, int nkz, double off,
-                          double *partials, double *Gproj, cudaStream_t s);
+// (one per frequency). partials: 2 n^2 nw lattice_blocks doubles.
+void launch_cpt_projected(int n, int nw, const double *G, const double *V0, const LatticeView &el, const int (&nk3)[3], double *partials, double *Gproj, cudaStream_t s);
 // G = R^T R on the device (p <= 16): R, R^{-1}; *fail = 1 if G is not positive
 // definite or a pivot is below pivot_min; with Rprev, B = R Rprev and B^T
 void launch_block_chol(int p, const double *G, double pivot_min, double *R, double *Rinv, const double *Rprev,

@@ -12,15 +12,19 @@
 // N multiplications per element instead of the N^3 of the whole product (the
 // elements couple neighbouring super cells: two or three per boundary site).
 // Gaussian elimination with partial pivoting then needs no row exchanges: the
-// pivot lane is the largest |re| + |im| among the lanes not used yet (one
-// redux.sync over the matrix's lanes) and its row goes round by shuffles.
+// pivot lane is the largest |re| + |im| among the lanes not used yet (a
+// maximum passed round the matrix's lanes) and its row goes round by shuffles.
 //
-// What bounds it: the FP64 pipe (elimination, divisions, phases) and the
-// shuffles (4 per broadcast complex entry, one warp instruction per cycle and
-// SM). On a B200, 64 x 4096 matrices of dimension 10: 293 us, and 1537 us with
-// one thread per matrix holding V, V G and the factors in local memory; the
-// averages of 64 x 1024 matrices of dimension 4: 17 us, and 354 us in 64 CTAs of
-// 64 threads.
+// What bounds it: the shuffles (4 per broadcast complex entry; the pipe they
+// share with shared memory is busy 53 % of the time) and the latency of the
+// elimination's serial chain (22 warps per SM, two instructions per cycle).
+// On a B200, 64 x 4096 matrices of dimension 10: 216 us, and 1537 us with one
+// thread per matrix holding V, V G and the factors in local memory; the averages
+// of 64 x 1024 matrices of dimension 4: 17 us, and 354 us in 64 CTAs of 64
+// threads. On the way: a sincospi per element and wavevector, divisions and a
+// redux.sync per elimination step 293 us; the phase table and fewer registers
+// 272 us; Newton-Raphson reciprocals and fused multiply-adds 254 us; the pivot
+// search by shuffles 216 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,24 +40,69 @@ namespace {
 constexpr int kLatThreads = 128;
 constexpr int kLatWarps = kLatThreads / 32;
 constexpr int kLatMaxN = 16;
+constexpr int lattice_ctas(int n) { return n <= 6 ? 8 : (n <= 10 ? 6 : (n <= 13 ? 5 : 4)); }
+
+// Grids of at most this many points along the three directions together keep
+// exp(2 pi i j / nk) of every direction in shared memory (6 KB): a phase is then
+// two or three products instead of a sincospi (about as many FP64 instructions
+// as one row of dimension 10). Larger grids evaluate sincospi.
+constexpr int kPhaseTable = 384;
 
 struct LatticeTerms {
-  const int *row;    // elements of matrix row r: row[r] .. row[r + 1]
-  const int *col;
-  const double *R;   // 3 per element
-  const double *v;   // complex
-  int nkx, nky, nkz;
-  double off;        // grid point i sits at (i + off) / nk
+  const int *row;               // elements of matrix row r: row[r] .. row[r + 1]
+  const LatticeElement *el;
+  int nk0, nk1, nk2;            // grid, the largest direction last
+  unsigned magic0, magic1, magic2;  // ceil(2^32 / nk): j mod nk by a multiplication, for j < nk^2
+  bool table;
 };
 
 struct Cplx {
   double x, y;
 };
 
-__device__ __forceinline__ Cplx cmul(Cplx a, Cplx b) { return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; }
+__device__ __forceinline__ Cplx cmul(Cplx a, Cplx b) {
+  return {fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x)};
+}
+// a -= l q
+__device__ __forceinline__ void csub(Cplx &a, Cplx l, Cplx q) {
+  a.x = fma(-l.x, q.x, fma(l.y, q.y, a.x));
+  a.y = fma(-l.x, q.y, fma(-l.y, q.x, a.y));
+}
+// 1 / d for d > 0 to about an ulp: the hardware's approximation (rcp.approx, at
+// least 20 bits) and two Newton-Raphson steps r += r (1 - d r), each doubling
+// the number of correct bits. A division instead costs a call with its checks
+// per elimination step. Zero, infinite and subnormal d take the division.
+__device__ __forceinline__ double reciprocal(double d) {
+  if (!(d > 1e-290 && d < 1e290)) return 1.0 / d;
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  r = fma(r, fma(-d, r, 1.0), r);
+  return fma(r, fma(-d, r, 1.0), r);
+}
 __device__ __forceinline__ Cplx shfl(Cplx a, int src) {
   return {__shfl_sync(0xffffffffu, a.x, src), __shfl_sync(0xffffffffu, a.y, src)};
 }
+
+// A point of the grid, advanced along its last direction.
+struct GridPoint {
+  unsigned i0, i1, i2;
+  __device__ GridPoint(const LatticeTerms &t, unsigned long long kid) {
+    const unsigned long long q = kid / (unsigned)t.nk2;
+    i2 = (unsigned)(kid - q * (unsigned)t.nk2);
+    i0 = (unsigned)(q / (unsigned)t.nk1);
+    i1 = (unsigned)(q - (unsigned long long)i0 * (unsigned)t.nk1);
+  }
+  __device__ __forceinline__ void advance(const LatticeTerms &t, unsigned n) {
+    i2 += n;
+    while (i2 >= (unsigned)t.nk2) {  // past the grid's end it starts over: those points are not used
+      i2 -= t.nk2;
+      if (++i1 == (unsigned)t.nk1) {
+        i1 = 0;
+        if (++i0 == (unsigned)t.nk0) i0 = 0;
+      }
+    }
+  }
+};
 
 // G of one frequency and +-(V0 G - 1) in shared memory, rows padded to N + 1
 // entries so that lanes reading different rows hit different banks.
@@ -80,86 +129,118 @@ template <int N> struct LatticeTile {
     __syncthreads();
   }
 
-  // row r of +-(V(k) G - 1)
-  __device__ __forceinline__ void row(const LatticeTerms &t, unsigned long long kid, int r, double sign,
-                                      Cplx (&a)[N]) const {
-    unsigned ix, iy, iz;
-    const unsigned nz = (unsigned)t.nkz, ny = (unsigned)t.nky;
-    if (kid <= 0xffffffffull) {  // 32-bit divisions unless the grid is larger
-      const unsigned k = (unsigned)kid, q = k / nz;
-      iz = k - q * nz;
-      ix = q / ny;
-      iy = q - ix * ny;
-    } else {
-      const unsigned long long q = kid / nz;
-      iz = (unsigned)(kid - q * nz);
-      ix = (unsigned)(q / ny);
-      iy = (unsigned)(q - (unsigned long long)ix * ny);
-    }
-    const double kx = (ix + t.off) / t.nkx, ky = (iy + t.off) / t.nky, kz = (iz + t.off) / t.nkz;
+  // row r of +-(V(k) G - 1) at grid point (i0, i1, i2); ph: the phase table, or unused
+  __device__ __forceinline__ void row(const LatticeTerms &t, const double2 *ph, const GridPoint &k, int e, int e1,
+                                      int r, double sign, Cplx (&a)[N]) const {
 #pragma unroll
     for (int b = 0; b < N; ++b) {
       const double2 v = w[r * kLd + b];
       a[b] = {v.x, v.y};
     }
-    const int e1 = __ldg(t.row + r + 1);
-    for (int e = __ldg(t.row + r); e < e1; ++e) {
-      double s, c;
-      sincospi(2.0 * (kx * __ldg(t.R + 3 * e) + ky * __ldg(t.R + 3 * e + 1) + kz * __ldg(t.R + 3 * e + 2)), &s, &c);
-      const double vr = sign * __ldg(t.v + 2 * e), vi = sign * __ldg(t.v + 2 * e + 1);
-      const Cplx p = {vr * c - vi * s, vr * s + vi * c};
-      const double2 *gr = g + __ldg(t.col + e) * kLd;
+    for (; e < e1; ++e) {
+      const double2 v = __ldg(&t.el[e].v);
+      const int4 m = __ldg(&t.el[e].where);  // column, R
+      Cplx p = {sign * v.x, sign * v.y};
+      if (t.table) {
+        auto turn = [&](unsigned j, int nk, unsigned magic, const double2 *tab) {
+          const double2 f = tab[j - (unsigned)nk * __umulhi(j, magic)];
+          p = cmul(p, Cplx{f.x, f.y});
+        };
+        if (t.nk0 > 1) turn(k.i0 * (unsigned)m.y, t.nk0, t.magic0, ph);
+        if (t.nk1 > 1) turn(k.i1 * (unsigned)m.z, t.nk1, t.magic1, ph + t.nk0);
+        turn(k.i2 * (unsigned)m.w, t.nk2, t.magic2, ph + t.nk0 + t.nk1);
+      } else {
+        auto part = [](unsigned i, int R, int nk) {
+          return (double)((unsigned long long)i * (unsigned)R % (unsigned)nk) / nk;
+        };
+        double s, c;
+        sincospi(2.0 * (part(k.i0, m.y, t.nk0) + part(k.i1, m.z, t.nk1) + part(k.i2, m.w, t.nk2)), &s, &c);
+        p = cmul(p, Cplx{c, s});
+      }
+      const double2 *gr = g + m.x * kLd;
+      p = {-p.x, -p.y};
 #pragma unroll
       for (int b = 0; b < N; ++b) {
         const double2 y = gr[b];
-        a[b].x += p.x * y.x - p.y * y.y;
-        a[b].y += p.x * y.y + p.y * y.x;
+        csub(a[b], p, Cplx{y.x, y.y});
       }
     }
   }
 };
 
-// The pivot lane (within the matrix's lanes `mask`) of one elimination step:
-// the largest |re| + |im| among the lanes with `open` set. The key is the high
-// word of that double (monotonic for values >= 0) with the lane in the last
-// four bits, so pivots equal to 1 part in 2^16 are told apart by lane only.
-__device__ __forceinline__ int pivot_lane(unsigned mask, bool open, Cplx v, int r) {
-  const unsigned hi = (unsigned)__double2hiint(fabs(v.x) + fabs(v.y));
-  return (int)(__reduce_max_sync(mask, open ? (0x80000000u | (hi & ~15u) | (unsigned)r) : 0u) & 15u);
+// The CTA's phase table (visible after the next barrier).
+__device__ __forceinline__ void fill_phases(const LatticeTerms &t, double2 *ph) {
+  if (!t.table) return;
+  for (int i = threadIdx.x; i < t.nk0 + t.nk1 + t.nk2; i += blockDim.x) {
+    const int j1 = i - t.nk0, j2 = j1 - t.nk1;
+    const double turn = j1 < 0 ? (double)i / t.nk0 : (j2 < 0 ? (double)j1 / t.nk1 : (double)j2 / t.nk2);
+    double s, c;
+    sincospi(2.0 * turn, &s, &c);
+    ph[i] = make_double2(c, s);
+  }
 }
+
+// The pivot lane of one elimination step among a matrix's N lanes: the largest
+// |re| + |im| among those with `open` set. The key is the high word of that
+// double (monotonic for values >= 0) with the lane in the last four bits, so
+// pivots equal to 1 part in 2^16 are told apart by lane only. The maximum goes
+// round the lanes in steps of 1, 2, 4, ... (a maximum may count a lane twice, so
+// N need not be a power of two); redux.sync with a mask per matrix took longer.
+template <int N> struct PivotRing {
+  static constexpr int kRounds = N > 8 ? 4 : (N > 4 ? 3 : (N > 2 ? 2 : N - 1));
+  int from[kRounds > 0 ? kRounds : 1];
+  __device__ PivotRing(int base, int r) {
+#pragma unroll
+    for (int o = 0; o < kRounds; ++o) from[o] = base + (r + (1 << o)) % N;
+  }
+  __device__ __forceinline__ int lane(bool open, Cplx v, int r) const {
+    const unsigned hi = (unsigned)__double2hiint(fabs(v.x) + fabs(v.y));
+    unsigned key = open ? (0x80000000u | (hi & ~15u) | (unsigned)r) : 0u;
+#pragma unroll
+    for (int o = 0; o < kRounds; ++o) key = max(key, __shfl_sync(0xffffffffu, key, from[o]));
+    return (int)(key & 15u);
+  }
+};
 
 // Per frequency (blockIdx.y) and CTA: the sum over its wavevectors of
 // log |det(V(k) G - 1)|. per_warp: wavevector batches of one warp.
 template <int N>
-__global__ void __launch_bounds__(kLatThreads) k_sef_logdet(const double *__restrict__ G,
+__global__ void __launch_bounds__(kLatThreads, lattice_ctas(N)) k_sef_logdet(const double *__restrict__ G,
                                                             const double *__restrict__ V0, LatticeTerms terms,
                                                             unsigned long long nk, int per_warp, double *partials) {
   constexpr int GW = 32 / N;  // matrices per warp
   __shared__ LatticeTile<N> tile;
+  __shared__ double2 ph[kPhaseTable];
   __shared__ double red[kLatWarps];
   const int iw = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  fill_phases(terms, ph);
   tile.load(G + 2 * (size_t)iw * N * N, V0, 1.0);
   const int grp = min(lane / N, GW - 1);  // lanes past the last whole matrix repeat it, without a say in the pivots
   const bool mine = lane < GW * N;
   const int base = grp * N, r = mine ? lane - base : 0;
-  const unsigned mask = mine ? ((1u << N) - 1u) << base : (0xffffffffu << (GW * N));
-  double sum = 0.0;
+  const PivotRing<N> ring(base, r);
+  // sum of the pivots' log |.|: half the log of the product of |.|^2, kept as a
+  // mantissa in [1, 2) and an exponent, so that a lane takes one logarithm in all
+  double sum = 0.0, prod = 1.0;
+  int expo = 0;
   const unsigned long long k0 = ((unsigned long long)blockIdx.x * kLatWarps + warp) * per_warp * GW + grp;
-  for (int it = 0; it < per_warp; ++it) {
+  GridPoint k(terms, k0 < nk ? k0 : 0);
+  const int e0 = mine ? __ldg(terms.row + r) : 0, e1 = mine ? __ldg(terms.row + r + 1) : 0;
+  for (int it = 0; it < per_warp; ++it, k.advance(terms, GW)) {
     const unsigned long long kid = k0 + (unsigned long long)it * GW;
     const bool valid = kid < nk;
     if (!__any_sync(0xffffffffu, valid)) break;
     Cplx a[N];
-    tile.row(terms, valid ? kid : 0, r, 1.0, a);
+    tile.row(terms, ph, k, e0, e1, r, 1.0, a);
     bool open = true;
     Cplx piv = {1.0, 0.0};
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      const int p = pivot_lane(mask, open, a[j], r);
+      const int p = ring.lane(open, a[j], r);
       const int src = base + p;
       const Cplx pv = shfl(a[j], src);
       const double d = pv.x * pv.x + pv.y * pv.y;
-      const double rd = d > 0.0 ? 1.0 / d : 0.0;  // a zero pivot: log 0 below, nothing eliminated
+      const double rd = d > 0.0 ? reciprocal(d) : 0.0;  // a zero pivot: log 0 below, nothing eliminated
       if (r == p) {
         piv = pv;
         open = false;
@@ -169,12 +250,22 @@ __global__ void __launch_bounds__(kLatThreads) k_sef_logdet(const double *__rest
 #pragma unroll
       for (int c = j + 1; c < N; ++c) {
         const Cplx q = shfl(a[c], src);
-        a[c].x -= l.x * q.x - l.y * q.y;
-        a[c].y -= l.x * q.y + l.y * q.x;
+        csub(a[c], l, q);
       }
     }
-    if (valid && mine) sum += log(hypot(piv.x, piv.y));
+    if (valid && mine) {
+      const double d = piv.x * piv.x + piv.y * piv.y;
+      if (d > 1e-290 && d < 1e290) {
+        prod *= d;
+        const int e = ((__double2hiint(prod) >> 20) & 0x7ff) - 1023;
+        expo += e;
+        prod = __hiloint2double(__double2hiint(prod) - (e << 20), __double2loint(prod));
+      } else {  // zero (log 0), not a number, or a square out of range
+        sum += log(hypot(piv.x, piv.y));
+      }
+    }
   }
+  sum += 0.5 * (log(prod) + expo * 0.69314718055994530942);
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
   if (lane == 0) red[warp] = sum;
   __syncthreads();
@@ -191,36 +282,40 @@ __global__ void __launch_bounds__(kLatThreads) k_sef_logdet(const double *__rest
 // holding the inverse's column p_c; every matrix slot of the CTA adds into its
 // own N x N accumulator in shared memory, and the slots are added in order.
 template <int N>
-__global__ void __launch_bounds__(kLatThreads) k_cpt_partial(const double *__restrict__ G,
+__global__ void __launch_bounds__(kLatThreads, lattice_ctas(N)) k_cpt_partial(const double *__restrict__ G,
                                                              const double *__restrict__ V0, LatticeTerms terms,
                                                              unsigned long long nk, int per_warp, double *partials) {
   constexpr int GW = 32 / N;
   __shared__ LatticeTile<N> tile;
+  __shared__ double2 ph[kPhaseTable];
   __shared__ double2 acc[kLatWarps * GW][N * N];
   const int iw = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  fill_phases(terms, ph);
   double2 *flat = &acc[0][0];
   for (int t = threadIdx.x; t < kLatWarps * GW * N * N; t += blockDim.x) flat[t] = make_double2(0.0, 0.0);
   tile.load(G + 2 * (size_t)iw * N * N, V0 + 2 * (size_t)iw * N * N, -1.0);
   const int grp = min(lane / N, GW - 1);
   const bool mine = lane < GW * N;
   const int base = grp * N, r = mine ? lane - base : 0;
-  const unsigned mask = mine ? ((1u << N) - 1u) << base : (0xffffffffu << (GW * N));
+  const PivotRing<N> ring(base, r);
   double2 *out = acc[warp * GW + grp];
   const unsigned long long k0 = ((unsigned long long)blockIdx.x * kLatWarps + warp) * per_warp * GW + grp;
-  for (int it = 0; it < per_warp; ++it) {
+  GridPoint k(terms, k0 < nk ? k0 : 0);
+  const int e0 = mine ? __ldg(terms.row + r) : 0, e1 = mine ? __ldg(terms.row + r + 1) : 0;
+  for (int it = 0; it < per_warp; ++it, k.advance(terms, GW)) {
     const unsigned long long kid = k0 + (unsigned long long)it * GW;
     const bool valid = kid < nk;
     if (!__any_sync(0xffffffffu, valid)) break;
     Cplx a[N];
-    tile.row(terms, valid ? kid : 0, r, -1.0, a);
+    tile.row(terms, ph, k, e0, e1, r, -1.0, a);
     int row = -1;                  // the inverse's row this lane ends with
     unsigned long long perm = 0;   // p_c in bits 4 c ..
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      const int p = pivot_lane(mask, row < 0, a[j], r);
+      const int p = ring.lane(row < 0, a[j], r);
       const int src = base + p;
       const Cplx pv = shfl(a[j], src);
-      const double rd = 1.0 / (pv.x * pv.x + pv.y * pv.y);
+      const double rd = reciprocal(pv.x * pv.x + pv.y * pv.y);
       const Cplx inv = {pv.x * rd, -pv.y * rd};
       const bool self = r == p;
       if (self) row = j;
@@ -230,12 +325,8 @@ __global__ void __launch_bounds__(kLatThreads) k_cpt_partial(const double *__res
       for (int c = 0; c < N; ++c) {
         if (c == j) continue;
         const Cplx q = cmul(shfl(a[c], src), inv);
-        if (self) {
-          a[c] = q;
-        } else {
-          a[c].x -= f.x * q.x - f.y * q.y;
-          a[c].y -= f.x * q.y + f.y * q.x;
-        }
+        if (self) a[c] = q;
+        else csub(a[c], f, q);
       }
       const Cplx fi = cmul(f, inv);
       a[j] = self ? inv : Cplx{-fi.x, -fi.y};
@@ -267,16 +358,28 @@ __global__ void __launch_bounds__(kLatThreads) k_cpt_partial(const double *__res
 // column-major; the inverses are row-major.
 __global__ void k_cpt_reduce(int n, int nblk, double nk, const double *__restrict__ G,
                              const double *__restrict__ partials, double *Gproj) {
-  __shared__ double2 s[kLatMaxN * kLatMaxN];
+  __shared__ double2 s[kLatMaxN * kLatMaxN], part[256];
   const int iw = blockIdx.x, nn = n * n;
-  for (int t = threadIdx.x; t < nn; t += blockDim.x) {
+  // nn entries by `slices` strided shares of the CTAs' sums (256 threads)
+  const int slices = max(1, (int)blockDim.x / nn), entry = threadIdx.x % nn, slice = threadIdx.x / nn;
+  if (slice < slices) {
     double sr = 0.0, si = 0.0;
-    for (int q = 0; q < nblk; ++q) {
-      const double *p = partials + 2 * ((size_t)iw * nblk + q) * nn;
-      sr += p[2 * t];
-      si += p[2 * t + 1];
+#pragma unroll 4
+    for (int q = slice; q < nblk; q += slices) {
+      const double *p = partials + 2 * (((size_t)iw * nblk + q) * nn + entry);
+      sr += p[0];
+      si += p[1];
     }
-    s[t] = make_double2(sr, si);
+    part[threadIdx.x] = make_double2(sr, si);
+  }
+  __syncthreads();
+  if (threadIdx.x < nn) {
+    double2 t = part[threadIdx.x];
+    for (int q = 1; q < slices; ++q) {
+      t.x += part[q * nn + threadIdx.x].x;
+      t.y += part[q * nn + threadIdx.x].y;
+    }
+    s[threadIdx.x] = t;
   }
   __syncthreads();
   const double *g = G + 2 * (size_t)iw * nn;
@@ -299,10 +402,15 @@ __global__ void k_cpt_reduce(int n, int nblk, double nk, const double *__restric
 int batches_per_warp(int n, int nw, unsigned long long nk) {
   const unsigned long long per = (unsigned long long)kLatWarps * (32 / n);
   const unsigned long long all = (nk + per - 1) / per * (unsigned long long)std::max(nw, 1);
-  return (int)std::min<unsigned long long>(16, std::max<unsigned long long>(1, all / (148 * 8)));
+  return (int)std::min<unsigned long long>(8, std::max<unsigned long long>(1, all / (148 * 8)));
 }
 
 using LatticeFn = void (*)(const double *, const double *, LatticeTerms, unsigned long long, int, double *);
+LatticeTerms lattice_terms(const LatticeView &el, int nk0, int nk1, int nk2) {
+  auto magic = [](int nk) { return nk > 1 ? (unsigned)((0x100000000ull + nk - 1) / (unsigned)nk) : 0u; };
+  return {el.row, el.el, nk0, nk1, nk2, magic(nk0), magic(nk1), magic(nk2), (long)nk0 + nk1 + nk2 <= kPhaseTable};
+}
+
 const LatticeFn kLogdet[kLatMaxN] = {k_sef_logdet<1>,  k_sef_logdet<2>,  k_sef_logdet<3>,  k_sef_logdet<4>,
                                      k_sef_logdet<5>,  k_sef_logdet<6>,  k_sef_logdet<7>,  k_sef_logdet<8>,
                                      k_sef_logdet<9>,  k_sef_logdet<10>, k_sef_logdet<11>, k_sef_logdet<12>,
@@ -321,26 +429,23 @@ int lattice_blocks(int n, int nw, long nk) {
   return (int)(((unsigned long long)nk + per - 1) / per);
 }
 
-void launch_sef_logdet(int n, int nw, const double *G, const double *V0, const int *row, const int *col,
-                       const double *eR, const double *ev, int nkx, int nky, int nkz, double *partials,
+void launch_sef_logdet(int n, int nw, const double *G, const double *V0, const LatticeView &el, const int (&nk3)[3], double *partials,
                        cudaStream_t s) {
-  const long nk = (long)nkx * nky * nkz;
+  const long nk = (long)nk3[0] * nk3[1] * nk3[2];
   const int nblk = lattice_blocks(n, nw, nk);
   if (nw <= 0 || nk <= 0) return;
   if (nw > 65535) fail(QED_ERR_ARGUMENT, "SEF grid integrand: more than 65535 frequencies");
-  const LatticeTerms t{row, col, eR, ev, nkx, nky, nkz, 0.0};
+  const LatticeTerms t = lattice_terms(el, nk3[0], nk3[1], nk3[2]);
   kLogdet[n - 1]<<<dim3(nblk, nw), kLatThreads, 0, s>>>(G, V0, t, (unsigned long long)nk,
                                                          batches_per_warp(n, nw, nk), partials);
   QED_LAUNCH();
 }
 
-void launch_cpt_projected(int n, int nw, const double *G, const double *V0, const int *row, const int *col,
-                          const double *eR, const double *ev, int nkx, int nky, int nkz, double off,
-                          double *partials, double *Gproj, cudaStream_t s) {
-  const long nk = (long)nkx * nky * nkz;
+void launch_cpt_projected(int n, int nw, const double *G, const double *V0, const LatticeView &el, const int (&nk3)[3], double *partials, double *Gproj, cudaStream_t s) {
+  const long nk = (long)nk3[0] * nk3[1] * nk3[2];
   const int nblk = lattice_blocks(n, std::min(nw, 65535), nk);
   if (nw <= 0 || nk <= 0) return;
-  const LatticeTerms t{row, col, eR, ev, nkx, nky, nkz, off};
+  const LatticeTerms t = lattice_terms(el, nk3[0], nk3[1], nk3[2]);
   for (int w0 = 0; w0 < nw; w0 += 65535) {  // the grid's second dimension ends there
     const int m = std::min(nw - w0, 65535);
     const size_t o = 2 * (size_t)w0 * n * n;

@@ -91,3 +91,29 @@ def test_singular_matrix_gives_minus_infinity(qed, fresh):
     out = qed.sef_integrand_grid(np.array([[2j]]), [], [], [], [], [2.0, 1.0], (2, 2), label=label)
     assert out[0] == -np.inf
     assert out[1] == 0.0  # |2i / i - 1| = 1
+
+
+@pytest.mark.parametrize("n,M", [(1, 2), (1, 1), (2, 7), (4, 360), (10, 481), (16, 300), (31, 97), (32, 1)])
+def test_green_function_of_poles(qed, fresh, n, M):
+    """G(z) of a loaded Lehmann representation: one slice of poles and many, more
+    pairs than threads (n = 32), several shared-memory chunks (n = 10, M = 481).
+    Sums of at most 481 terms: error below 481 eps sum |terms| < 1e-12 here."""
+    rng = np.random.default_rng(n + M)
+    suffix, label = fresh()
+    name = "gfp" + suffix
+    qed.new_model(name, n)
+    qed.new_operator(name, "mu", "one-body", [(i, i, -1.0) for i in range(2 * n)])
+    qed.new_operator(name, "U", "interaction", [(i, i + n, 1.0) for i in range(n)])
+    qed.new_model_instance(name, {"mu": 1.0, "U": 2.0}, f"R0:N{n}:S{n % 2}", label)
+    e, v = rng.uniform(-4, 4, M), rng.standard_normal((n, M)) / np.sqrt(M)
+    dp = C.POINTER(C.c_double)
+    lib, i = qed.lib(), C.c_int()
+    vt = np.ascontiguousarray(v.T)
+    qed._check(lib.qed_instance_load_begin(label, -1.0, 0, 0))
+    qed._check(lib.qed_instance_load_state(label, b"R0:N0:S0", -1.0, 1.0, C.byref(i)))
+    qed._check(lib.qed_instance_load_qmatrix(label, 0, 0, n, M, e.ctypes.data_as(dp), vt.ctypes.data_as(dp)))
+    qed._check(lib.qed_instance_load_end(label))
+    z = np.array([0.3 + 0.4j, -2.0 + 0.5j, 0.9j])
+    got = qed.Green_function(z, label=label)
+    ref = np.einsum("am,zm,bm->zab", v, 1.0 / (z[:, None] - e[None, :]), v)
+    assert np.max(np.abs(got - ref)) < 1e-12
