@@ -1,6 +1,7 @@
 // Symmetry-adapted (mixed) basis Hamiltonian on the device: see mixed.hpp.
 #include "mixed.hpp"
 
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 
@@ -336,6 +337,274 @@ __global__ void __launch_bounds__(256) k_mixed_full(const Rows R, const double *
   }
 }
 
+// ---- packed matrix ----------------------------------------------------------
+//
+// What bounds the CSR product is the 12 bytes per entry (2x7 ladder with both
+// mirrors, 2.9e6 states, 98e6 entries: 1.2 GB, 331 us = 3.6 TB/s); the packed
+// form moves 4 and gathers better (see the times at launch_packed).
+
+constexpr uint32_t kPadCode = 255;
+constexpr int kPackedThreads = 256;
+
+// Amplitude classes of the off-diagonal terms, down-spin terms first.
+struct PackTerms {
+  int n, nlog;          // terms; log2 of the group order
+  const int *r, *c;
+  const uint8_t *cls;   // class | 128 where the amplitude is negative
+};
+
+// Images of every string of one spin under every group element: index of the
+// permuted string | phase (units of pi / g, mod 2 g) << 24, at img[e * dim + i].
+__global__ void k_sym_images(SymGroup G, const uint32_t *__restrict__ str, uint32_t dim, uint32_t *__restrict__ img) {
+  const uint64_t n = (uint64_t)dim * G.g;
+  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
+    const int e = (int)(t / dim);
+    int ph = 0;
+    const uint32_t b = sym_apply_half(G, e, str[t - (uint64_t)e * dim], ph);
+    img[t] = colex_rank(b) | (uint32_t)(ph % (2 * G.g)) << 24;
+  }
+}
+
+// Hops that the Pauli principle allows from state b (images that vanish in the
+// irrep included: their slots stay padded).
+__device__ __forceinline__ bool hop_allowed(uint64_t b, uint64_t mc, uint64_t mr) { return (b & mc) && !(b & mr); }
+
+// width[s] = the largest hop count among the 32 rows of slice s (one warp each)
+__global__ void __launch_bounds__(256) k_pack_width(int N, PackTerms t, const uint64_t *__restrict__ states,
+                                                    uint64_t D, uint64_t nslices, uint32_t *__restrict__ width) {
+  const uint64_t sl = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  if (sl >= nslices) return;
+  const uint64_t J = sl * 32 + (threadIdx.x & 31);
+  unsigned k = 0;
+  if (J < D) {
+    const uint64_t b = states[J];
+    for (int e = 0; e < t.n; ++e) k += hop_allowed(b, orb_mask(t.c[e], N), orb_mask(t.r[e], N));
+  }
+  k = __reduce_max_sync(0xffffffffu, k);
+  if ((threadIdx.x & 31) == 0) width[sl] = k;
+}
+
+// off[0 .. n] = exclusive sums of width[0 .. n); one CTA of 1024 threads
+__global__ void __launch_bounds__(1024) k_scan_widths(const uint32_t *__restrict__ width, uint64_t n,
+                                                      uint64_t *__restrict__ off) {
+  __shared__ uint64_t warp_sum[32];
+  uint64_t carry = 0;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (uint64_t base = 0; base < n; base += 1024) {
+    const uint64_t i = base + threadIdx.x;
+    uint64_t v = i < n ? width[i] : 0;
+    const uint64_t own = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    if (lane == 31) warp_sum[w] = v;
+    __syncthreads();
+    uint64_t before = 0, all = 0;
+    for (int q = 0; q < 32; ++q) {
+      if (q < w) before += warp_sum[q];
+      all += warp_sum[q];
+    }
+    if (i < n) off[i] = carry + before + v - own;
+    carry += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) off[n] = carry;
+}
+
+// Row J's entries, the matrix elements of k_mixed_rows. The representative of a
+// hopped state comes from the strings' image tables: the smallest factorized
+// index over the group (the order of the indices is that of the states), its
+// phase, and the stabiliser's order, as sym_representative finds them. A thread
+// per row; *nnz counts the entries.
+template <bool wide>
+__global__ void __launch_bounds__(128) k_pack_rows(SymGroup G, int irrep, PackTerms t,
+                                                   const uint32_t *__restrict__ img_up,
+                                                   const uint32_t *__restrict__ img_dn, uint32_t du, uint32_t dd,
+                                                   const uint64_t *__restrict__ states,
+                                                   const uint8_t *__restrict__ len, uint64_t D,
+                                                   const int32_t *__restrict__ fmap, const uint64_t *__restrict__ off,
+                                                   uint32_t *__restrict__ ent, uint8_t *__restrict__ code,
+                                                   unsigned long long *nnz) {
+  const uint64_t J = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  const uint64_t sl = J >> 5;
+  const int N = G.N, gm = 2 * G.g - 1;  // g is a power of two
+  uint32_t found = 0;
+  if (sl * 32 < D) {
+    const uint64_t s0 = off[sl], s1 = off[sl + 1];
+    const int lane = threadIdx.x & 31;
+    uint64_t k = s0;
+    if (J < D) {
+      const uint64_t b = states[J];
+      const uint32_t u = colex_rank((uint32_t)b), d = colex_rank((uint32_t)(b >> 32));
+      const int lj = __ffs((int)len[J]) - 1;
+      for (int e = 0; e < t.n; ++e) {
+        const uint64_t mc = orb_mask(t.c[e], N), mr = orb_mask(t.r[e], N);
+        if (!hop_allowed(b, mc, mr)) continue;
+        const uint64_t lo = mc < mr ? mc : mr, hi = mc < mr ? mr : mc;
+        int neg = __popcll(b & (hi - (lo << 1))) & 1;
+        const uint64_t nb = b - mc + mr;
+        const bool down = (mc >> 32) != 0;
+        const uint32_t u2 = down ? u : colex_rank((uint32_t)nb), d2 = down ? colex_rank((uint32_t)(nb >> 32)) : d;
+        const uint32_t f0 = u2 + du * d2;  // below 2^31
+        uint32_t rep = f0;
+        int ph = 0, h = 1;
+        bool null = false;
+        for (int q = 1; q < G.g; ++q) {
+          const uint32_t a = __ldg(img_up + (uint64_t)q * du + u2), c = __ldg(img_dn + (uint64_t)q * dd + d2);
+          const uint32_t f = (a & 0xffffffu) + du * (c & 0xffffffu);
+          const int pq = (int)((a >> 24) + (c >> 24) + 2 * G.phi[q][irrep]) & gm;
+          if (f == f0) {
+            ++h;
+            if (pq != 0 && (2 * G.g) % pq == 0) null = true;
+          }
+          if (f < rep) {
+            rep = f;
+            ph = pq;
+          }
+        }
+        if (null) continue;
+        const int32_t K = fmap[rep];
+        if (K < 0) continue;
+        const int lk = __ffs(G.g / h) - 1;
+        const uint8_t cls = t.cls[e];
+        neg ^= (ph != 0) ^ (cls >> 7);
+        const uint32_t cd = (uint32_t)((((cls & 127) * (2 * t.nlog + 1)) + (lj - lk + t.nlog)) * 2 + neg);
+        const uint64_t at = k * 32 + lane;
+        if (wide) {
+          ent[at] = (uint32_t)K;
+          code[at] = (uint8_t)cd;
+        } else {
+          ent[at] = (uint32_t)K | cd << 24;
+        }
+        ++k;
+        ++found;
+      }
+    }
+    for (; k < s1; ++k) {
+      const uint64_t at = k * 32 + lane;
+      ent[at] = wide ? 0u : kPadCode << 24;
+      if (wide) code[at] = (uint8_t)kPadCode;
+    }
+  }
+  found = __reduce_add_sync(0xffffffffu, found);
+  if ((threadIdx.x & 31) == 0 && found) atomicAdd(nnz, (unsigned long long)found);
+}
+
+// What a packed product does with a row's sum: the three epilogues of the CSR
+// kernels above. result() returns how many sums finish() writes per CTA.
+struct EpiSpmv {
+  static constexpr int kRed = 0;
+  const double *dg, *x;
+  double *y;
+  __device__ bool off() const { return false; }
+  __device__ __forceinline__ void row(uint64_t J, double s, double *) const { y[J] = dg[J] * x[J] + s; }
+  __device__ __forceinline__ void out(int, double) const {}
+};
+
+struct EpiLanczos {
+  static constexpr int kRed = 1;
+  const double *dg, *v, *vprev, *beta;
+  double *w, *partials;
+  int ld;
+  __device__ bool off() const { return false; }
+  __device__ __forceinline__ void row(uint64_t J, double s, double *red) const {
+    const double vj = v[J];
+    const double wj = dg[J] * vj + s - *beta * vprev[J];
+    w[J] = wj;
+    red[0] += vj * wj;
+  }
+  __device__ __forceinline__ void out(int, double t) const { partials[(size_t)blockIdx.x * ld] = t; }
+};
+
+struct EpiFull {
+  static constexpr int kRed = 3;
+  const double *dg, *x;
+  double xs;
+  double *y;
+  SubList sub;
+  int red_mask;
+  double *partials;
+  const int *skip;
+  __device__ bool off() const { return skip && *skip; }
+  __device__ __forceinline__ void row(uint64_t J, double s, double *red) const {
+    const double xj = x[J];
+    double yj = xs * (dg[J] * xj + s);
+    for (int k = 0; k < sub.n; ++k) yj -= (sub.cdev ? sub.cdev[k] : sub.c[k]) * sub.z[k][J];
+    y[J] = yj;
+    red[0] += xs * xj * yj;
+    red[1] += yj * yj;
+    red[2] += xs * xs * xj * xj;
+  }
+  __device__ __forceinline__ void out(int i, double t) const {
+    if (red_mask) partials[(size_t)blockIdx.x * Reducer::kMaxRed + i] = t;
+  }
+};
+
+// W warps share a slice (slots w, w + W, ...), a lane per row: W > 1 where the
+// sector has too few slices to fill the SMs. Six entries are in flight per lane.
+template <int W, bool wide, class Epi>
+__global__ void __launch_bounds__(kPackedThreads) k_packed(const PackedView P, const double *__restrict__ x,
+                                                           uint64_t D, uint64_t nslices, const Epi epi) {
+  if (epi.off()) return;
+  constexpr int kWarps = kPackedThreads / 32, kPer = kWarps / W;  // slices of the CTA per pass
+  constexpr int kDeep = 6;
+  __shared__ double values[256];
+  __shared__ double part[W > 1 ? kWarps : 1][32];
+  __shared__ double sums[Epi::kRed > 0 ? Epi::kRed : 1][kWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  values[threadIdx.x] = P.values[threadIdx.x];
+  __syncthreads();
+  double red[Epi::kRed > 0 ? Epi::kRed : 1] = {};
+  for (uint64_t base = (uint64_t)blockIdx.x * kPer; base < nslices; base += (uint64_t)gridDim.x * kPer) {
+    const uint64_t sl = base + warp / W;
+    double acc = 0.0;
+    if (sl < nslices) {
+      const uint64_t s1 = P.off[sl + 1];
+      for (uint64_t k = P.off[sl] + warp % W; k < s1; k += (uint64_t)W * kDeep) {
+        uint32_t e[kDeep], c[kDeep];
+#pragma unroll
+        for (int q = 0; q < kDeep; ++q) {
+          const bool in = k + (uint64_t)q * W < s1;
+          const uint64_t at = (k + (uint64_t)q * W) * 32 + lane;
+          e[q] = in ? __ldcs(P.ent + at) : kPadCode << 24;
+          c[q] = wide ? (in ? (uint32_t)__ldcs(P.code + at) : kPadCode) : e[q] >> 24;
+        }
+        double xv[kDeep];
+#pragma unroll
+        for (int q = 0; q < kDeep; ++q)
+          xv[q] = c[q] != kPadCode ? __ldg(x + (wide ? e[q] : e[q] & 0xffffffu)) : 0.0;
+#pragma unroll
+        for (int q = 0; q < kDeep; ++q) acc += values[c[q]] * xv[q];  // values[255] = 0
+      }
+    }
+    if (W > 1) {
+      part[warp][lane] = acc;
+      __syncthreads();
+      if (warp % W == 0) {
+        for (int q = 1; q < W; ++q) acc += part[warp + q][lane];
+      }
+    }
+    const uint64_t J = sl * 32 + lane;
+    if (warp % W == 0 && J < D) epi.row(J, acc, red);
+    if (W > 1) __syncthreads();  // part is read before the next slices
+  }
+  if (Epi::kRed > 0) {
+#pragma unroll
+    for (int i = 0; i < Epi::kRed; ++i) {
+      double v = red[i];
+      for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) sums[i][warp] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < Epi::kRed) {
+      double t = 0.0;
+      for (int k = 0; k < kWarps; ++k) t += sums[threadIdx.x][k];
+      epi.out(threadIdx.x, t);
+    }
+  }
+}
+
 struct OrbCoef {
   double c[kMaxSymOrb];
 };
@@ -482,9 +751,9 @@ MixedHamiltonian::MixedHamiltonian(const SymmetryGroup &G, const MixedTerms &t, 
   k_mixed_scatter<<<(unsigned)ntiles, kMarkThreads, 0, s>>>(lenf.p, nf, dtoff.p, us.p, (uint32_t)du, ds.p, fmap.p,
                                                             states.p, len.p);
   QED_LAUNCH();
-  row_ptr.alloc(D + 1);
   dg.alloc(D);
   if (D == 0) {
+    row_ptr.alloc(1);
     const uint64_t zero = 0;
     row_ptr.upload(&zero, 1, s);
     QED_CUDA(cudaStreamSynchronize(s));
@@ -495,6 +764,13 @@ MixedHamiltonian::MixedHamiltonian(const SymmetryGroup &G, const MixedTerms &t, 
   term_v.upload(t.v, s);
   n_terms = (int)t.r.size();
   const OffTerms ot{n_terms, term_r.p, term_c.p, term_v.p};
+  DevBuf<uint64_t> dm;
+  DevBuf<double> dv;
+  dm.upload(t.dmask, s);
+  dv.upload(t.dval, s);
+  k_mixed_diag<<<grid_for(D, 256), 256, 0, s>>>(states.p, D, dm.p, dv.p, (int)t.dmask.size(), dg.p);
+  QED_LAUNCH();
+  if (pack(t, us.p, ds.p, s)) return;
   DevBuf<uint32_t> cnt(D);
   k_mixed_rows<false><<<grid_for(D, 128), 128, 0, s>>>(G.tab, irrep, ot, states.p, len.p, D, fmap.p, (uint32_t)du,
                                                        cnt.p, nullptr, nullptr, nullptr);
@@ -521,13 +797,82 @@ MixedHamiltonian::MixedHamiltonian(const SymmetryGroup &G, const MixedTerms &t, 
                                                           (uint32_t)du, nullptr, row_ptr.p, col.p, val.p);
     QED_LAUNCH();
   }
-  DevBuf<uint64_t> dm;
-  DevBuf<double> dv;
-  dm.upload(t.dmask, s);
-  dv.upload(t.dval, s);
-  k_mixed_diag<<<grid_for(D, 256), 256, 0, s>>>(states.p, D, dm.p, dv.p, (int)t.dmask.size(), dg.p);
-  QED_LAUNCH();
   QED_CUDA(cudaStreamSynchronize(s));
+}
+
+// Builds the packed form where it applies (see mixed.hpp); false: nothing done.
+bool MixedHamiltonian::pack(const MixedTerms &t, const uint32_t *ustr, const uint32_t *dstr, cudaStream_t s) {
+  const int g = group.g, N = group.N;
+  if ((long)D < opt_int("max_dim_full") || opt_bool("mixed_on_the_fly")) return false;
+  if ((g & (g - 1)) || du >= (1u << 24) || dd >= (1u << 24) || t.r.empty()) return false;
+  int nlog = 0;
+  while ((1 << nlog) < g) ++nlog;
+  // classes of equal |amplitude|, terms with the down-spin ones first
+  std::vector<double> amp;
+  std::vector<int> hr, hc;
+  std::vector<uint8_t> cls;
+  for (int spin = 1; spin >= 0; --spin)
+    for (size_t e = 0; e < t.r.size(); ++e) {
+      if ((t.c[e] >= N) != (spin == 1)) continue;
+      const double a = std::fabs(t.v[e]);
+      const size_t k = std::find(amp.begin(), amp.end(), a) - amp.begin();
+      if (k == amp.size()) amp.push_back(a);
+      if (k >= 127) return false;
+      hr.push_back(t.r[e]);
+      hc.push_back(t.c[e]);
+      cls.push_back((uint8_t)(k | (t.v[e] < 0.0 ? 128 : 0)));
+    }
+  const int nr = 2 * nlog + 1;
+  if (amp.size() * nr * 2 > kPadCode) return false;
+  std::vector<double> hv(256, 0.0);
+  for (size_t k = 0; k < amp.size(); ++k)
+    for (int q = 0; q < nr; ++q) {  // sqrt(len_J / len_K) = sqrt(2^(q - nlog))
+      const double v = amp[k] * std::sqrt(std::ldexp(1.0, q - nlog));
+      hv[(k * nr + q) * 2] = v;
+      hv[(k * nr + q) * 2 + 1] = -v;
+    }
+  DevBuf<int> dr, dc;
+  DevBuf<uint8_t> dcls;
+  dr.upload(hr, s);
+  dc.upload(hc, s);
+  dcls.upload(cls, s);
+  values.upload(hv, s);
+  const PackTerms pt{(int)hr.size(), nlog, dr.p, dc.p, dcls.p};
+  const uint64_t nslices = (D + 31) / 32;
+  DevBuf<uint32_t> width(nslices);
+  slice_off.alloc(nslices + 1);
+  k_pack_width<<<(unsigned)((nslices * 32 + 255) / 256), 256, 0, s>>>(N, pt, states.p, D, nslices, width.p);
+  QED_LAUNCH();
+  k_scan_widths<<<1, 1024, 0, s>>>(width.p, nslices, slice_off.p);
+  QED_LAUNCH();
+  uint64_t slots = 0;
+  QED_CUDA(cudaMemcpyAsync(&slots, slice_off.p + nslices, sizeof(slots), cudaMemcpyDeviceToHost, s));
+  QED_CUDA(cudaStreamSynchronize(s));
+  const bool wide = D > (1u << 24);
+  if ((wide ? 5.0 : 4.0) * 32.0 * (double)slots > opt_double("mixed_csr_max_gb") * 1e9) {
+    slice_off.release();
+    values.release();
+    return false;
+  }
+  DevBuf<uint32_t> iu((size_t)g * du), id((size_t)g * dd);
+  k_sym_images<<<grid_for((uint64_t)g * du, 256), 256, 0, s>>>(group, ustr, du, iu.p);
+  QED_LAUNCH();
+  k_sym_images<<<grid_for((uint64_t)g * dd, 256), 256, 0, s>>>(group, dstr, dd, id.p);
+  QED_LAUNCH();
+  ent.alloc(32 * slots);
+  if (wide) code.alloc(32 * slots);
+  DevBuf<unsigned long long> dn(1);
+  QED_CUDA(cudaMemsetAsync(dn.p, 0, dn.bytes(), s));
+  auto rows = wide ? k_pack_rows<true> : k_pack_rows<false>;
+  rows<<<(unsigned)((D + 127) / 128), 128, 0, s>>>(group, irrep, pt, iu.p, id.p, du, dd, states.p, len.p, D, fmap.p,
+                                                   slice_off.p, ent.p, code.p, dn.p);
+  QED_LAUNCH();
+  unsigned long long n = 0;
+  dn.download(&n, 1, s);
+  QED_CUDA(cudaStreamSynchronize(s));
+  nnz = n;
+  packed = true;
+  return true;
 }
 
 namespace {
@@ -536,10 +881,33 @@ OtfRows otf_rows(const MixedHamiltonian &H) {
   return OtfRows{H.group, H.irrep, OffTerms{H.n_terms, H.term_r.p, H.term_c.p, H.term_v.p}, H.states.p, H.len.p,
                  H.fmap.p, H.du};
 }
+
+// Warps per slice: enough that the launch has about 24 warps per SM.
+template <int W, class Epi>
+int launch_packed_w(const MixedHamiltonian &H, const double *x, const Epi &epi, int max_blocks, cudaStream_t s) {
+  const uint64_t nslices = (H.D + 31) / 32, per = kPackedThreads / 32 / W;
+  unsigned nb = (unsigned)std::min<uint64_t>((nslices + per - 1) / per, grid_for(~0ull >> 1, 1));
+  if (max_blocks > 0 && nb > (unsigned)max_blocks) nb = (unsigned)max_blocks;
+  if (H.code.p)
+    k_packed<W, true><<<nb, kPackedThreads, 0, s>>>(H.packed_view(), x, H.D, nslices, epi);
+  else
+    k_packed<W, false><<<nb, kPackedThreads, 0, s>>>(H.packed_view(), x, H.D, nslices, epi);
+  QED_LAUNCH();
+  return (int)nb;
+}
+template <class Epi>
+int launch_packed(const MixedHamiltonian &H, const double *x, const Epi &epi, int max_blocks, cudaStream_t s) {
+  const uint64_t nslices = (H.D + 31) / 32;
+  if (nslices >= 148 * 24) return launch_packed_w<1>(H, x, epi, max_blocks, s);
+  if (nslices >= 148 * 8) return launch_packed_w<2>(H, x, epi, max_blocks, s);
+  if (nslices >= 148 * 2) return launch_packed_w<4>(H, x, epi, max_blocks, s);
+  return launch_packed_w<8>(H, x, epi, max_blocks, s);
+}
 }  // namespace
 
 int MixedHamiltonian::lanczos_w(const double *v, const double *vprev, const double *beta_dev, double *w,
                                 double *partials, int ld, int max_blocks, cudaStream_t s) const {
+  if (packed) return launch_packed(*this, v, EpiLanczos{dg.p, v, vprev, beta_dev, w, partials, ld}, max_blocks, s);
   unsigned nb = grid_for(D * 8, 256);
   if (nb > (unsigned)max_blocks) nb = (unsigned)max_blocks;
   if (on_the_fly)
@@ -552,6 +920,10 @@ int MixedHamiltonian::lanczos_w(const double *v, const double *vprev, const doub
 
 void MixedHamiltonian::apply(const double *x, double *y, cudaStream_t s) const {
   if (!D) return;
+  if (packed) {
+    launch_packed(*this, x, EpiSpmv{dg.p, x, y}, 0, s);
+    return;
+  }
   if (on_the_fly)
     k_mixed_spmv<<<grid_for(D * 8, 256), 256, 0, s>>>(otf_rows(*this), dg.p, x, y, D);
   else
@@ -562,6 +934,9 @@ void MixedHamiltonian::apply(const double *x, double *y, cudaStream_t s) const {
 int MixedHamiltonian::apply_full(const double *x, double xs, double *y, const SubList &sub, int red_mask,
                                  Reducer &r, cudaStream_t s, const int *skip) const {
   if (!D) return 0;
+  if (packed)
+    return launch_packed(*this, x, EpiFull{dg.p, x, xs, y, sub, red_mask, r.partials, skip}, red_mask ? r.max_blocks : 0,
+                         s);
   unsigned nb = grid_for(D * 8, 256);
   if (red_mask && nb > (unsigned)r.max_blocks) nb = (unsigned)r.max_blocks;
   if (on_the_fly)
@@ -573,7 +948,7 @@ int MixedHamiltonian::apply_full(const double *x, double xs, double *y, const Su
 }
 
 std::vector<double> MixedHamiltonian::dense(cudaStream_t s) const {
-  if (on_the_fly) fail(QED_ERR_INTERNAL, "dense form of an on-the-fly mixed Hamiltonian");
+  if (on_the_fly || packed) fail(QED_ERR_INTERNAL, "dense form of a mixed Hamiltonian without CSR");
   std::vector<uint64_t> rp(D + 1);
   std::vector<uint32_t> c(nnz);
   std::vector<double> v(nnz), d(D), out(D * D, 0.0);

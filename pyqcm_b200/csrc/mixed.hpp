@@ -17,12 +17,19 @@
 // diagonal and interaction elements, mask rule of
 // src_ed/Operators/HS_interaction_operator.hpp:44-53) is its own vector.
 //
-// H x is then a CSR product: eight lanes per row, HBM-bound on the column and
-// value arrays (12 bytes per entry), x gathered through L2. Sectors whose CSR
-// would exceed mixed_csr_max_gb (or every sector of at least max_dim_full
-// states, with mixed_on_the_fly) store no matrix: each product recomputes the
-// entries from the states, eight lanes per row over the one-body elements
-// (on_the_fly), with the same epilogues.
+// The matrix takes one of three forms, with the same products and epilogues:
+//  * packed (the usual one): a value is +-|amplitude| sqrt(len_J / len_K), one of
+//    a few dozen doubles, so an entry is a 24-bit column and an 8-bit code into
+//    their table (32-bit column and separate code above 2^24 states). Rows are
+//    stored in slices of 32, entry k of a slice's rows side by side, a lane per
+//    row; see PackedView.
+//  * CSR (12 bytes per entry, eight lanes per row): sectors small enough for full
+//    diagonalisation, which read the matrix back, and those outside the packed
+//    form (more than 255 values, a half basis of 2^24 strings).
+//  * on the fly: sectors whose stored matrix would exceed mixed_csr_max_gb (or
+//    every sector of at least max_dim_full states, with mixed_on_the_fly) store
+//    none; each product recomputes the entries from the states, eight lanes per
+//    row over the one-body elements.
 #pragma once
 
 #include <cstdint>
@@ -49,6 +56,19 @@ struct MixedTerms {
 };
 MixedTerms mixed_terms(const Model &m, const std::map<std::string, double> &value);
 
+// The packed matrix (see above): slice s holds rows 32 s .. 32 s + 31 and the
+// slots off[s] .. off[s + 1]; slot k's entry of row 32 s + l is ent[32 k + l],
+// column | code << 24 (code == null) or the column alone with its code at
+// code[32 k + l]. Entries come down-spin hops first, so that the rows of a slice,
+// which mostly share their down string, gather the same hop's targets side by
+// side. Code 255 pads short rows and is skipped.
+struct PackedView {
+  const uint64_t *off = nullptr;
+  const uint32_t *ent = nullptr;
+  const uint8_t *code = nullptr;
+  const double *values = nullptr;  // 256
+};
+
 struct MixedHamiltonian {
   size_t D = 0;          // basis dimension
   size_t nnz = 0;        // off-diagonal entries
@@ -62,12 +82,18 @@ struct MixedHamiltonian {
   DevBuf<uint32_t> col;
   DevBuf<double> val;
   DevBuf<double> dg;         // diagonal
+  bool packed = false;       // the packed form holds the matrix (row_ptr, col, val are empty)
+  DevBuf<uint64_t> slice_off;
+  DevBuf<uint32_t> ent;
+  DevBuf<uint8_t> code;
+  DevBuf<double> values;
   bool on_the_fly = false;   // no stored matrix: entries recomputed by every product
   int n_terms = 0;           // off-diagonal one-body elements (kept for the on-the-fly products)
   DevBuf<int> term_r, term_c;
   DevBuf<double> term_v;
 
   MixedHamiltonian(const SymmetryGroup &G, const MixedTerms &t, int irrep, int n_up, int n_dn, cudaStream_t s);
+  PackedView packed_view() const { return {slice_off.p, ent.p, code.p, values.p}; }
   // y = H x on device vectors of D doubles, on stream s
   void apply(const double *x, double *y, cudaStream_t s) const;
   // y = xs H x - sum_k sub.c[k] sub.z[k], with the column pass's reductions of
@@ -78,6 +104,7 @@ struct MixedHamiltonian {
                  cudaStream_t s, const int *skip = nullptr) const;
   // the matrix as D x D dense (column-major), for full diagonalisation of small sectors
   std::vector<double> dense(cudaStream_t s) const;
+  bool pack(const MixedTerms &t, const uint32_t *ustr, const uint32_t *dstr, cudaStream_t s);
   // w = H v - (*beta_dev) vprev, with per-block partials of <v, w> at
   // partials[block * ld]; returns the number of blocks (at most max_blocks)
   int lanczos_w(const double *v, const double *vprev, const double *beta_dev, double *w, double *partials, int ld,
