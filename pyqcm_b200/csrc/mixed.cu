@@ -346,9 +346,9 @@ __global__ void __launch_bounds__(256) k_mixed_full(const Rows R, const double *
 constexpr uint32_t kPadCode = 255;
 constexpr int kPackedThreads = 256;
 
-// Amplitude classes of the off-diagonal terms, down-spin terms first.
+// Amplitude classes of the off-diagonal terms.
 struct PackTerms {
-  int n, nlog;          // terms; log2 of the group order
+  int n, n_up, nlog;    // terms, the up-spin ones first; log2 of the group order
   const int *r, *c;
   const uint8_t *cls;   // class | 128 where the amplitude is negative
 };
@@ -369,19 +369,29 @@ __global__ void k_sym_images(SymGroup G, const uint32_t *__restrict__ str, uint3
 // irrep included: their slots stay padded).
 __device__ __forceinline__ bool hop_allowed(uint64_t b, uint64_t mc, uint64_t mr) { return (b & mc) && !(b & mr); }
 
-// width[s] = the largest hop count among the 32 rows of slice s (one warp each)
+// up[s] and width[s] = the largest up-spin hop count among the 32 rows of slice s,
+// and that plus the largest down-spin one (one warp each)
 __global__ void __launch_bounds__(256) k_pack_width(int N, PackTerms t, const uint64_t *__restrict__ states,
-                                                    uint64_t D, uint64_t nslices, uint32_t *__restrict__ width) {
+                                                    uint64_t D, uint64_t nslices, uint8_t *__restrict__ up,
+                                                    uint32_t *__restrict__ width) {
   const uint64_t sl = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   if (sl >= nslices) return;
   const uint64_t J = sl * 32 + (threadIdx.x & 31);
-  unsigned k = 0;
+  unsigned ku = 0, kd = 0;
   if (J < D) {
     const uint64_t b = states[J];
-    for (int e = 0; e < t.n; ++e) k += hop_allowed(b, orb_mask(t.c[e], N), orb_mask(t.r[e], N));
+    for (int e = 0; e < t.n; ++e) {
+      const bool has = hop_allowed(b, orb_mask(t.c[e], N), orb_mask(t.r[e], N));
+      if (e < t.n_up) ku += has;
+      else kd += has;
+    }
   }
-  k = __reduce_max_sync(0xffffffffu, k);
-  if ((threadIdx.x & 31) == 0) width[sl] = k;
+  ku = __reduce_max_sync(0xffffffffu, ku);
+  kd = __reduce_max_sync(0xffffffffu, kd);
+  if ((threadIdx.x & 31) == 0) {
+    up[sl] = (uint8_t)ku;
+    width[sl] = ku + kd;
+  }
 }
 
 // off[0 .. n] = exclusive sums of width[0 .. n); one CTA of 1024 threads
@@ -424,6 +434,7 @@ __global__ void __launch_bounds__(128) k_pack_rows(SymGroup G, int irrep, PackTe
                                                    const uint64_t *__restrict__ states,
                                                    const uint8_t *__restrict__ len, uint64_t D,
                                                    const int32_t *__restrict__ fmap, const uint64_t *__restrict__ off,
+                                                   const uint8_t *__restrict__ up, uint8_t *__restrict__ row_up,
                                                    uint32_t *__restrict__ ent, uint8_t *__restrict__ code,
                                                    unsigned long long *nnz) {
   const uint64_t J = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -431,14 +442,25 @@ __global__ void __launch_bounds__(128) k_pack_rows(SymGroup G, int irrep, PackTe
   const int N = G.N, gm = 2 * G.g - 1;  // g is a power of two
   uint32_t found = 0;
   if (sl * 32 < D) {
-    const uint64_t s0 = off[sl], s1 = off[sl + 1];
+    const uint64_t s0 = off[sl], s1 = off[sl + 1], su = s0 + up[sl];
     const int lane = threadIdx.x & 31;
     uint64_t k = s0;
+    auto pad_to = [&](uint64_t end) {
+      for (; k < end; ++k) {
+        const uint64_t at = k * 32 + lane;
+        ent[at] = wide ? 0u : kPadCode << 24;
+        if (wide) code[at] = (uint8_t)kPadCode;
+      }
+    };
     if (J < D) {
       const uint64_t b = states[J];
       const uint32_t u = colex_rank((uint32_t)b), d = colex_rank((uint32_t)(b >> 32));
       const int lj = __ffs((int)len[J]) - 1;
       for (int e = 0; e < t.n; ++e) {
+        if (e == t.n_up) {
+          row_up[J] = (uint8_t)(k - s0);
+          pad_to(su);
+        }
         const uint64_t mc = orb_mask(t.c[e], N), mr = orb_mask(t.r[e], N);
         if (!hop_allowed(b, mc, mr)) continue;
         const uint64_t lo = mc < mr ? mc : mr, hi = mc < mr ? mr : mc;
@@ -481,25 +503,21 @@ __global__ void __launch_bounds__(128) k_pack_rows(SymGroup G, int irrep, PackTe
         ++found;
       }
     }
-    for (; k < s1; ++k) {
-      const uint64_t at = k * 32 + lane;
-      ent[at] = wide ? 0u : kPadCode << 24;
-      if (wide) code[at] = (uint8_t)kPadCode;
-    }
+    pad_to(s1);
   }
   found = __reduce_add_sync(0xffffffffu, found);
   if ((threadIdx.x & 31) == 0 && found) atomicAdd(nnz, (unsigned long long)found);
 }
 
 // What a packed product does with a row's sum: the three epilogues of the CSR
-// kernels above. result() returns how many sums finish() writes per CTA.
+// kernels above; out(b, i, t) takes sum i of virtual block b.
 struct EpiSpmv {
   static constexpr int kRed = 0;
   const double *dg, *x;
   double *y;
   __device__ bool off() const { return false; }
   __device__ __forceinline__ void row(uint64_t J, double s, double *) const { y[J] = dg[J] * x[J] + s; }
-  __device__ __forceinline__ void out(int, double) const {}
+  __device__ __forceinline__ void out(uint64_t, int, double) const {}
 };
 
 struct EpiLanczos {
@@ -514,7 +532,7 @@ struct EpiLanczos {
     w[J] = wj;
     red[0] += vj * wj;
   }
-  __device__ __forceinline__ void out(int, double t) const { partials[(size_t)blockIdx.x * ld] = t; }
+  __device__ __forceinline__ void out(uint64_t b, int, double t) const { partials[(size_t)b * ld] = t; }
 };
 
 struct EpiFull {
@@ -536,26 +554,142 @@ struct EpiFull {
     red[1] += yj * yj;
     red[2] += xs * xs * xj * xj;
   }
-  __device__ __forceinline__ void out(int i, double t) const {
-    if (red_mask) partials[(size_t)blockIdx.x * Reducer::kMaxRed + i] = t;
+  __device__ __forceinline__ void out(uint64_t b, int i, double t) const {
+    if (red_mask) partials[(size_t)b * Reducer::kMaxRed + i] = t;
   }
 };
 
-// W warps share a slice (slots w, w + W, ...), a lane per row: W > 1 where the
-// sector has too few slices to fill the SMs. Six entries are in flight per lane.
+// Every sum is taken in the order of the CSR kernels (eight lanes per row, 256
+// threads per block of 32 rows), so that both give the same bits - the solver's
+// recurrences stop at thresholds that last digits can tip (HvOperator::keep_order):
+// a row keeps the eight partial sums of its entries k mod 8 (entry j of the down
+// part is entry row_up + j of the row) and adds them as the shuffles did; virtual
+// block b of `nb` owns the slices b, b + nb, ... and adds its rows as block b did.
+// A lane per row; W warps share a virtual block's slice, slots w, w + W, ... of each
+// part (between the parts the partial sums change hands in shared memory).
+//
+// Bound by latency (offsets -> entries -> gathers) where a sector has a slice or
+// two per warp, by the gathers where it has many: a warp's first entries of both
+// parts are requested together, before the up part's gathers.
+template <int W> struct PackedBatch {
+  static constexpr int Q = 8 / W;                                  // partial sums of a warp
+  static constexpr int R = W == 4 ? 3 : 4;  // rounds of eight slots per batch
+};
+template <int W, bool wide>
+__device__ __forceinline__ void packed_entries(const PackedView &P, uint64_t k, uint64_t s1, int lane,
+                                               uint32_t (&e)[PackedBatch<W>::Q * PackedBatch<W>::R],
+                                               uint32_t (&c)[PackedBatch<W>::Q * PackedBatch<W>::R]) {
+#pragma unroll
+  for (int q = 0; q < PackedBatch<W>::Q * PackedBatch<W>::R; ++q) {
+    const bool in = k + q * W < s1;
+    const uint64_t at = (k + q * W) * 32 + lane;
+    e[q] = in ? __ldcs(P.ent + at) : kPadCode << 24;
+    c[q] = wide ? (in ? (uint32_t)__ldcs(P.code + at) : kPadCode) : e[q] >> 24;
+  }
+}
+template <int W, bool wide>
+__device__ __forceinline__ void packed_apply(const double *__restrict__ x, const double *values,
+                                             const uint32_t (&e)[PackedBatch<W>::Q * PackedBatch<W>::R],
+                                             const uint32_t (&c)[PackedBatch<W>::Q * PackedBatch<W>::R],
+                                             double (&acc)[PackedBatch<W>::Q]) {
+  constexpr int Q = PackedBatch<W>::Q, N = Q * PackedBatch<W>::R;
+  double xv[N];
+#pragma unroll
+  for (int q = 0; q < N; ++q) xv[q] = c[q] != kPadCode ? __ldg(x + (wide ? e[q] : e[q] & 0xffffffu)) : 0.0;
+#pragma unroll
+  for (int q = 0; q < N; ++q) acc[q % Q] = fma(values[c[q]], xv[q], acc[q % Q]);  // values[255] = 0
+}
+// slots k, k + W, ... of a part, the first batch of entries already there
+template <int W, bool wide>
+__device__ __forceinline__ void packed_part(const PackedView &P, const double *__restrict__ x, const double *values,
+                                            uint64_t k, uint64_t s1, int lane,
+                                            uint32_t (&e)[PackedBatch<W>::Q * PackedBatch<W>::R],
+                                            uint32_t (&c)[PackedBatch<W>::Q * PackedBatch<W>::R],
+                                            double (&acc)[PackedBatch<W>::Q]) {
+  constexpr int kStep = 8 * PackedBatch<W>::R;
+  packed_apply<W, wide>(x, values, e, c, acc);
+  for (k += kStep; k < s1; k += kStep) {
+    packed_entries<W, wide>(P, k, s1, lane, e, c);
+    packed_apply<W, wide>(x, values, e, c, acc);
+  }
+}
+
 template <int W, bool wide, class Epi>
 __global__ void __launch_bounds__(kPackedThreads) k_packed(const PackedView P, const double *__restrict__ x,
-                                                           uint64_t D, uint64_t nslices, const Epi epi) {
+                                                           uint64_t D, uint64_t nslices, uint64_t nb, const Epi epi) {
   if (epi.off()) return;
-  constexpr int kWarps = kPackedThreads / 32, kPer = kWarps / W;  // slices of the CTA per pass
-  constexpr int kDeep = 6;
+  constexpr int kWarps = kPackedThreads / 32, kBlocks = kWarps / W, Q = 8 / W;
+  __shared__ double values[256];
+  __shared__ double part[kBlocks][8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w = warp % W, own = warp / W;
+  values[threadIdx.x] = P.values[threadIdx.x];
+  __syncthreads();
+  const uint64_t vb = (uint64_t)blockIdx.x * kBlocks + own;
+  double red[Epi::kRed > 0 ? Epi::kRed : 1] = {};
+  for (uint64_t base = 0; base < nslices; base += nb) {
+    const uint64_t sl = base + vb, J = sl * 32 + lane;
+    const bool on = vb < nb && sl < nslices;
+    uint64_t s0 = 0, su = 0, s1 = 0;
+    int first = 0;
+    constexpr int kBatch = Q * PackedBatch<W>::R;
+    uint32_t eu[kBatch], cu[kBatch], ed[kBatch], cd[kBatch];
+    double acc[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) acc[q] = 0.0;
+    if (on) {
+      s0 = P.off[sl];
+      s1 = P.off[sl + 1];
+      su = s0 + P.up[sl];
+      first = J < D ? P.row_up[J] : 0;
+      packed_entries<W, wide>(P, s0 + w, su, lane, eu, cu);
+      packed_entries<W, wide>(P, su + w, s1, lane, ed, cd);
+      packed_part<W, wide>(P, x, values, s0 + w, su, lane, eu, cu, acc);
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) part[own][w + q * W][lane] = acc[q];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < Q; ++q) acc[q] = part[own][(first + w + q * W) & 7][lane];
+    if (on) packed_part<W, wide>(P, x, values, su + w, s1, lane, ed, cd, acc);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) part[own][(first + w + q * W) & 7][lane] = acc[q];
+    __syncthreads();
+    if (w == 0 && on && J < D) {
+      double p[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) p[q] = part[own][q][lane];
+      epi.row(J, ((p[0] + p[4]) + (p[2] + p[6])) + ((p[1] + p[5]) + (p[3] + p[7])), red);
+    }
+    __syncthreads();  // part is read before the next slice
+  }
+  if (Epi::kRed > 0 && w == 0 && vb < nb) {
+#pragma unroll
+    for (int i = 0; i < Epi::kRed; ++i) {
+      double v = red[i];  // rows 4 k .. 4 k + 3 were one warp of block vb
+      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      double t = 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) t += __shfl_sync(0xffffffffu, v, 4 * k);
+      if (lane == 0) epi.out(vb, i, t);
+    }
+  }
+}
+
+// y = H x for callers outside the recurrences: the same entries, summed as they
+// come by one lane per row, W warps per slice. Half the time of the ordered form on
+// large sectors (no exchange between the parts, one accumulator, six entries in
+// flight whatever the part).
+template <int W, bool wide>
+__global__ void __launch_bounds__(kPackedThreads) k_packed_free(const PackedView P, const double *__restrict__ x,
+                                                                uint64_t D, uint64_t nslices,
+                                                                const double *__restrict__ dg, double *y) {
+  constexpr int kWarps = kPackedThreads / 32, kPer = kWarps / W, kDeep = 6;
   __shared__ double values[256];
   __shared__ double part[W > 1 ? kWarps : 1][32];
-  __shared__ double sums[Epi::kRed > 0 ? Epi::kRed : 1][kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   values[threadIdx.x] = P.values[threadIdx.x];
   __syncthreads();
-  double red[Epi::kRed > 0 ? Epi::kRed : 1] = {};
   for (uint64_t base = (uint64_t)blockIdx.x * kPer; base < nslices; base += (uint64_t)gridDim.x * kPer) {
     const uint64_t sl = base + warp / W;
     double acc = 0.0;
@@ -565,43 +699,27 @@ __global__ void __launch_bounds__(kPackedThreads) k_packed(const PackedView P, c
         uint32_t e[kDeep], c[kDeep];
 #pragma unroll
         for (int q = 0; q < kDeep; ++q) {
-          const bool in = k + (uint64_t)q * W < s1;
-          const uint64_t at = (k + (uint64_t)q * W) * 32 + lane;
+          const bool in = k + q * W < s1;
+          const uint64_t at = (k + q * W) * 32 + lane;
           e[q] = in ? __ldcs(P.ent + at) : kPadCode << 24;
           c[q] = wide ? (in ? (uint32_t)__ldcs(P.code + at) : kPadCode) : e[q] >> 24;
         }
         double xv[kDeep];
 #pragma unroll
-        for (int q = 0; q < kDeep; ++q)
-          xv[q] = c[q] != kPadCode ? __ldg(x + (wide ? e[q] : e[q] & 0xffffffu)) : 0.0;
+        for (int q = 0; q < kDeep; ++q) xv[q] = c[q] != kPadCode ? __ldg(x + (wide ? e[q] : e[q] & 0xffffffu)) : 0.0;
 #pragma unroll
-        for (int q = 0; q < kDeep; ++q) acc += values[c[q]] * xv[q];  // values[255] = 0
+        for (int q = 0; q < kDeep; ++q) acc += values[c[q]] * xv[q];
       }
     }
     if (W > 1) {
       part[warp][lane] = acc;
       __syncthreads();
-      if (warp % W == 0) {
+      if (warp % W == 0)
         for (int q = 1; q < W; ++q) acc += part[warp + q][lane];
-      }
     }
     const uint64_t J = sl * 32 + lane;
-    if (warp % W == 0 && J < D) epi.row(J, acc, red);
+    if (warp % W == 0 && J < D) y[J] = dg[J] * x[J] + acc;
     if (W > 1) __syncthreads();  // part is read before the next slices
-  }
-  if (Epi::kRed > 0) {
-#pragma unroll
-    for (int i = 0; i < Epi::kRed; ++i) {
-      double v = red[i];
-      for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) sums[i][warp] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < Epi::kRed) {
-      double t = 0.0;
-      for (int k = 0; k < kWarps; ++k) t += sums[threadIdx.x][k];
-      epi.out(threadIdx.x, t);
-    }
   }
 }
 
@@ -807,21 +925,21 @@ bool MixedHamiltonian::pack(const MixedTerms &t, const uint32_t *ustr, const uin
   if ((g & (g - 1)) || du >= (1u << 24) || dd >= (1u << 24) || t.r.empty()) return false;
   int nlog = 0;
   while ((1 << nlog) < g) ++nlog;
-  // classes of equal |amplitude|, terms with the down-spin ones first
-  std::vector<double> amp;
-  std::vector<int> hr, hc;
+  std::vector<double> amp;  // classes of equal |amplitude|
   std::vector<uint8_t> cls;
-  for (int spin = 1; spin >= 0; --spin)
-    for (size_t e = 0; e < t.r.size(); ++e) {
-      if ((t.c[e] >= N) != (spin == 1)) continue;
-      const double a = std::fabs(t.v[e]);
-      const size_t k = std::find(amp.begin(), amp.end(), a) - amp.begin();
-      if (k == amp.size()) amp.push_back(a);
-      if (k >= 127) return false;
-      hr.push_back(t.r[e]);
-      hc.push_back(t.c[e]);
-      cls.push_back((uint8_t)(k | (t.v[e] < 0.0 ? 128 : 0)));
-    }
+  for (size_t e = 0; e < t.r.size(); ++e) {
+    const double a = std::fabs(t.v[e]);
+    const size_t k = std::find(amp.begin(), amp.end(), a) - amp.begin();
+    if (k == amp.size()) amp.push_back(a);
+    if (k >= 127) return false;
+    cls.push_back((uint8_t)(k | (t.v[e] < 0.0 ? 128 : 0)));
+  }
+  // up-spin hops, then down-spin ones, none between the spins: the order of t
+  int n_up = 0;
+  while (n_up < n_terms && t.r[n_up] < N) ++n_up;
+  for (int e = 0; e < n_terms; ++e)
+    if ((t.r[e] < N) != (e < n_up) || (t.c[e] < N) != (e < n_up)) return false;
+  if (n_up == 0 || n_up == n_terms || n_up > 255) return false;
   const int nr = 2 * nlog + 1;
   if (amp.size() * nr * 2 > kPadCode) return false;
   std::vector<double> hv(256, 0.0);
@@ -831,17 +949,15 @@ bool MixedHamiltonian::pack(const MixedTerms &t, const uint32_t *ustr, const uin
       hv[(k * nr + q) * 2] = v;
       hv[(k * nr + q) * 2 + 1] = -v;
     }
-  DevBuf<int> dr, dc;
   DevBuf<uint8_t> dcls;
-  dr.upload(hr, s);
-  dc.upload(hc, s);
   dcls.upload(cls, s);
   values.upload(hv, s);
-  const PackTerms pt{(int)hr.size(), nlog, dr.p, dc.p, dcls.p};
+  const PackTerms pt{n_terms, n_up, nlog, term_r.p, term_c.p, dcls.p};
   const uint64_t nslices = (D + 31) / 32;
   DevBuf<uint32_t> width(nslices);
   slice_off.alloc(nslices + 1);
-  k_pack_width<<<(unsigned)((nslices * 32 + 255) / 256), 256, 0, s>>>(N, pt, states.p, D, nslices, width.p);
+  slice_up.alloc(nslices);
+  k_pack_width<<<(unsigned)((nslices * 32 + 255) / 256), 256, 0, s>>>(N, pt, states.p, D, nslices, slice_up.p, width.p);
   QED_LAUNCH();
   k_scan_widths<<<1, 1024, 0, s>>>(width.p, nslices, slice_off.p);
   QED_LAUNCH();
@@ -851,6 +967,7 @@ bool MixedHamiltonian::pack(const MixedTerms &t, const uint32_t *ustr, const uin
   const bool wide = D > (1u << 24);
   if ((wide ? 5.0 : 4.0) * 32.0 * (double)slots > opt_double("mixed_csr_max_gb") * 1e9) {
     slice_off.release();
+    slice_up.release();
     values.release();
     return false;
   }
@@ -859,13 +976,14 @@ bool MixedHamiltonian::pack(const MixedTerms &t, const uint32_t *ustr, const uin
   QED_LAUNCH();
   k_sym_images<<<grid_for((uint64_t)g * dd, 256), 256, 0, s>>>(group, dstr, dd, id.p);
   QED_LAUNCH();
+  row_up.alloc(D);
   ent.alloc(32 * slots);
   if (wide) code.alloc(32 * slots);
   DevBuf<unsigned long long> dn(1);
   QED_CUDA(cudaMemsetAsync(dn.p, 0, dn.bytes(), s));
   auto rows = wide ? k_pack_rows<true> : k_pack_rows<false>;
   rows<<<(unsigned)((D + 127) / 128), 128, 0, s>>>(group, irrep, pt, iu.p, id.p, du, dd, states.p, len.p, D, fmap.p,
-                                                   slice_off.p, ent.p, code.p, dn.p);
+                                                   slice_off.p, slice_up.p, row_up.p, ent.p, code.p, dn.p);
   QED_LAUNCH();
   unsigned long long n = 0;
   dn.download(&n, 1, s);
@@ -882,34 +1000,49 @@ OtfRows otf_rows(const MixedHamiltonian &H) {
                  H.fmap.p, H.du};
 }
 
-// Warps per slice: enough that the launch has about 24 warps per SM.
+// nb virtual blocks (those of the CSR kernels where there are sums to keep in
+// order), W warps each: enough that the launch has about 32 warps per SM.
 template <int W, class Epi>
-int launch_packed_w(const MixedHamiltonian &H, const double *x, const Epi &epi, int max_blocks, cudaStream_t s) {
-  const uint64_t nslices = (H.D + 31) / 32, per = kPackedThreads / 32 / W;
-  unsigned nb = (unsigned)std::min<uint64_t>((nslices + per - 1) / per, grid_for(~0ull >> 1, 1));
-  if (max_blocks > 0 && nb > (unsigned)max_blocks) nb = (unsigned)max_blocks;
+void launch_packed_w(const MixedHamiltonian &H, const double *x, const Epi &epi, unsigned nb, cudaStream_t s) {
+  const uint64_t nslices = (H.D + 31) / 32;
+  const unsigned per = kPackedThreads / 32 / W, grid = (nb + per - 1) / per;
   if (H.code.p)
-    k_packed<W, true><<<nb, kPackedThreads, 0, s>>>(H.packed_view(), x, H.D, nslices, epi);
+    k_packed<W, true><<<grid, kPackedThreads, 0, s>>>(H.packed_view(), x, H.D, nslices, nb, epi);
   else
-    k_packed<W, false><<<nb, kPackedThreads, 0, s>>>(H.packed_view(), x, H.D, nslices, epi);
+    k_packed<W, false><<<grid, kPackedThreads, 0, s>>>(H.packed_view(), x, H.D, nslices, nb, epi);
   QED_LAUNCH();
-  return (int)nb;
 }
 template <class Epi>
-int launch_packed(const MixedHamiltonian &H, const double *x, const Epi &epi, int max_blocks, cudaStream_t s) {
+int launch_packed(const MixedHamiltonian &H, const double *x, const Epi &epi, unsigned nb, cudaStream_t s) {
+  if (nb >= 148 * 3) launch_packed_w<4>(H, x, epi, nb, s);
+  else launch_packed_w<8>(H, x, epi, nb, s);
+  return (int)nb;
+}
+
+template <int W> void launch_packed_free_w(const MixedHamiltonian &H, const double *x, double *y, cudaStream_t s) {
+  const uint64_t nslices = (H.D + 31) / 32, per = kPackedThreads / 32 / W;
+  const unsigned grid = (unsigned)std::min<uint64_t>((nslices + per - 1) / per, 148 * 16);
+  if (H.code.p)
+    k_packed_free<W, true><<<grid, kPackedThreads, 0, s>>>(H.packed_view(), x, H.D, nslices, H.dg.p, y);
+  else
+    k_packed_free<W, false><<<grid, kPackedThreads, 0, s>>>(H.packed_view(), x, H.D, nslices, H.dg.p, y);
+  QED_LAUNCH();
+}
+// Warps per slice: about 24 slices per SM fill it with one warp each.
+void launch_packed_free(const MixedHamiltonian &H, const double *x, double *y, cudaStream_t s) {
   const uint64_t nslices = (H.D + 31) / 32;
-  if (nslices >= 148 * 24) return launch_packed_w<1>(H, x, epi, max_blocks, s);
-  if (nslices >= 148 * 8) return launch_packed_w<2>(H, x, epi, max_blocks, s);
-  if (nslices >= 148 * 2) return launch_packed_w<4>(H, x, epi, max_blocks, s);
-  return launch_packed_w<8>(H, x, epi, max_blocks, s);
+  if (nslices >= 148 * 24) launch_packed_free_w<1>(H, x, y, s);
+  else if (nslices >= 148 * 16) launch_packed_free_w<2>(H, x, y, s);
+  else if (nslices >= 148 * 3) launch_packed_free_w<4>(H, x, y, s);
+  else launch_packed_free_w<8>(H, x, y, s);
 }
 }  // namespace
 
 int MixedHamiltonian::lanczos_w(const double *v, const double *vprev, const double *beta_dev, double *w,
                                 double *partials, int ld, int max_blocks, cudaStream_t s) const {
-  if (packed) return launch_packed(*this, v, EpiLanczos{dg.p, v, vprev, beta_dev, w, partials, ld}, max_blocks, s);
   unsigned nb = grid_for(D * 8, 256);
   if (nb > (unsigned)max_blocks) nb = (unsigned)max_blocks;
+  if (packed) return launch_packed(*this, v, EpiLanczos{dg.p, v, vprev, beta_dev, w, partials, ld}, nb, s);
   if (on_the_fly)
     k_mixed_lanczos_w<<<nb, 256, 0, s>>>(otf_rows(*this), dg.p, v, vprev, beta_dev, w, D, partials, ld);
   else
@@ -919,9 +1052,16 @@ int MixedHamiltonian::lanczos_w(const double *v, const double *vprev, const doub
 }
 
 void MixedHamiltonian::apply(const double *x, double *y, cudaStream_t s) const {
+  if (D && packed)
+    launch_packed_free(*this, x, y, s);
+  else
+    apply_ordered(x, y, s);
+}
+
+void MixedHamiltonian::apply_ordered(const double *x, double *y, cudaStream_t s) const {
   if (!D) return;
   if (packed) {
-    launch_packed(*this, x, EpiSpmv{dg.p, x, y}, 0, s);
+    launch_packed(*this, x, EpiSpmv{dg.p, x, y}, (unsigned)std::min<uint64_t>((D + 31) / 32, 148 * 256), s);
     return;
   }
   if (on_the_fly)
@@ -934,11 +1074,9 @@ void MixedHamiltonian::apply(const double *x, double *y, cudaStream_t s) const {
 int MixedHamiltonian::apply_full(const double *x, double xs, double *y, const SubList &sub, int red_mask,
                                  Reducer &r, cudaStream_t s, const int *skip) const {
   if (!D) return 0;
-  if (packed)
-    return launch_packed(*this, x, EpiFull{dg.p, x, xs, y, sub, red_mask, r.partials, skip}, red_mask ? r.max_blocks : 0,
-                         s);
   unsigned nb = grid_for(D * 8, 256);
   if (red_mask && nb > (unsigned)r.max_blocks) nb = (unsigned)r.max_blocks;
+  if (packed) return launch_packed(*this, x, EpiFull{dg.p, x, xs, y, sub, red_mask, r.partials, skip}, nb, s);
   if (on_the_fly)
     k_mixed_full<<<nb, 256, 0, s>>>(otf_rows(*this), dg.p, x, xs, y, D, sub, red_mask, r.partials, skip);
   else

@@ -57,13 +57,16 @@ struct MixedTerms {
 MixedTerms mixed_terms(const Model &m, const std::map<std::string, double> &value);
 
 // The packed matrix (see above): slice s holds rows 32 s .. 32 s + 31 and the
-// slots off[s] .. off[s + 1]; slot k's entry of row 32 s + l is ent[32 k + l],
-// column | code << 24 (code == null) or the column alone with its code at
-// code[32 k + l]. Entries come down-spin hops first, so that the rows of a slice,
-// which mostly share their down string, gather the same hop's targets side by
-// side. Code 255 pads short rows and is skipped.
+// slots off[s] .. off[s + 1], up-spin hops in the first up[s] of them, down-spin
+// hops in the others; slot k's entry of row 32 s + l is ent[32 k + l], column |
+// code << 24 (code == null) or the column alone with its code at code[32 k + l].
+// Each part holds a row's entries in the CSR's order, where the up-spin hops come
+// first, row_up[J] of them. The rows of a slice mostly share their down string: with
+// a part of their own its hops stand side by side and gather side by side. Code 255
+// pads short rows and is skipped.
 struct PackedView {
   const uint64_t *off = nullptr;
+  const uint8_t *up = nullptr, *row_up = nullptr;
   const uint32_t *ent = nullptr;
   const uint8_t *code = nullptr;
   const double *values = nullptr;  // 256
@@ -85,7 +88,7 @@ struct MixedHamiltonian {
   bool packed = false;       // the packed form holds the matrix (row_ptr, col, val are empty)
   DevBuf<uint64_t> slice_off;
   DevBuf<uint32_t> ent;
-  DevBuf<uint8_t> code;
+  DevBuf<uint8_t> code, slice_up, row_up;
   DevBuf<double> values;
   bool on_the_fly = false;   // no stored matrix: entries recomputed by every product
   int n_terms = 0;           // off-diagonal one-body elements (kept for the on-the-fly products)
@@ -93,9 +96,11 @@ struct MixedHamiltonian {
   DevBuf<double> term_v;
 
   MixedHamiltonian(const SymmetryGroup &G, const MixedTerms &t, int irrep, int n_up, int n_dn, cudaStream_t s);
-  PackedView packed_view() const { return {slice_off.p, ent.p, code.p, values.p}; }
+  PackedView packed_view() const { return {slice_off.p, slice_up.p, row_up.p, ent.p, code.p, values.p}; }
   // y = H x on device vectors of D doubles, on stream s
   void apply(const double *x, double *y, cudaStream_t s) const;
+  // the same with every sum in the order of the CSR product (the recurrences)
+  void apply_ordered(const double *x, double *y, cudaStream_t s) const;
   // y = xs H x - sum_k sub.c[k] sub.z[k], with the column pass's reductions of
   // the result (red_mask bit 0: <xs x, y>, bit 1: <y, y>, bit 2: <xs x, xs x>)
   // as per-block partials (stride Reducer::kMaxRed); nothing at all when

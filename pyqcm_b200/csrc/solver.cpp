@@ -932,7 +932,7 @@ void lanczos_eigenvector_mixed(const MixedHamiltonian &H, Workspace &ws, const L
   launch_axpby(D, 0.0, psi.p, Z[0], B.p, 0, ws.red, s);
   double *pa = A.p, *pb = B.p, *pc = C.p;
   for (int j = 1; j < M; ++j) {
-    H.apply(pb, pc, s);                                         // H v_{j-1}
+    H.apply_ordered(pb, pc, s);                                 // H v_{j-1}
     launch_axpby(D, 1.0, pc, -alpha[j - 1], pb, 0, ws.red, s);  // - alpha_{j-1} v_{j-1}
     if (j >= 2) launch_axpby(D, 1.0, pc, -beta[j - 2], pa, 0, ws.red, s);  // - beta_{j-2} v_{j-2}
     launch_scale(D, pc, 1.0 / beta[j - 1], s);
