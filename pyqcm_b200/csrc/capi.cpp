@@ -1462,7 +1462,7 @@ int qed_hamiltonian_diag(qed_hamiltonian *h, double *d) {
     H.up->diag.download(du.data(), du.size(), w.stream);
     H.dn->diag.download(dd.data(), dd.size(), w.stream);
     std::vector<double> vin;
-    if (H.op.inter.mode >= 2) {
+    if (H.op.inter.mode == 2 || H.op.inter.mode == 3) {
       vin.resize(H.vinter.n);
       H.vinter.download(vin.data(), vin.size(), w.stream);
     }
@@ -1474,6 +1474,7 @@ int qed_hamiltonian_diag(qed_hamiltonian *h, double *d) {
         double s = du[a] + dd[b];
         const auto &it = H.op.inter;
         if (it.mode == 1) s += it.u * __builtin_popcount(up & dn);
+        else if (it.mode == 4) s += it.sum[__builtin_popcount(up & dn & it.mask)];
         else if (it.mode == 2) { for (int r = 0; r < n; ++r) if ((up & dn) >> r & 1u) s += vin[r]; }
         else if (it.mode == 3) {
           for (int r = 0; r < n; ++r)

@@ -17,6 +17,7 @@
 
 #include "common.hpp"
 #include "options.hpp"
+#include "hv_device.cuh"
 #include "kernels.cuh"
 #include "winhv.hpp"
 
@@ -66,24 +67,6 @@ __device__ __forceinline__ uint32_t colex_unrank(uint32_t I, int L, int N) {
     --p;
   }
   return b;
-}
-
-template <int NRED>
-__device__ __forceinline__ void block_reduce_store(double (&v)[NRED], double *partials, int nred) {
-  __shared__ double sm[NRED > 0 ? NRED : 1][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int i = 0; i < NRED; ++i) {
-    double x = v[i];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sm[i][warp] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x < nred) {
-    double s = 0.0;
-    for (int w = 0; w < nw; ++w) s += sm[threadIdx.x][w];
-    partials[(size_t)blockIdx.x * Reducer::kMaxRed + threadIdx.x] = s;
-  }
 }
 
 __global__ void k_finalize(const double *partials, int nblocks, double *out) {
@@ -212,32 +195,6 @@ __global__ void k_cdag_gather(int L, int spin, int a, int pm, const uint32_t *tu
 }
 
 // ------------------------------------------------------------------ H.v ----
-
-__device__ __forceinline__ double inter_term(const InterSpin &it, uint32_t up, uint32_t dn) {
-  if (it.mode == 1) return it.u * (double)__popc(up & dn);
-  double s = 0.0;
-  if (it.mode == 2) {
-    uint32_t w = up & dn;
-    while (w) {
-      int r = __ffs(w) - 1;
-      s += __ldg(it.v + r);
-      w &= w - 1;
-    }
-  } else if (it.mode == 3) {
-    uint32_t wd = dn;
-    while (wd) {
-      int r = __ffs(wd) - 1;
-      uint32_t wu = up;
-      while (wu) {
-        int c = __ffs(wu) - 1;
-        s += __ldg(it.v + r * it.n + c);
-        wu &= wu - 1;
-      }
-      wd &= wd - 1;
-    }
-  }
-  return s;
-}
 
 // Dense Hamiltonian: thread I writes row I (diagonal, up hops along the row,
 // dn hops across rows), the same matrix elements the H.v passes apply.
@@ -1504,7 +1461,8 @@ constexpr size_t kRowSmem2Max = 220 * 1024;  // below the 227 KB per-CTA limit
 
 // Launch variant of the H.v passes of sectors without the staged kernels (the
 // solver option hv_variant; bit 0: column-pass gathers cached in L2 only; bit 1:
-// row pass with four gathers in flight; bit 2: staged kernels off). Default 2
+// row pass with four gathers in flight; bit 2: staged kernels off; bit 3:
+// one-launch and tiled forms off). Default 2
 // (on the 4x4 sector with the staged kernels off: 5.47 ms per H.v against 5.57 ms
 // for 0). The staged kernels pick their launch shape by timing (below).
 int hv_variant() {
@@ -1542,6 +1500,7 @@ size_t cols16_smem(const HvOperator &op) {
 }
 
 bool staged_disabled() { return (hv_variant() & 4) != 0; }
+bool fused_disabled() { return (hv_variant() & 8) != 0; }
 
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
@@ -1579,7 +1538,7 @@ int hv_cols_grid(const HvOperator &op) {
   const int g = (int)std::max<size_t>(1, std::min<size_t>(nitems, (size_t)device_sms() * 8));
   // the staged pass runs one CTA per column pair, at most one per SM
   const int g16 = (int)std::max<size_t>(1, std::min<size_t>(du / 2, (size_t)device_sms()));
-  return std::max(g, g16);
+  return std::max({g, g16, fused_applies(op) ? fused_grid(op) : 1, tile_applies(op) ? tile_grid(op) : 1});
 }
 
 std::atomic<bool> g_staged_used{false};  // set by the first staged H.v launch
@@ -1801,6 +1760,12 @@ int staged_shape(const HvOperator &op, const double *x, double *y, Reducer &r, s
 int launch_hv_impl(const HvOperator &op, const double *x, double xs, double *y, const SubList &sub, int red_mask,
                    Reducer &r, cudaStream_t s, bool may_tune) {
   if (op.win && window_usable(op, x, y, sub)) return launch_hv_windows(op, x, xs, y, sub, red_mask, r, s);
+  if (!op.keep_order && !fused_disabled()) {
+    bool apart = true;  // the column pass would overwrite a term of the row pass
+    for (int k = 0; k < sub.n; ++k) apart = apart && sub.z[k] != y;
+    if (apart && tile_applies(op)) return launch_hv_tile(op, x, xs, y, sub, red_mask, r, s);
+    if (fused_applies(op)) return launch_hv_fused(op, x, xs, y, sub, red_mask, r, s);
+  }
   const size_t smr = staged_disabled() ? 0 : rows16_smem(op);
   const size_t smc = smr ? cols16_smem(op) : 0;
   bool staged = smr && smc && aligned16(x) && aligned16(y);
@@ -1846,7 +1811,9 @@ void launch_block_hv(const HvOperator &op, int p, const BlockIn &X, const BlockO
   for (int c = 0; c < p && staged; ++c) staged = aligned16(X.v[c]) && aligned16(Y.v[c]);
   if (staged) {  // large sectors: the staged single-vector kernels, one vector at a time
     SubList none;
-    for (int c = 0; c < p; ++c) launch_hv(op, X.v[c], 1.0, Y.v[c], none, 0, r, s);
+    HvOperator ordered = op;
+    ordered.keep_order = true;
+    for (int c = 0; c < p; ++c) launch_hv(ordered, X.v[c], 1.0, Y.v[c], none, 0, r, s);
     return;
   }
   const int grid = grid_for(D, device_sms(), 8);

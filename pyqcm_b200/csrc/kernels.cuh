@@ -24,6 +24,7 @@ struct SpinTable {
   const double *vals = nullptr;
   const double *diag = nullptr;
   uint32_t dim = 0;
+  int width = 0;  // rows of ell (entries past a string's count are undefined)
   int nvals = 0;
   // Packed form of the same hops for the staged-row kernels (null when the
   // table does not fit it; see PackedHops in bank_order.hpp): one list per
@@ -33,16 +34,26 @@ struct SpinTable {
   const uint2 *pk[2] = {nullptr, nullptr};
   const uint8_t *cntw = nullptr;
   double mag[2] = {0.0, 0.0};
+  // The same hops in groups of eight strings for the tiled kernels (null where
+  // they do not apply; see group_hops in solver.hpp).
+  const uint8_t *tile_steps = nullptr;
+  int tile_max = 0;
+  const uint4 *tile_ent = nullptr;
 };
+constexpr uint32_t kTileMinDim = 300, kTileMaxDim = 3468;  // half bases with a grouped copy
 
 // Inter-spin density-density terms sum_{r,s} v[r][s] dn_r up_s.
 //   mode 0: none; 1: diagonal and uniform (u * popc(up & dn));
+//   mode 4: diagonal and uniform on the sites of mask: sum[popc(up & dn & mask)], the
+//   sums u + u + ... as mode 2 would add them (4 u and u + u + u + u may differ);
 //   mode 2: diagonal per site (vdiag[r]); 3: general n x n (vfull, row r = dn bit).
 struct InterSpin {
   int mode = 0;
   int n = 0;
   double u = 0.0;
-  const double *v = nullptr;  // device: n (mode 2) or n*n (mode 3)
+  uint32_t mask = 0;
+  double sum[33] = {};
+  const double *v = nullptr;  // device: n (modes 2 and 4) or n*n (mode 3)
 };
 
 struct HvOperator {
@@ -50,6 +61,14 @@ struct HvOperator {
   InterSpin inter;
   int num_sms = 148;
   const int *skip = nullptr;  // if set and *skip != 0 (device), the H.v passes do nothing
+  // The solver's recurrences set it: the two-pass or staged kernels take the
+  // product, whose sums keep their order. The recurrences stop or deflate at
+  // thresholds, which the last digits of H x can tip: a ground state 1e-8 below the
+  // next level (weakly coupled baths) stops at a residual of 1e-12 with an error of
+  // 1e-4 of that level, a Green function whose lowest level stalls stops a block
+  // earlier or later (G then moved by 5e-6 to 5e-5), band Lanczos deflates where a
+  // norm that vanishes but for round-off crosses 1e-7.
+  bool keep_order = false;
   // host-side binding of the window kernels (WinBinding, winhv.hpp), null when
   // the sector does not use them; device code never reads it
   const void *win = nullptr;
@@ -213,6 +232,21 @@ void launch_hv_cols_rows(const HvOperator &op, const double *x, double xs, doubl
 // row pass and the column pass above.
 int launch_hv(const HvOperator &op, const double *x, double xs, double *y, const SubList &sub, int red_mask,
               Reducer &r, cudaStream_t s);
+// The one-launch form of small sectors (hv_fused.cu).
+// Above kFusedMaxStates one launch no longer beats two (853776 states: 24.4 us
+// against 24.9); below kFusedMinStates the sums keep their order (see keep_order).
+constexpr uint64_t kFusedMinStates = 1024, kFusedMaxStates = 400000;
+bool fused_applies(const HvOperator &op);
+int fused_grid(const HvOperator &op);
+int launch_hv_fused(const HvOperator &op, const double *x, double xs, double *y, const SubList &sub, int red_mask,
+                    Reducer &r, cudaStream_t s);
+// The tiled two-pass form (hv_tile.cu) of half bases that fit shared memory eight
+// vectors wide. From kTileMinStates on (213444 states: 10.5 us, the one-launch form 10.3-14).
+constexpr uint64_t kTileMinStates = 180000;
+bool tile_applies(const HvOperator &op);
+int tile_grid(const HvOperator &op);
+int launch_hv_tile(const HvOperator &op, const double *x, double xs, double *y, const SubList &sub, int red_mask,
+                   Reducer &r, cudaStream_t s);
 // JSON list of the staged H.v launch shapes chosen so far, with the timings
 // that chose them (one entry per (dim_up, dim_dn)).
 std::string hv_tuning_report();

@@ -84,7 +84,7 @@ struct Table {
     i["lanczos_graphs_min_dim"] = 131072;
     // solver option: launch variant of the H.v kernels of sectors without the
     // staged kernels (bits: 1 L2-only column gathers, 2 row pass with four
-    // gathers in flight, 4 staged kernels off); see hv_variant (kernels.cu).
+    // gathers in flight, 4 staged kernels off, 8 one-launch and tiled forms off); see hv_variant (kernels.cu).
     i["hv_variant"] = 2;
     // solver option: spin tables of at most this many strings are built on the
     // host (the same tables as the device build, uploaded at once).

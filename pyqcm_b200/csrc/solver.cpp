@@ -93,9 +93,39 @@ constexpr uint64_t kPackMinDim = 512;
 // device path.
 }  // namespace
 
+void group_hops(const std::vector<uint32_t> &ell, const std::vector<uint8_t> &cnt, uint32_t dim,
+                std::vector<uint8_t> &steps, std::vector<uint32_t> &ent) {
+  const uint32_t ng = (dim + 7) / 8;
+  steps.assign(ng, 0);
+  uint32_t most = 0;
+  for (uint32_t i = 0; i < dim; ++i) {
+    steps[i / 8] = std::max<uint8_t>(steps[i / 8], (uint8_t)((cnt[i] + 1) / 2));
+    most = std::max<uint32_t>(most, steps[i / 8]);
+  }
+  ent.resize((size_t)ng * most * 32);
+  for (size_t q = 0; q < ent.size(); q += 2) {
+    ent[q] = dim * 64;
+    ent[q + 1] = 0;
+  }
+  for (uint32_t i = 0; i < dim; ++i) {
+    uint32_t *own = ent.data() + (size_t)(i / 8) * most * 32 + (i % 8) * 4;
+    uint32_t k = 0;
+    for (uint32_t parity : {i & 1u, 1u - (i & 1u)})
+      for (uint32_t q = 0; q < cnt[i]; ++q) {
+        const uint32_t e = ell[(size_t)q * dim + i];
+        if (((e >> 8) & 1u) != parity) continue;
+        uint32_t *dst = own + (k / 2) * 32 + (k % 2) * 2;
+        dst[0] = (e >> 8) * 64;
+        dst[1] = (e & 255u) * 8;
+        ++k;
+      }
+  }
+}
+
 HostHalf host_half_tables(int L, int N, uint32_t dim, const std::vector<double> &tdiag,
                           const std::vector<double> &vsame, const std::vector<int> &pd, const std::vector<int> &ps,
-                          const std::vector<int> &pslot, const std::vector<double> &vals, int width, bool bank_order) {
+                          const std::vector<int> &pslot, const std::vector<double> &vals, int width, bool bank_order,
+                          bool tiles) {
   HostHalf T;
   std::vector<uint32_t> &hb = T.bits;
   hb.reserve(dim);
@@ -134,6 +164,8 @@ HostHalf host_half_tables(int L, int N, uint32_t dim, const std::vector<double> 
       }
     hd[i] = sd;
   }
+  if (tiles && width > 0 && dim >= kTileMinDim && dim <= kTileMaxDim && vals.size() <= 256)
+    group_hops(he, hc, dim, T.tile_steps, T.tile_ent);
   // the bank-ordered copy: packed for the staged kernels, and the ELL itself for the up spin
   T.vals = vals;
   T.width = width;
@@ -194,8 +226,8 @@ namespace {
 void build_half_host(HalfTables &h, int L, int N, const std::vector<double> &tdiag,
                      const std::vector<double> &vsame, const std::vector<int> &pd, const std::vector<int> &ps,
                      const std::vector<int> &pslot, const std::vector<double> &vals, int width, Workspace &ws,
-                     bool bank_order) {
-  HostHalf T = host_half_tables(L, N, h.dim, tdiag, vsame, pd, ps, pslot, vals, width, bank_order);
+                     bool bank_order, bool tiles) {
+  HostHalf T = host_half_tables(L, N, h.dim, tdiag, vsame, pd, ps, pslot, vals, width, bank_order, tiles);
   h.width = T.width;
   h.nvals = (int)T.vals.size();
   h.bits.upload(T.bits, ws.stream);
@@ -213,12 +245,16 @@ void build_half_host(HalfTables &h, int L, int N, const std::vector<double> &tdi
     h.mag[0] = T.ph.mag[0];
     h.mag[1] = T.ph.mag[1];
   }
+  if (!T.tile_steps.empty()) {
+    h.tile_steps.upload(T.tile_steps, ws.stream);
+    h.tile_ent.upload(T.tile_ent, ws.stream);
+  }
   h.hbits = std::move(T.bits);
   ws.sync();
 }
 
 void build_half(HalfTables &h, int L, int N, const std::vector<double> &t,
-                const std::vector<double> &vsame, Workspace &ws, bool bank_order) {
+                const std::vector<double> &vsame, Workspace &ws, bool bank_order, bool tiles) {
   h.L = L;
   h.N = N;
   uint64_t dim = (N < 0 || N > L) ? 0 : binom(L, N);
@@ -242,7 +278,7 @@ void build_half(HalfTables &h, int L, int N, const std::vector<double> &t,
   // uploaded once (one stream synchronisation instead of five, no kernel
   // launches): a batch of small clusters builds tens of thousands of them.
   if ((long)dim <= opt_int("host_table_max_dim")) {
-    build_half_host(h, L, N, tdiag, vsame, pd, ps, pslot, vals, width, ws, bank_order);
+    build_half_host(h, L, N, tdiag, vsame, pd, ps, pslot, vals, width, ws, bank_order, tiles);
     return;
   }
   h.bits.alloc(dim);
@@ -317,7 +353,11 @@ SpinTable view(const HalfTables &h) {
   s.vals = h.vals.p;
   s.diag = h.diag.p;
   s.dim = h.dim;
+  s.width = h.width;
   s.nvals = h.nvals;
+  s.tile_steps = h.tile_steps.p;
+  s.tile_max = h.tile_steps.n ? (int)(h.tile_ent.n / (32 * h.tile_steps.n)) : 0;
+  s.tile_ent = reinterpret_cast<const uint4 *>(h.tile_ent.p);
   if (h.cntw.n) {
     for (int c = 0; c < 2; ++c) {
       s.pk[c] = reinterpret_cast<const uint2 *>(h.pk[c].p);
@@ -339,7 +379,9 @@ SectorOp::SectorOp(const SpinData &t, const Sector &s, Workspace &ws, HalfCache 
   auto table = [&](int spin, int N) -> std::shared_ptr<const HalfTables> {
     auto make = [&] {
       auto h = std::make_shared<HalfTables>();
-      build_half(*h, L, N, spin ? t.t_dn : t.t_up, spin ? t.v_dd : t.v_uu, ws, spin == 0);
+      // tables shared by an instance's sectors serve the recurrences, which keep the
+      // two-pass and staged kernels (HvOperator::keep_order): no grouped copy
+      build_half(*h, L, N, spin ? t.t_dn : t.t_up, spin ? t.v_dd : t.v_uu, ws, spin == 0, !cache);
       return std::shared_ptr<const HalfTables>(h);
     };
     if (!cache) return make();
@@ -364,16 +406,28 @@ SectorOp::SectorOp(const SpinData &t, const Sector &s, Workspace &ws, HalfCache 
   if (!any) {
     op.inter.mode = 0;
   } else if (!offdiag) {
-    double u0 = t.v_du[0];
+    // one value on some of the sites (U on the cluster, none on the bath) or on all
+    double u0 = 0.0;
+    uint32_t mask = 0;
     bool uniform = true;
-    for (int r = 0; r < n; ++r)
-      if (t.v_du[(size_t)r * n + r] != u0) uniform = false;
-    if (uniform) {
+    std::vector<double> dg(n);
+    for (int r = 0; r < n; ++r) {
+      dg[r] = t.v_du[(size_t)r * n + r];
+      if (dg[r] == 0.0) continue;
+      if (!mask) u0 = dg[r];
+      if (dg[r] != u0) uniform = false;
+      mask |= 1u << r;
+    }
+    if (uniform && mask == (n >= 32 ? 0xffffffffu : (1u << n) - 1u)) {
       op.inter.mode = 1;
       op.inter.u = u0;
+    } else if (uniform) {
+      op.inter.mode = 4;
+      op.inter.mask = mask;
+      for (int r = 1; r <= n; ++r) op.inter.sum[r] = op.inter.sum[r - 1] + u0;
+      vinter.upload(dg, ws.stream);  // the window kernels read the values
+      op.inter.v = vinter.p;
     } else {
-      std::vector<double> dg(n);
-      for (int r = 0; r < n; ++r) dg[r] = t.v_du[(size_t)r * n + r];
       vinter.upload(dg, ws.stream);
       op.inter.mode = 2;
       op.inter.v = vinter.p;
@@ -422,6 +476,7 @@ int KrylovOp::apply(const double *x, double xs, double *y, const SubList &sub, i
   if (mixed) return mixed->apply_full(x, xs, y, sub, red_mask, r, s, skip);
   HvOperator op = fact->op;
   op.skip = skip;
+  op.keep_order = true;
   return launch_hv(op, x, xs, y, sub, red_mask, r, s);
 }
 
@@ -709,6 +764,8 @@ LanczosResult lanczos_energy(const SectorOp &H, Workspace &ws, uint64_t seed) {
   SubList sub;  // w = H v_j - beta_{j-1} v_{j-1}, beta from device memory
   sub.n = 1;
   sub.cdev = ls.beta_prev;
+  HvOperator op = H.op;
+  op.keep_order = true;
   double *pa = A.p, *pb = B.p, *pc = C.p;
   std::vector<double> &alpha = res.alpha, &beta = res.beta;
   double lambda0 = 0.0;
@@ -722,7 +779,7 @@ LanczosResult lanczos_energy(const SectorOp &H, Workspace &ws, uint64_t seed) {
   // rotation by one).
   auto one_step = [&] {
     sub.z[0] = pa;
-    int nb = launch_hv(H.op, pb, 1.0, pc, sub, 1, ws.red, s);
+    int nb = launch_hv(op, pb, 1.0, pc, sub, 1, ws.red, s);
     launch_finalize(ws.red.partials, nb, 1, ls.alpha_cur, s);      // alpha_j = <v_j, w>
     nb = launch_axpy_dev(D, pc, pb, ls.alpha_cur, ws.red, s);      // w -= alpha_j v_j
     launch_finalize(ws.red.partials, nb, 1, ls.b2_cur, s);          // |w|^2
@@ -802,6 +859,8 @@ void lanczos_eigenvector(const SectorOp &H, Workspace &ws, const LanczosResult &
   DevBuf<double> A(D), B(D), C(D);
   start_vector(D, seed, B.p, ws);
   launch_axpby(D, 0.0, psi.p, Z[0], B.p, 0, ws.red, s);
+  HvOperator op = H.op;
+  op.keep_order = true;
   double *pa = A.p, *pb = B.p, *pc = C.p;
   for (int j = 1; j < M; ++j) {
     SubList sub;
@@ -813,7 +872,7 @@ void lanczos_eigenvector(const SectorOp &H, Workspace &ws, const LanczosResult &
       sub.c[1] = beta[j - 2];
       sub.z[1] = pa;
     }
-    launch_hv(H.op, pb, 1.0, pc, sub, 0, ws.red, s);
+    launch_hv(op, pb, 1.0, pc, sub, 0, ws.red, s);
     launch_scale(D, pc, 1.0 / beta[j - 1], s);
     launch_axpby(D, 1.0, psi.p, Z[j], pc, 0, ws.red, s);
     std::swap(pa, pb);

@@ -52,6 +52,9 @@ struct HalfTables {
   DevBuf<uint16_t> pk[2];
   DevBuf<uint8_t> cntw;
   double mag[2] = {0.0, 0.0};
+  // grouped copy for the tiled kernels (empty where they do not apply)
+  DevBuf<uint8_t> tile_steps;
+  DevBuf<uint32_t> tile_ent;
   // the directed hopping pairs (destination r, source c) and their t[r][c]
   std::vector<int> pd, ps;
   std::vector<double> pv;
@@ -75,10 +78,23 @@ struct HostHalf {
   int width = 0;
   PackedHops ph;
   bool packed = false;
+  std::vector<uint8_t> tile_steps;  // grouped copy (group_hops)
+  std::vector<uint32_t> tile_ent;
 };
+// The hops of an ELL table in groups of eight strings for the tiled H.v kernels
+// (hv_tile.cu): group g has steps[g] steps of two entries per string, at most `max`
+// over the groups; the entries of its step j for string 8 g + s are the words
+// ent[((g max + j) 8 + s) 4 ..], per entry the byte offset of its target's tile row (64 bytes per string) and the byte
+// offset of its value (8 per slot). Short lists end in entries aimed at row `dim`,
+// which holds zeros. Even strings list targets of even index first, odd strings
+// those of odd index: the two strings of a pair, which share a phase of the
+// 16-byte gathers, then mostly hit different halves of a 128-byte row.
+void group_hops(const std::vector<uint32_t> &ell, const std::vector<uint8_t> &cnt, uint32_t dim,
+                std::vector<uint8_t> &steps, std::vector<uint32_t> &ent);
 HostHalf host_half_tables(int L, int N, uint32_t dim, const std::vector<double> &tdiag,
                           const std::vector<double> &vsame, const std::vector<int> &pd, const std::vector<int> &ps,
-                          const std::vector<int> &pslot, const std::vector<double> &vals, int width, bool bank_order);
+                          const std::vector<int> &pslot, const std::vector<double> &vals, int width, bool bank_order,
+                          bool tiles = false);
 
 // Per-instance cache of the spin tables: a sector (N_up, N_dn) uses the up
 // table of N_up and the down table of N_dn, so the sectors of one instance

@@ -652,7 +652,7 @@ int launch_hv_windows(const HvOperator &op, const double *x, double xs, double *
   const int *skip = op.skip;
   const double *dup = op.up.diag, *ddn = op.dn.diag, *iv = op.inter.v;
   const uint32_t *bup = op.up.bits, *bdn = op.dn.bits;
-  int imode = op.inter.mode, in = op.inter.n, rm = red_mask;
+  int imode = op.inter.mode == 4 ? 2 : op.inter.mode, in = op.inter.n, rm = red_mask;
   double iu = op.inter.u;
   double *part = r.partials;
   int vec16 = (du % 2 == 0 && ((uintptr_t)x & 15u) == 0) ? 1 : 0;
