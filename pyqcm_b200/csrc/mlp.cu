@@ -37,27 +37,37 @@ inline int pad16(int x) { return (x + 15) / 16 * 16; }
 
 // ---- matrix products on the 5th-generation tensor cores (tcgen05) ----------
 //
-// One CTA of 128 threads computes a 128 x BN tile of C = A B^T (A: M x K, B: N x K,
-// both bf16 with K contiguous) into a TMEM accumulator (fp32, 128 lanes x BN
-// columns). Per round of 64 K-elements the CTA stages the A and B tiles in
-// shared memory with cp.async in the canonical K-major layout without swizzle
-// (8 x 8 core matrices of 128 contiguous bytes, core matrices adjacent in K 128
-// bytes apart, 8-row groups 1024 bytes apart); one elected thread then issues
-// the round's four 128 x BN x 16 tcgen05.mma (kind::f16, bf16 inputs, fp32
-// accumulation) and commits them to an mbarrier, which every thread waits on
-// (bounded) before the tiles are overwritten. The epilogue reads the
-// accumulator back with tcgen05.ld (each warp its 32 lanes = 32 rows).
+// One CTA of 256 threads computes a 128 x bn tile of C = A B^T (A: M x K, B: N x K,
+// bf16) into a TMEM accumulator (fp32, 128 lanes x bn columns). K goes in rounds of
+// 64 through kUmmaStages stages of shared memory, filled with cp.async in the
+// canonical layouts without swizzle, so that an operand may be contiguous along K
+// or along its own rows (the products of the backward pass, which sum over the
+// batch or read W transposed): core matrices of 128 contiguous bytes, eight rows
+// of eight K-elements, or eight K of eight row elements. The rounds' loads are in
+// flight together; one elected thread issues a round's four 128 x bn x 16
+// tcgen05.mma (kind::f16, bf16 inputs, fp32 accumulation) and commits them to the
+// stage's mbarrier, on which the threads wait (bounded) before the stage is filled
+// again. The epilogue reads the accumulator back with tcgen05.ld (warps w and w + 4
+// hold lanes 32 w .. 32 w + 31) and finishes the layer: bias and GELU, or GELU'.
+//
+// At 256 x 256 x 256 (0.03 GFLOP) the latency of one chain - load, multiply, read
+// back - is all there is: a training step was 32 launches with four-CTA products
+// whose rounds waited for one another, 210 us for a batch of 256; with the rounds
+// in flight, 32-column tiles, no transposes and the elementwise work in the
+// epilogues it is eight launches and 72 us. Every sum keeps its
+// order, so that both train to the same bits.
 
 constexpr int kUmmaM = 128;       // rows of a tile = TMEM lanes (cta_group::1)
 constexpr int kUmmaBK = 64;       // K elements staged per round
 constexpr int kUmmaMaxBN = 128;   // columns of a tile
-constexpr int kUmmaThreads = 128;
-constexpr uint32_t kUmmaSbo = kUmmaBK / 8 * 128;  // bytes between 8-row groups
-constexpr uint32_t kUmmaLbo = 128;                // bytes between K-adjacent core matrices
+constexpr int kUmmaThreads = 256;
+constexpr int kUmmaStages = 4;
 constexpr size_t kUmmaTileBytes = (size_t)kUmmaM * kUmmaBK * 2;
-// Dynamic shared memory per CTA: both tiles, the barrier and the TMEM address,
-// rounded up so that at most three CTAs share an SM (3 x 128 TMEM columns <= 512).
-constexpr size_t kUmmaSmem = 72 * 1024;
+// Dynamic shared memory: kUmmaStages of both tiles. At least 72 KB, so that at most
+// three CTAs share an SM (3 x 128 TMEM columns <= 512).
+inline size_t umma_smem(int bn) {
+  return std::max<size_t>(72 * 1024, kUmmaStages * (kUmmaTileBytes + (size_t)bn * kUmmaBK * 2));
+}
 
 // Set when a bounded wait for the tensor core gave up; read by the host.
 __device__ int g_mlp_wait_timeout = 0;
@@ -66,15 +76,17 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)_
 
 // Shared-memory matrix descriptor (sm_100 format): start address, leading and
 // stride byte offsets (all >> 4), descriptor version 1 at bit 46, no swizzle.
-__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((kUmmaLbo >> 4) & 0x3FFFu) << 16) |
-         ((uint64_t)((kUmmaSbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
+         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-// Instruction descriptor of kind::f16: fp32 D (bits 4-5 = 1), bf16 A and B
-// (bits 7-9 and 10-12 = 1), both K-major, N >> 3 at bit 17, M >> 4 at bit 24.
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+// Instruction descriptor of kind::f16: fp32 D (bits 4-5 = 1), bf16 A and B (bits
+// 7-9 and 10-12 = 1), bits 15 and 16 set for an A or B contiguous along its rows,
+// N >> 3 at bit 17, M >> 4 at bit 24.
+__device__ __forceinline__ uint32_t umma_idesc_bf16(int m, int n, int a_mn, int b_mn) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
+         ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, int src_bytes) {
@@ -105,64 +117,108 @@ __device__ __forceinline__ bool umma_wait(uint64_t *bar, uint32_t parity) {
   }
 }
 
-// Stages rows [r0, r0 + rows_tile) x K-elements [k0, k0 + kc) of a row-major
-// bf16 matrix (leading dimension ld) in the canonical layout; rows at or past
-// `rows_total` are zero-filled.
-__device__ __forceinline__ void umma_stage(uint32_t sdst, const bf16 *src, int ld, int r0, int rows_tile,
-                                           int rows_total, int k0, int kc) {
-  const int chunks = kc >> 3;  // 16-byte chunks per row
-  for (int c = threadIdx.x; c < rows_tile * chunks; c += kUmmaThreads) {
-    const int r = c / chunks, q = c - r * chunks;
-    const bool in = r0 + r < rows_total;
-    const bf16 *g = src + (size_t)(in ? r0 + r : 0) * ld + k0 + 8 * q;
-    cp_async16(sdst + (uint32_t)(r >> 3) * kUmmaSbo + (uint32_t)q * kUmmaLbo + (uint32_t)(r & 7) * 16, g,
-               in ? 16 : 0);
+// An operand tile in shared memory: `rows` (a multiple of 16) rows by one round of
+// K. mn: the source is K x rows with the rows contiguous.
+struct UmmaTile {
+  uint32_t lbo, sbo;  // byte strides of the core matrices (descriptor meaning)
+  __device__ UmmaTile(int rows, int mn) : lbo(mn ? (uint32_t)rows / 8 * 128 : 128u), sbo(mn ? 128u : 1024u) {}
+  __device__ uint32_t step() const { return 2 * lbo; }  // 16 K further
+};
+
+// Stages rows [r0, r0 + rows) x K-elements [k0, k0 + kc) of a bf16 operand
+// (leading dimension ld); rows at or past `total` are zero-filled.
+__device__ __forceinline__ void umma_stage(uint32_t sdst, const bf16 *src, int ld, int mn, int r0, int rows,
+                                           int total, int k0, int kc) {
+  if (!mn) {
+    for (int c = threadIdx.x; c < rows * (kUmmaBK / 8); c += kUmmaThreads) {
+      const int r = c >> 3, q = c & 7;
+      if (8 * q >= kc) continue;
+      const bool in = r0 + r < total;
+      cp_async16(sdst + (uint32_t)(r >> 3) * 1024u + (uint32_t)q * 128u + (uint32_t)(r & 7) * 16u,
+                 src + (size_t)(in ? r0 + r : 0) * ld + k0 + 8 * q, in ? 16 : 0);
+    }
+  } else {
+    const int across = rows >> 3;
+    for (int c = threadIdx.x; c < across * kc; c += kUmmaThreads) {
+      const int k = c / across, q = c - k * across;
+      const bool in = r0 + 8 * q < total;
+      cp_async16(sdst + ((uint32_t)(k >> 3) * across + (uint32_t)q) * 128u + (uint32_t)(k & 7) * 16u,
+                 src + (size_t)(k0 + k) * ld + (in ? r0 + 8 * q : 0), in ? 16 : 0);
+    }
   }
 }
 
-// C[M x N] (fp32 row-major, ldc) (+)= A[M x K] B[N x K]^T. A and B are bf16
-// row-major with K contiguous (lda, ldb multiples of 8, 16-byte aligned rows);
-// K a multiple of 16; bn (columns per tile) a multiple of 16 in [16, 128].
-__global__ void __launch_bounds__(kUmmaThreads) k_umma_gemm(int M, int N, int K, const bf16 *__restrict__ A, int lda,
-                                                            const bf16 *__restrict__ B, int ldb, float *__restrict__ C,
-                                                            int ldc, int accumulate, int bn) {
-  extern __shared__ __align__(1024) unsigned char sm[];
-  const uint32_t sa = smem_u32(sm), sb = sa + (uint32_t)kUmmaTileBytes;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(sm + 2 * kUmmaTileBytes);
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 1);
-  const int m0 = blockIdx.x * kUmmaM, n0 = blockIdx.y * bn;
+__device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
+__device__ __forceinline__ float gelu_grad(float z) {
+  return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
+}
+
+// One product and what its epilogue does with C (fp32, row-major, ldc):
+//   kStore:    C
+//   kForward:  C += bias; H = bf16(GELU(C))
+//   kBackward: C *= GELU'(Z); H = bf16(C)
+enum { kStore, kForward, kBackward };
+struct GemmJob {
+  int M = 0, N = 0, K = 0;
+  const bf16 *A = nullptr, *B = nullptr;
+  int lda = 0, ldb = 0, a_mn = 0, b_mn = 0;
+  float *C = nullptr;
+  int ldc = 0, epi = kStore;
+  const float *bias = nullptr, *Z = nullptr;
+  bf16 *H = nullptr;
+  int bn = 16, tiles_n = 0, tiles = 0;
+};
+
+__device__ void umma_tile(const GemmJob &j, int tile, unsigned char *sm) {
+  __shared__ __align__(8) uint64_t bar[kUmmaStages];
+  __shared__ uint32_t tslot;
+  const uint32_t sa = smem_u32(sm), sb = sa + kUmmaStages * (uint32_t)kUmmaTileBytes;
+  const uint32_t b_bytes = (uint32_t)j.bn * kUmmaBK * 2;
+  const int m0 = tile / j.tiles_n * kUmmaM, n0 = tile % j.tiles_n * j.bn;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t ncols = bn <= 32 ? 32u : bn <= 64 ? 64u : 128u;  // a power of two >= 32
+  const uint32_t ncols = j.bn <= 32 ? 32u : j.bn <= 64 ? 64u : 128u;  // a power of two >= 32
+  const int rounds = (j.K + kUmmaBK - 1) / kUmmaBK;
+  auto fill = [&](int r) {
+    const int k0 = r * kUmmaBK, kc = min(kUmmaBK, j.K - k0), st = r % kUmmaStages;
+    umma_stage(sa + st * (uint32_t)kUmmaTileBytes, j.A, j.lda, j.a_mn, m0, kUmmaM, j.M, k0, kc);
+    umma_stage(sb + st * b_bytes, j.B, j.ldb, j.b_mn, n0, j.bn, j.N, k0, kc);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int r = 0; r < min(kUmmaStages, rounds); ++r) fill(r);
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tslot)),
                  "r"(ncols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (threadIdx.x == 32) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
+    for (int st = 0; st < kUmmaStages; ++st)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar[st])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tslot;
-  const uint32_t idesc = umma_idesc_bf16(kUmmaM, bn);
-  uint32_t phase = 0;
+  const uint32_t tmem = tslot;
+  const uint32_t idesc = umma_idesc_bf16(kUmmaM, j.bn, j.a_mn, j.b_mn);
+  const UmmaTile ta(kUmmaM, j.a_mn), tb(j.bn, j.b_mn);
   bool ok = true;
-  for (int k0 = 0; k0 < K; k0 += kUmmaBK) {
-    const int kc = min(kUmmaBK, K - k0);
-    umma_stage(sa, A, lda, m0, kUmmaM, M, k0, kc);
-    umma_stage(sb, B, ldb, n0, bn, N, k0, kc);
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+  for (int r = 0; r < rounds && ok; ++r) {
+    const int st = r % kUmmaStages, kc = min(kUmmaBK, j.K - r * kUmmaBK);
+    switch (min(rounds, r + kUmmaStages) - (r + 1)) {  // rounds that may still be in flight
+      case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+      case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+      case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+      default: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the tensor core's reads
     __syncthreads();
     if (threadIdx.x == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       for (int kk = 0; kk < kc / 16; ++kk) {
-        const uint64_t ad = umma_smem_desc(sa + 2u * kUmmaLbo * (uint32_t)kk);
-        const uint64_t bd = umma_smem_desc(sb + 2u * kUmmaLbo * (uint32_t)kk);
-        const uint32_t acc = (k0 > 0 || kk > 0) ? 1u : 0u;
+        const uint64_t ad = umma_smem_desc(sa + st * (uint32_t)kUmmaTileBytes + ta.step() * (uint32_t)kk, ta.lbo, ta.sbo);
+        const uint64_t bd = umma_smem_desc(sb + st * b_bytes + tb.step() * (uint32_t)kk, tb.lbo, tb.sbo);
+        const uint32_t acc = (r > 0 || kk > 0) ? 1u : 0u;
         asm volatile(
             "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
             " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
@@ -170,34 +226,57 @@ __global__ void __launch_bounds__(kUmmaThreads) k_umma_gemm(int M, int N, int K,
             : "memory");
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       smem_u32(bar))
+                       smem_u32(&bar[st]))
                    : "memory");
     }
-    ok = __syncthreads_and(umma_wait(bar, phase));  // the MMAs have read the tiles
-    phase ^= 1u;
-    if (!ok) break;
+    if (r + kUmmaStages < rounds) {  // the MMAs have read the stage: fill it again
+      ok = __syncthreads_and(umma_wait(&bar[st], (uint32_t)(r / kUmmaStages) & 1u));
+      if (ok) fill(r + kUmmaStages);
+    } else if (r + 1 == rounds) {  // the last commit covers every MMA
+      ok = __syncthreads_and(umma_wait(&bar[st], (uint32_t)(r / kUmmaStages) & 1u));
+    }
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (ok) {
-    const int row = m0 + warp * 32 + lane;
-    for (int c0 = 0; c0 < bn; c0 += 16) {
+    const int row = m0 + (warp & 3) * 32 + lane;
+    for (int c0 = (warp >> 2) * 16; c0 < j.bn; c0 += 32) {
       uint32_t v[16];
       asm volatile(
           "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
           "%14, %15}, [%16];"
           : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
             "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0));
+          : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0));
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (row < M) {
-        float *crow = C + (size_t)row * ldc + n0 + c0;
+      const int n = n0 + c0;  // N and n are multiples of 16: the chunk is inside or outside as a whole
+      if (row < j.M && n < j.N) {
+        const size_t at = (size_t)row * j.ldc + n;
+        float c[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (n0 + c0 + j < N) crow[j] = (accumulate ? crow[j] : 0.0f) + __uint_as_float(v[j]);
+        for (int q = 0; q < 16; ++q) c[q] = 0.0f + __uint_as_float(v[q]);
+        if (j.epi == kForward) {
+#pragma unroll
+          for (int q = 0; q < 16; ++q) c[q] = c[q] + j.bias[n + q];
+        } else if (j.epi == kBackward) {
+#pragma unroll
+          for (int q = 0; q < 16; ++q) c[q] = c[q] * gelu_grad(j.Z[at + q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 16; q += 4)
+          *reinterpret_cast<float4 *>(j.C + at + q) = make_float4(c[q], c[q + 1], c[q + 2], c[q + 3]);
+        if (j.epi != kStore) {
+          __align__(16) bf16 h[16];
+#pragma unroll
+          for (int q = 0; q < 16; ++q) h[q] = __float2bfloat16_rn(j.epi == kForward ? gelu(c[q]) : c[q]);
+          reinterpret_cast<uint4 *>(j.H + at)[0] = reinterpret_cast<const uint4 *>(h)[0];
+          reinterpret_cast<uint4 *>(j.H + at)[1] = reinterpret_cast<const uint4 *>(h)[1];
+        }
       }
     }
   } else {
-    umma_wait(bar, phase ^ 1u);  // a commit still in flight has had its bounded chance to land
+    for (int st = 0; st < kUmmaStages; ++st)  // commits still in flight have their bounded chance to land
+      if (st < rounds) umma_wait(&bar[st], (uint32_t)((rounds - 1 - st) / kUmmaStages) & 1u);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -205,31 +284,72 @@ __global__ void __launch_bounds__(kUmmaThreads) k_umma_gemm(int M, int N, int K,
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
 }
 
-// out[c][r] = in[r][c] for an R x Cn bf16 matrix (leading dimensions ld_in, ld_out).
-__global__ void k_transpose_bf16(int R, int Cn, const bf16 *__restrict__ in, int ld_in, bf16 *__restrict__ out,
-                                 int ld_out) {
-  __shared__ bf16 t[32][34];
-  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int r = r0 + i, c = c0 + threadIdx.x;
-    t[i][threadIdx.x] = (r < R && c < Cn) ? in[(size_t)r * ld_in + c] : __float2bfloat16_rn(0.0f);
+// out[f] = sum_b w[b] X[b][f] over rows b in order (w null: 1), F columns of an
+// fp32 or bf16 matrix: a CTA takes 32 columns, stages 256 rows at a time in shared
+// memory and a thread per column adds them up (the order of the sums is the rows',
+// so only the loads can be spread).
+struct ColJob {
+  int rows = 0, F = 0;
+  const float *X = nullptr;
+  const bf16 *Xh = nullptr;
+  const float *w = nullptr;
+  float *out = nullptr;
+  int ctas = 0;  // 0: no job
+};
+constexpr int kColRows = 256;
+
+__device__ void column_sums(const ColJob &j, int cta, float *sm) {
+  const int f0 = cta * 32, lane = threadIdx.x & 31, f = f0 + lane;
+  float *wr = sm + kColRows * 32;
+  float s = 0.0f;
+  for (int b0 = 0; b0 < j.rows; b0 += kColRows) {
+    const int n = min(kColRows, j.rows - b0);
+    if (b0) __syncthreads();
+    for (int r = threadIdx.x >> 5; r < n; r += kUmmaThreads / 32) {
+      const size_t at = (size_t)(b0 + r) * j.F + f;
+      if (f < j.F) sm[r * 32 + lane] = j.Xh ? __bfloat162float(j.Xh[at]) : j.X[at];
+    }
+    if ((int)threadIdx.x < n) wr[threadIdx.x] = j.w ? j.w[b0 + threadIdx.x] : 1.0f;
+    __syncthreads();
+    if (threadIdx.x < 32 && f < j.F) {
+#pragma unroll 16
+      for (int r = 0; r < n; ++r) s = fmaf(sm[r * 32 + lane], wr[r], s);
+    }
   }
-  __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int c = c0 + i, r = r0 + threadIdx.x;
-    if (c < Cn && r < R) out[(size_t)c * ld_out + r] = t[threadIdx.x][i];
-  }
+  if (threadIdx.x < 32 && f < j.F) j.out[f] = s;
 }
 
-void transpose(int R, int Cn, const bf16 *in, int ld_in, bf16 *out, int ld_out, cudaStream_t s) {
-  k_transpose_bf16<<<dim3((Cn + 31) / 32, (R + 31) / 32), dim3(32, 8), 0, s>>>(R, Cn, in, ld_in, out, ld_out);
-  QED_LAUNCH();
+// The products and column sums of one stage of the network (all independent).
+struct StageJobs {
+  GemmJob g[2];
+  ColJob c[3];
+};
+__global__ void __launch_bounds__(kUmmaThreads) k_mlp_stage(const __grid_constant__ StageJobs jobs) {
+  extern __shared__ __align__(1024) unsigned char sm[];
+  int cta = blockIdx.x;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (cta < jobs.g[i].tiles) {
+      umma_tile(jobs.g[i], cta, sm);
+      return;
+    }
+    cta -= jobs.g[i].tiles;
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    if (cta < jobs.c[i].ctas) {
+      column_sums(jobs.c[i], cta, reinterpret_cast<float *>(sm));
+      return;
+    }
+    cta -= jobs.c[i].ctas;
+  }
 }
 
 void umma_setup() {
   static bool done = false;  // the attribute is per function, once per process is enough
   if (!done) {
-    QED_CUDA(cudaFuncSetAttribute(k_umma_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUmmaSmem));
+    QED_CUDA(cudaFuncSetAttribute(k_mlp_stage, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)umma_smem(kUmmaMaxBN)));
     done = true;
   }
 }
@@ -247,104 +367,76 @@ void check_umma_wait(cudaStream_t s) {
   }
 }
 
-// C[M x N] (+)= A B^T on the tensor cores, A: M x K, B: N x K (K contiguous).
-void gemm_tn(int M, int N, int K, const bf16 *A, int lda, const bf16 *B, int ldb, float *C, int ldc, bool acc,
-             cudaStream_t s) {
+// The product C = A B^T of one stage: checked, with its tile width - the widest
+// that still gives every SM a tile, at least 32 columns (256 x 256 x 256 in 16
+// tiles of 32 columns; 4 of 128 left 144 SMs idle).
+GemmJob gemm_job(int M, int N, int K, const bf16 *A, int lda, bool a_mn, const bf16 *B, int ldb, bool b_mn, float *C,
+                 int ldc) {
   if (M <= 0 || N <= 0 || K <= 0 || K % 16 || N % 16 || lda % 8 || ldb % 8)
     fail(QED_ERR_ARGUMENT, "mlp: tensor-core product needs K and N multiples of 16 and 16-byte rows");
-  const int bn = std::min(N, kUmmaMaxBN);
-  dim3 grid((M + kUmmaM - 1) / kUmmaM, (N + bn - 1) / bn);
-  k_umma_gemm<<<grid, kUmmaThreads, kUmmaSmem, s>>>(M, N, K, A, lda, B, ldb, C, ldc, acc ? 1 : 0, bn);
+  GemmJob j;
+  j.M = M;
+  j.N = N;
+  j.K = K;
+  j.A = A;
+  j.lda = lda;
+  j.a_mn = a_mn;
+  j.B = B;
+  j.ldb = ldb;
+  j.b_mn = b_mn;
+  j.C = C;
+  j.ldc = ldc;
+  const int tiles_m = (M + kUmmaM - 1) / kUmmaM;
+  j.bn = std::min(N, kUmmaMaxBN);
+  while (j.bn >= 64 && j.bn % 32 == 0 && tiles_m * ((N + j.bn - 1) / j.bn) < 148) j.bn /= 2;
+  j.tiles_n = (N + j.bn - 1) / j.bn;
+  j.tiles = tiles_m * j.tiles_n;
+  return j;
+}
+
+ColJob col_job(int rows, int F, const float *X, const bf16 *Xh, const float *w, float *out) {
+  return {rows, F, X, Xh, w, out, (F + 31) / 32};
+}
+
+void run_stage(const StageJobs &jobs, cudaStream_t s) {
+  size_t smem = (kColRows * 32 + kColRows) * sizeof(float);
+  int grid = 0;
+  for (const GemmJob &j : jobs.g) {
+    if (j.tiles) smem = std::max(smem, umma_smem(j.bn));
+    grid += j.tiles;
+  }
+  for (const ColJob &j : jobs.c) grid += j.ctas;
+  k_mlp_stage<<<grid, kUmmaThreads, smem, s>>>(jobs);
   QED_LAUNCH();
 }
 
-// C[M x N] (fp32, row-major, ldc) (+)= op(A) op(B), op(A) M x K, op(B) K x N.
-// TA: A stored K x M, else M x K row-major. TB: B stored N x K, else K x N
-// row-major. Operands not already K-contiguous are transposed into the
-// scratch buffers ta / tb first (each at least M*K / N*K elements).
-template <bool TA, bool TB>
-void gemm(int M, int N, int K, const bf16 *A, int lda, const bf16 *B, int ldb, float *C, int ldc, bool acc,
-          bf16 *ta, bf16 *tb, cudaStream_t s) {
-  if (TA) {
-    transpose(K, M, A, lda, ta, K, s);
-    A = ta;
-    lda = K;
-  }
-  if (!TB) {
-    transpose(K, N, B, ldb, tb, K, s);
-    B = tb;
-    ldb = K;
-  }
-  gemm_tn(M, N, K, A, lda, B, ldb, C, ldc, acc, s);
-}
-
-__device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float z) {
-  return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
-}
-
-// Z[b][f] += bias[f]; H = bf16(GELU(Z))
-__global__ void k_bias_gelu(int rows, int F, float *Z, const float *bias, bf16 *H) {
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)rows * F; t += (size_t)gridDim.x * blockDim.x) {
-    const float z = Z[t] + bias[t % F];
-    Z[t] = z;
-    H[t] = __float2bfloat16_rn(gelu(z));
-  }
-}
-
-// y[b] = sum_k H[b][k] w[k] + b0 (fp32 accumulation), one warp per row
-__global__ void k_head(int rows, int F, const bf16 *H, const bf16 *w, const float *b0, float *y) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x % 32;
-  if (warp >= rows) return;
+// The output layer, one warp per row b: y = sum_k H[b][k] w[k] + b0 (fp32
+// accumulation) and, with targets, the loss terms (y - t)^2 / n, dy = 2 (y - t) / n
+// and dZ[b][k] = dy w[k] GELU'(Z[b][k]) (fp32 and bf16 copies). step, if given, is
+// the optimiser's step count, advanced here once per training step.
+__global__ void k_head(int rows, int F, const bf16 *H, const bf16 *w, const float *b0, float *y, const float *t,
+                       float *dy, float *loss_terms, const float *Z, float *dZ, bf16 *dZh, int *step) {
+  if (step && blockIdx.x == 0 && threadIdx.x == 0) *step += 1;
+  const int b = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x % 32;
+  if (b >= rows) return;
   float s = 0.0f;
-  for (int k = lane; k < F; k += 32) s += __bfloat162float(H[(size_t)warp * F + k]) * __bfloat162float(w[k]);
+  for (int k = lane; k < F; k += 32) s += __bfloat162float(H[(size_t)b * F + k]) * __bfloat162float(w[k]);
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) y[warp] = s + b0[0];
-}
-
-// dy = 2 (y - t) / n and the loss terms (y - t)^2 / n per row
-__global__ void k_mse(int rows, const float *y, const float *t, float *dy, float *loss_terms) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows) return;
-  const float d = y[i] - t[i];
-  dy[i] = 2.0f * d / rows;
-  loss_terms[i] = d * d / rows;
-}
-
-// head backward: dZ[b][k] = dy[b] w[k] GELU'(Z[b][k]) (fp32 and bf16 copies)
-__global__ void k_head_back(int rows, int F, const float *dy, const bf16 *w, const float *Z, float *dZ, bf16 *dZh) {
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)rows * F; t += (size_t)gridDim.x * blockDim.x) {
-    const float g = dy[t / F] * __bfloat162float(w[t % F]) * gelu_grad(Z[t]);
-    dZ[t] = g;
-    dZh[t] = __float2bfloat16_rn(g);
+  const float yb = s + b0[0];
+  if (lane == 0) y[b] = yb;
+  if (!t) return;
+  const float d = yb - t[b];
+  const float g = 2.0f * d / rows;
+  if (lane == 0) {
+    dy[b] = g;
+    loss_terms[b] = d * d / rows;
   }
-}
-
-// dZ = dH GELU'(Z) in place (fp32) plus a bf16 copy
-__global__ void k_gelu_back(int rows, int F, float *dH, const float *Z, bf16 *dZh) {
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)rows * F; t += (size_t)gridDim.x * blockDim.x) {
-    const float g = dH[t] * gelu_grad(Z[t]);
-    dH[t] = g;
-    dZh[t] = __float2bfloat16_rn(g);
+  for (int k = lane; k < F; k += 32) {
+    const size_t at = (size_t)b * F + k;
+    const float z = g * __bfloat162float(w[k]) * gelu_grad(Z[at]);
+    dZ[at] = z;
+    dZh[at] = __float2bfloat16_rn(z);
   }
-}
-
-// out[f] = sum_b X[b][f] * (wrow ? wrow[b] : 1), fixed order, one thread per column
-__global__ void k_colsum(int rows, int F, const float *X, const float *wrow, float *out) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= F) return;
-  float s = 0.0f;
-  for (int b = 0; b < rows; ++b) s += X[(size_t)b * F + f] * (wrow ? wrow[b] : 1.0f);
-  out[f] = s;
-}
-
-// head weight gradient: g[k] = sum_b dy[b] H[b][k]
-__global__ void k_head_wgrad(int rows, int F, const float *dy, const bf16 *H, float *g) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= F) return;
-  float s = 0.0f;
-  for (int b = 0; b < rows; ++b) s += dy[b] * __bfloat162float(H[(size_t)b * F + k]);
-  g[k] = s;
 }
 
 // Adam (Kingma & Ba 2015, Algorithm 1) on fp32 master weights; the step count
@@ -365,8 +457,6 @@ __global__ void k_adam(int n, float *w, const float *g, float *m, float *v, bf16
   w[i] = wi;
   if (wh) wh[i] = __float2bfloat16_rn(wi);
 }
-
-__global__ void k_incr(int *step) { *step += 1; }
 
 __global__ void k_to_bf16(int n, const float *x, bf16 *y) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -406,8 +496,6 @@ struct MLP {
   int cap = 0;
   DevBuf<bf16> X, H[3], dZh[3];
   DevBuf<float> T, Z[3], dZ[3], y, dy, lt;
-  DevBuf<float> tmp;
-  DevBuf<bf16> ta, tb;  // transposed operands of the backward products
   DevBuf<int> perm;
   DevBuf<float> data_x, data_t;
   int n_data = 0;
@@ -510,54 +598,59 @@ struct MLP {
     y.alloc(cap);
     dy.alloc(cap);
     lt.alloc(cap);
-    tmp.alloc((size_t)cap * 16);
-    ta.alloc((size_t)W * std::max(cap, W));
-    tb.alloc((size_t)W * std::max(cap, W));
   }
 
-  // forward on rows [0, rows) of X (bf16, padded); y = network output
-  void forward(int rows) {
-    const bf16 *in = X.p;
-    int kin = k_in;
+  // hidden layers on rows [0, rows) of X (bf16, padded)
+  void hidden(int rows) {
     for (int l = 0; l < 3; ++l) {
-      gemm_tn(rows, W, kin, in, kin, Ph(2 * l), kin, Z[l].p, W, false, s);
-      k_bias_gelu<<<blocks_for((size_t)rows * W), 256, 0, s>>>(rows, W, Z[l].p, P(2 * l + 1), H[l].p);
-      QED_LAUNCH();
-      in = H[l].p;
-      kin = W;
+      const int kin = l ? W : k_in;
+      StageJobs st;
+      GemmJob &j = st.g[0];
+      j = gemm_job(rows, W, kin, l ? H[l - 1].p : X.p, kin, false, Ph(2 * l), kin, false, Z[l].p, W);
+      j.epi = kForward;
+      j.bias = P(2 * l + 1);
+      j.H = H[l].p;
+      run_stage(st, s);
     }
-    k_head<<<(rows * 32 + 255) / 256, 256, 0, s>>>(rows, W, H[2].p, Ph(6), P(7), y.p);
+  }
+
+  // y = network output
+  void forward(int rows) {
+    hidden(rows);
+    k_head<<<(rows * 32 + 255) / 256, 256, 0, s>>>(rows, W, H[2].p, Ph(6), P(7), y.p, nullptr, nullptr, nullptr,
+                                                  nullptr, nullptr, nullptr, nullptr);
     QED_LAUNCH();
   }
 
-  // gradients of the mean squared error over rows [0, rows) into g
-  void backward(int rows) {
-    k_mse<<<(rows + 255) / 256, 256, 0, s>>>(rows, y.p, T.p, dy.p, lt.p);
-    QED_LAUNCH();
-    k_head_wgrad<<<(W + 255) / 256, 256, 0, s>>>(rows, W, dy.p, H[2].p, Gr(6));
-    QED_LAUNCH();
-    k_colsum<<<1, 32, 0, s>>>(rows, 1, dy.p, nullptr, Gr(7));
-    QED_LAUNCH();
-    k_head_back<<<blocks_for((size_t)rows * W), 256, 0, s>>>(rows, W, dy.p, Ph(6), Z[2].p, dZ[2].p, dZh[2].p);
+  // forward and the gradients of the mean squared error over rows [0, rows) into g.
+  // Three launches forward, the output layer, and one per layer backward: dW_l =
+  // dZ_l^T prev, db_l and dZ_{l-1} = dZ_l W_l GELU'(Z_{l-1}) all read dZ_l only.
+  void gradients(int rows, bool training) {
+    hidden(rows);
+    k_head<<<(rows * 32 + 255) / 256, 256, 0, s>>>(rows, W, H[2].p, Ph(6), P(7), y.p, T.p, dy.p, lt.p, Z[2].p,
+                                                  dZ[2].p, dZh[2].p, training ? step.p : nullptr);
     QED_LAUNCH();
     for (int l = 2; l >= 0; --l) {
-      const bf16 *prev = l > 0 ? H[l - 1].p : X.p;
-      const int kin = l > 0 ? W : k_in;
-      // dW_l [W][kin] = dZ_l^T prev ; db_l = column sums of dZ_l
-      gemm<true, false>(W, kin, rows, dZh[l].p, W, prev, kin, Gr(2 * l), kin, false, ta.p, tb.p, s);
-      k_colsum<<<(W + 255) / 256, 256, 0, s>>>(rows, W, dZ[l].p, nullptr, Gr(2 * l + 1));
-      QED_LAUNCH();
-      if (l > 0) {  // dH_{l-1} = dZ_l W_l, then through GELU'
-        gemm<false, false>(rows, W, W, dZh[l].p, W, Ph(2 * l), W, dZ[l - 1].p, W, false, ta.p, tb.p, s);
-        k_gelu_back<<<blocks_for((size_t)rows * W), 256, 0, s>>>(rows, W, dZ[l - 1].p, Z[l - 1].p, dZh[l - 1].p);
-        QED_LAUNCH();
+      const int kin = l ? W : k_in;
+      StageJobs st;
+      if (l > 0) {
+        GemmJob &j = st.g[0];
+        j = gemm_job(rows, W, W, dZh[l].p, W, false, Ph(2 * l), W, true, dZ[l - 1].p, W);
+        j.epi = kBackward;
+        j.Z = Z[l - 1].p;
+        j.H = dZh[l - 1].p;
       }
+      st.g[1] = gemm_job(W, kin, rows, dZh[l].p, W, true, l ? H[l - 1].p : X.p, kin, true, Gr(2 * l), kin);
+      st.c[0] = col_job(rows, W, dZ[l].p, nullptr, nullptr, Gr(2 * l + 1));
+      if (l == 2) {  // the output layer's weights and bias
+        st.c[1] = col_job(rows, W, nullptr, H[2].p, dy.p, Gr(6));
+        st.c[2] = col_job(rows, 1, dy.p, nullptr, nullptr, Gr(7));
+      }
+      run_stage(st, s);
     }
   }
 
   void adam(float lr) {
-    k_incr<<<1, 1, 0, s>>>(step.p);
-    QED_LAUNCH();
     k_adam<<<blocks_for(n_par), 256, 0, s>>>((int)n_par, p.p, g.p, m.p, v.p, ph.p, step.p, lr, 0.9f, 0.999f,
                                               1e-8f, mask.p);
     QED_LAUNCH();
@@ -661,8 +754,7 @@ int qed_mlp_gradients(void *handle, int rows, const float *x, const float *t, fl
     MLP &h = *static_cast<MLP *>(handle);
     if (rows <= 0 || rows % 16) qed::fail(QED_ERR_ARGUMENT, "mlp: gradient batches are a positive multiple of 16 rows");
     h.load_rows(rows, x, t);
-    h.forward(rows);
-    h.backward(rows);
+    h.gradients(rows, false);
     std::vector<float> lt(rows);
     QED_CUDA(cudaMemcpyAsync(grads, h.g.p, h.n_par * sizeof(float), cudaMemcpyDeviceToHost, h.s));
     QED_CUDA(cudaMemcpyAsync(lt.data(), h.lt.p, rows * sizeof(float), cudaMemcpyDeviceToHost, h.s));
@@ -701,8 +793,7 @@ int qed_mlp_train(void *handle, int rows, const float *x, const float *t, int ep
         for (int st = 0; st < steps; ++st) {
           h.X.p = X0 + (size_t)st * batch * h.k_in;  // views into the gathered rows
           h.T.p = T0 + (size_t)st * batch;
-          h.forward(batch);
-          h.backward(batch);
+          h.gradients(batch, true);
           h.adam(lr);
         }
       } catch (...) {
@@ -766,7 +857,9 @@ int qed_mlp_tensor_product(int M, int N, int K, const uint16_t *A, const uint16_
     QED_CUDA(cudaStreamSynchronize(qed::alloc_stream()));  // the allocations are usable on s
     a.upload(reinterpret_cast<const bf16 *>(A), (size_t)M * K, s);
     b.upload(reinterpret_cast<const bf16 *>(B), (size_t)N * K, s);
-    qed::gemm_tn(M, N, K, a.p, K, b.p, K, c.p, N, false, s);
+    qed::StageJobs st;
+    st.g[0] = qed::gemm_job(M, N, K, a.p, K, false, b.p, K, false, c.p, N);
+    qed::run_stage(st, s);
     c.download(C, (size_t)M * N, s);
     qed::check_umma_wait(s);
   });
