@@ -586,16 +586,98 @@ void Instance::state_vector(State &st, Workspace &ws) {
 // (HS_Hermitian_operator::expectation_value, src_ed/Operators/HS_Hermitian_operator.hpp:46-52),
 // variance = second - first^2; operators on cluster orbitals only (target 1)
 // are scaled by norm = 1/n_sites (-1/n_sites for "mu"), Hermitian_operator.hpp:41-43.
-// O psi is one H.v with the operator's own tables and the <x,y>, <y,y>
-// reductions of the column pass.
+// Sectors of at most kAverageMaxStates states take every operator in one launch
+// that works from the strings (launch_op_averages): building the two spin tables of
+// each operator costs the host about half a millisecond, 10 ms for the 19 operators
+// of the plaquette with eight bath orbitals, where the one launch takes 0.1. In
+// larger sectors O psi is one H.v with the operator's own tables and the <x,y>,
+// <y,y> reductions of the column pass: ranking every hop's string anew would cost
+// more there than the tables save.
+constexpr size_t kAverageMaxStates = 1u << 22;
+
+static void one_pass_averages(const Model &m, const std::map<std::string, double> &value, const SectorOp &H,
+                              const double *psi, std::vector<double> &out, Workspace &ws) {
+  const int n = m.n_orb, nop = (int)value.size();
+  std::vector<int> doff(1, 0), hoff(1, 0);
+  std::vector<uint2> dterm;
+  std::vector<int3> hop;
+  std::vector<double> dval, hval;
+  for (auto &v : value) {
+    const SpinData t = collect_terms(m, {{v.first, 1.0}});
+    auto density = [&](uint32_t up, uint32_t dn, double x) {
+      if (x == 0.0) return;
+      dterm.push_back(make_uint2(up, dn));
+      dval.push_back(x);
+    };
+    for (int r = 0; r < n; ++r) {
+      density(1u << r, 0u, t.t_up[(size_t)r * n + r]);
+      density(0u, 1u << r, t.t_dn[(size_t)r * n + r]);
+      for (int c = 0; c < n; ++c) {
+        if (c >= r) {
+          density(1u << r | 1u << c, 0u, t.v_uu[(size_t)r * n + c]);
+          density(0u, 1u << r | 1u << c, t.v_dd[(size_t)r * n + c]);
+        }
+        density(1u << c, 1u << r, t.v_du[(size_t)r * n + c]);
+      }
+    }
+    for (int spin = 0; spin < 2; ++spin) {
+      std::vector<int> pd, ps, slot;
+      std::vector<double> vals;
+      hop_pairs(n, spin ? t.t_dn : t.t_up, pd, ps, slot, vals);
+      for (size_t q = 0; q < pd.size(); ++q) {
+        hop.push_back(make_int3(spin, pd[q], ps[q]));
+        hval.push_back(vals[slot[q]]);
+      }
+    }
+    doff.push_back((int)dterm.size());
+    hoff.push_back((int)hop.size());
+  }
+  auto atleast = [](auto &v) { if (v.empty()) v.resize(1); };
+  atleast(dterm);
+  atleast(dval);
+  atleast(hop);
+  atleast(hval);
+  DevBuf<int> ddoff, dhoff;
+  DevBuf<uint2> ddterm;
+  DevBuf<int3> dhop;
+  DevBuf<double> ddval, dhval, part(2 * (size_t)nop * op_average_blocks(H.D)), res(2 * (size_t)nop);
+  ddoff.upload(doff, ws.stream);
+  dhoff.upload(hoff, ws.stream);
+  ddterm.upload(dterm, ws.stream);
+  ddval.upload(dval, ws.stream);
+  dhop.upload(hop, ws.stream);
+  dhval.upload(hval, ws.stream);
+  launch_op_averages(nop, OpTerms{ddoff.p, dhoff.p, ddterm.p, ddval.p, dhop.p, dhval.p}, H.up->bits.p, H.up->dim,
+                     H.dn->bits.p, H.dn->dim, psi, part.p, res.p, ws.stream);
+  out.resize(2 * (size_t)nop);
+  res.download(out.data(), out.size(), ws.stream);
+  ws.sync();
+}
+
 void Instance::finish_gs(Workspace &ws) {
   PhaseScope ps(kPhAverages);
   averages.clear();
+  // one_pass[i]: (<O>, |O psi|^2) of every operator in state i, empty where the
+  // operators' own tables are used
+  std::vector<std::vector<double>> one_pass(states.size());
+  for (size_t i = 0; i < states.size() && !has_group(); ++i) {
+    const Sector &sec = states[i]->sec;
+    if (sector_dim(sec) == 0 || sector_dim(sec) > kAverageMaxStates || model->n_orb > 32) continue;
+    const SectorOp H(terms, sec, ws, &tables);
+    one_pass_averages(*model, value, H, states[i]->psi.p, one_pass[i], ws);
+  }
+  size_t k = 0;
   for (auto &v : value) {
     const Operator &op = *model->term.at(v.first);
     const SpinData t = collect_terms(*model, {{v.first, 1.0}});
     double ave = 0.0, var = 0.0;
-    for (auto &st : states) {
+    for (size_t i = 0; i < states.size(); ++i) {
+      auto &st = states[i];
+      if (!one_pass[i].empty()) {
+        ave += st->weight * one_pass[i][2 * k];
+        var += st->weight * one_pass[i][2 * k + 1];
+        continue;
+      }
       SubList none;
       if (has_group()) {  // the operator in the state's symmetry-adapted basis
         MixedHamiltonian O(*model->group, mixed_terms(*model, {{v.first, 1.0}}), st->sec.irrep, st->sec.Nup(),
@@ -616,6 +698,7 @@ void Instance::finish_gs(Workspace &ws) {
       ave += st->weight * r[0];
       var += st->weight * r[1];
     }
+    ++k;
     var -= ave * ave;
     if (op.target == 1) {
       const double norm = (v.first == "mu" ? -1.0 : 1.0) / model->n_sites;

@@ -84,6 +84,21 @@ __global__ void k_finalize(const double *partials, int nblocks, double *out) {
   if (threadIdx.x == 0) out[slot] = sm[0];
 }
 
+// out[2 k + i] = sum over blocks b < nblocks of partials[(k nblocks + b) 2 + i]
+__global__ void k_pair_sums(const double *partials, int nblocks, double *out) {
+  __shared__ double sm[64];
+  const int i = threadIdx.x & 1;
+  double s = 0.0;
+  for (int b = threadIdx.x >> 1; b < nblocks; b += 32) s += partials[((size_t)blockIdx.x * nblocks + b) * 2 + i];
+  sm[threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    double t = 0.0;
+    for (int q = 0; q < 32; ++q) t += sm[2 * q + threadIdx.x];
+    out[2 * blockIdx.x + threadIdx.x] = t;
+  }
+}
+
 int grid_for(size_t n, int num_sms, int per_sm = 4) {
   size_t g = (n + kThreads - 1) / kThreads;
   size_t cap = (size_t)num_sms * per_sm;
@@ -213,6 +228,58 @@ __global__ void k_dense_hamiltonian(HvOperator op, double *__restrict__ h) {
       const uint32_t e = op.dn.ell[(size_t)k * dd + d];
       row[(size_t)(e >> 8) * du + u] += op.dn.vals[e & 255u];
     }
+  }
+}
+
+// Operator averages (see launch_op_averages): a thread per state and operator
+// (blockIdx.y), ranks from binomials in shared memory (lanes read different ones).
+__global__ void __launch_bounds__(kThreads) k_op_averages(OpTerms t, const uint32_t *__restrict__ up, uint32_t du,
+                                                          const uint32_t *__restrict__ dn, size_t D,
+                                                          const double *__restrict__ psi, double *partials) {
+  __shared__ uint32_t bin[33 * 33];
+  __shared__ double sm[2][kThreads / 32];
+  for (int i = threadIdx.x; i < 33 * 33; i += kThreads) bin[i] = c_binom[i / 33][i % 33];
+  __syncthreads();
+  const int op = blockIdx.y, d0 = t.doff[op], d1 = t.doff[op + 1], h0 = t.hoff[op], h1 = t.hoff[op + 1];
+  double a = 0.0, b = 0.0;
+  for (size_t I = blockIdx.x * (size_t)kThreads + threadIdx.x; I < D; I += (size_t)gridDim.x * kThreads) {
+    const uint32_t d = (uint32_t)(I / du), u = (uint32_t)(I - (size_t)d * du);
+    const uint32_t ub = up[u], db = dn[d];
+    double dg = 0.0;
+    for (int k = d0; k < d1; ++k) {
+      const uint2 m = __ldg(t.dterm + k);
+      if ((ub & m.x) == m.x && (db & m.y) == m.y) dg += __ldg(t.dval + k);
+    }
+    const double x = psi[I];
+    double y = dg * x;
+    for (int k = h0; k < h1; ++k) {
+      const int3 h = t.hop[k];
+      const uint32_t w = h.x ? db : ub;
+      if (!((w >> h.z) & 1u) || ((w >> h.y) & 1u)) continue;
+      const uint32_t nb = w ^ (1u << h.z) ^ (1u << h.y);
+      uint32_t rank = 0, rest = nb;
+      for (int i = 1; rest; ++i, rest &= rest - 1) rank += bin[(__ffs(rest) - 1) * 33 + i];
+      const size_t J = h.x ? (size_t)rank * du + u : (size_t)d * du + rank;
+      const double v = (__popc(nb & between_mask(h.y, h.z)) & 1) ? -__ldg(t.hval + k) : __ldg(t.hval + k);
+      y += v * psi[J];
+    }
+    a += x * y;
+    b += y * y;
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int o = 16; o; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  if (lane == 0) {
+    sm[0][warp] = a;
+    sm[1][warp] = b;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    double s = 0.0;
+    for (int w = 0; w < kThreads / 32; ++w) s += sm[threadIdx.x][w];
+    partials[((size_t)op * gridDim.x + blockIdx.x) * 2 + threadIdx.x] = s;
   }
 }
 
@@ -1451,6 +1518,26 @@ void launch_dense_hamiltonian(const HvOperator &op, double *h, cudaStream_t s) {
   if (!D) return;
   QED_CUDA(cudaMemsetAsync(h, 0, D * D * sizeof(double), s));
   k_dense_hamiltonian<<<grid_for(D, device_sms()), kThreads, 0, s>>>(op, h);
+  QED_LAUNCH();
+}
+
+int op_average_blocks(size_t D) { return grid_for(D, device_sms(), 2); }
+
+void launch_op_averages(int nop, const OpTerms &t, const uint32_t *up, uint32_t du, const uint32_t *dn, uint32_t dd,
+                        const double *psi, double *partials, double *out, cudaStream_t s) {
+  ensure_binom();
+  const size_t D = (size_t)du * dd;
+  if (nop <= 0 || !D) return;
+  const int nb = op_average_blocks(D);
+  for (int k = 0; k < nop; k += 65535) {  // the grid's second dimension ends there
+    const int n = std::min(nop - k, 65535);
+    OpTerms tk = t;
+    tk.doff += k;
+    tk.hoff += k;
+    k_op_averages<<<dim3(nb, n), kThreads, 0, s>>>(tk, up, du, dn, D, psi, partials + 2 * (size_t)k * nb);
+    QED_LAUNCH();
+  }
+  k_pair_sums<<<nop, 64, 0, s>>>(partials, nb, out);
   QED_LAUNCH();
 }
 

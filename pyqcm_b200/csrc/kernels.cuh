@@ -115,6 +115,22 @@ void launch_cdag_gather(int L, int spin, int a, int pm, const uint32_t *tgt_up_b
 // hold D*D doubles; it is overwritten.
 void launch_dense_hamiltonian(const HvOperator &op, double *h, cudaStream_t s);
 
+// <psi|O|psi> and |O psi|^2 of nop operators in one pass, without their spin tables:
+// operator k's density terms are dterm[doff[k]] .. dterm[doff[k + 1]] (a state
+// counts dval where it has every bit of the up mask .x and of the down mask .y), its
+// hops hop[hoff[k]] .. (spin, r, c: c+_r c_c, amplitude hval). partials: 2 * nop *
+// op_average_blocks(D) doubles; out[2 k], out[2 k + 1] on return.
+struct OpTerms {
+  const int *doff, *hoff;
+  const uint2 *dterm;
+  const double *dval;
+  const int3 *hop;
+  const double *hval;
+};
+int op_average_blocks(size_t D);
+void launch_op_averages(int nop, const OpTerms &t, const uint32_t *up, uint32_t du, const uint32_t *dn, uint32_t dd,
+                        const double *psi, double *partials, double *out, cudaStream_t s);
+
 // ---- device-resident Lanczos step ------------------------------------------
 // Scalars of a ground-state Lanczos run kept in device memory, so that a chunk
 // of iterations runs without host round trips (LanczosEigenvalue,
