@@ -195,41 +195,55 @@ const bool g_parallel_for_set = [] {
   return true;
 }();
 
-// The inter-cluster elements (r, c, R, v) of V(k) on the device as LatticeView
-// wants them: ordered by row (the order of a row's elements kept), the grid's
-// directions by size, R reduced to the grid, the phase of the grid's offset (the
-// same along every direction, in units of a grid step) in v.
-struct LatticeElements {
-  DevBuf<int> row;
-  DevBuf<LatticeElement> el;
+// The input of a lattice sum on the device: frequencies i w, the k-independent
+// parts of V and the inter-cluster elements (r, c, R, v) as LatticeView wants them
+// (ordered by row, the order of a row's elements kept; the grid's directions by
+// size, R reduced to the grid; the phase of the grid's offset, the same along every
+// direction in units of a grid step, in v). One pinned copy and one allocation
+// instead of five each: the sums themselves take some ten microseconds.
+struct LatticeInput {
+  DevBuf<double> buf;
+  std::vector<cplx> z;
+  const double *dz, *V0;
+  LatticeView el;
   int nk[3];
-  LatticeElements(int dim, int nel, const int *r, const int *c, const int *R, const double *vv, int nkx, int nky,
-                  int nkz, double off, cudaStream_t s) {
+  LatticeInput(int dim, int nw, const double *w, size_t nV0, const double *hV0, int nel, const int *r, const int *c,
+               const int *R, const double *vv, int nkx, int nky, int nkz, double off, Workspace &W)
+      : z(nw) {
     const int given[3] = {nkx, nky, nkz};
     int dir[3] = {0, 1, 2};
     std::stable_sort(dir, dir + 3, [&](int a, int b) { return given[a] < given[b]; });
     for (int i = 0; i < 3; ++i) nk[i] = given[dir[i]];
-    std::vector<int> first(dim + 1, 0);
+    // [elements | z | V0 | first element of each row], in doubles
+    const size_t ne = std::max(nel, 1) * (sizeof(LatticeElement) / sizeof(double)), nz = 2 * (size_t)nw;
+    const size_t total = ne + nz + nV0 + (dim + 2) / 2 + 1;
+    double *h = W.pinned(total);
+    LatticeElement *he = reinterpret_cast<LatticeElement *>(h);
+    int *first = reinterpret_cast<int *>(h + ne + nz + nV0);
+    std::fill(first, first + dim + 1, 0);
     for (int e = 0; e < nel; ++e) ++first[r[e] + 1];
     for (int a = 0; a < dim; ++a) first[a + 1] += first[a];
-    std::vector<int> next(first.begin(), first.end() - 1);
-    std::vector<LatticeElement> h(std::max(nel, 1), LatticeElement{{0.0, 0.0}, {0, 0, 0, 0}});
+    std::vector<int> next(first, first + dim);
     for (int e = 0; e < nel; ++e) {
-      int w[3];
+      int q[3];
       double turn = 0.0;
       for (int i = 0; i < 3; ++i) {
         const long Ri = R[3 * e + dir[i]];
-        w[i] = (int)((Ri % nk[i] + nk[i]) % nk[i]);
+        q[i] = (int)((Ri % nk[i] + nk[i]) % nk[i]);
         turn += off * Ri / nk[i];
       }
       std::complex<double> x(vv[2 * e], vv[2 * e + 1]);
       if (off != 0.0) x *= std::polar(1.0, 2.0 * M_PI * turn);
-      h[next[r[e]]++] = LatticeElement{{x.real(), x.imag()}, {c[e], w[0], w[1], w[2]}};
+      he[next[r[e]]++] = LatticeElement{{x.real(), x.imag()}, {c[e], q[0], q[1], q[2]}};
     }
-    row.upload(first, s);
-    el.upload(h, s);
+    for (int i = 0; i < nw; ++i) z[i] = cplx(0.0, w[i]);
+    std::memcpy(h + ne, z.data(), nz * sizeof(double));
+    std::memcpy(h + ne + nz, hV0, nV0 * sizeof(double));
+    buf.upload(h, total, W.stream);
+    dz = buf.p + ne;
+    V0 = dz + nz;
+    el = {reinterpret_cast<const int *>(V0 + nV0), reinterpret_cast<const LatticeElement *>(buf.p)};
   }
-  LatticeView view() const { return {row.p, el.p}; }
 };
 
 // Weighted tasks run longest-first (LPT) on the batch thread pool.
@@ -770,18 +784,17 @@ int qed_sef_integrand_grid(int label, int spin_down, int dim, const double *V0, 
         fail(QED_ERR_ARGUMENT, "qed_sef_integrand_grid: element index outside the Green function");
     if (nw == 0) return;
     Workspace &W = ws();
-    std::vector<cplx> z(nw);
-    for (int i = 0; i < nw; ++i) z[i] = cplx(0.0, w[i]);
     const size_t nn = (size_t)dim * dim;
     const long nk = (long)nkx * nky * nkz;
     const int nblk = lattice_blocks(dim, nw, nk);
-    DevBuf<double> dG(2 * nn * nw), dV0(2 * nn), part((size_t)nblk * nw);
-    I->green_function_device(z.data(), nw, spin_down != 0, dG.p, W);
-    dV0.upload(V0, 2 * nn, W.stream);
-    const LatticeElements el(dim, nel, r, c, R, v, nkx, nky, nkz, 0.0, W.stream);
-    launch_sef_logdet(dim, nw, dG.p, dV0.p, el.view(), el.nk, part.p, W.stream);
+    I->require_green_function(spin_down != 0, W);
+    const LatticeInput in(dim, nw, w, 2 * nn, V0, nel, r, c, R, v, nkx, nky, nkz, 0.0, W);
+    DevBuf<double> dG(2 * nn * nw + (size_t)nblk * nw);
+    double *part = dG.p + 2 * nn * nw;
+    I->green_function_device(in.z.data(), in.dz, nw, spin_down != 0, dG.p, W);
+    launch_sef_logdet(dim, nw, dG.p, in.V0, in.el, in.nk, part, W.stream);
     std::vector<double> h((size_t)nblk * nw);
-    part.download(h.data(), h.size(), W.stream);
+    QED_CUDA(cudaMemcpyAsync(h.data(), part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, W.stream));
     W.sync();
     for (int i = 0; i < nw; ++i) {
       double s = 0.0;
@@ -806,16 +819,15 @@ int qed_cpt_projected_green_function(int label, int spin_down, int dim, const do
         fail(QED_ERR_ARGUMENT, "qed_cpt_projected_green_function: element index outside the Green function");
     if (nw == 0) return;
     Workspace &W = ws();
-    std::vector<cplx> z(nw);
-    for (int i = 0; i < nw; ++i) z[i] = cplx(0.0, w[i]);
     const size_t nn = (size_t)dim * dim;
     const int nblk = lattice_blocks(dim, std::min(nw, 65535), (long)nkx * nky * nkz);
-    DevBuf<double> dG(2 * nn * nw), dV0(2 * nn * nw), part(2 * nn * nw * nblk), dP(2 * nn * nw);
-    I->green_function_device(z.data(), nw, spin_down != 0, dG.p, W);
-    dV0.upload(V0, 2 * nn * nw, W.stream);
-    const LatticeElements el(dim, nel, r, c, R, v, nkx, nky, nkz, offset, W.stream);
-    launch_cpt_projected(dim, nw, dG.p, dV0.p, el.view(), el.nk, part.p, dP.p, W.stream);
-    dP.download(Gproj, 2 * nn * nw, W.stream);
+    I->require_green_function(spin_down != 0, W);
+    const LatticeInput in(dim, nw, w, 2 * nn * nw, V0, nel, r, c, R, v, nkx, nky, nkz, offset, W);
+    DevBuf<double> dG(2 * nn * nw * (nblk + 2));
+    double *part = dG.p + 2 * nn * nw, *dP = part + 2 * nn * nw * nblk;
+    I->green_function_device(in.z.data(), in.dz, nw, spin_down != 0, dG.p, W);
+    launch_cpt_projected(dim, nw, dG.p, in.V0, in.el, in.nk, part, dP, W.stream);
+    QED_CUDA(cudaMemcpyAsync(Gproj, dP, 2 * nn * nw * sizeof(double), cudaMemcpyDeviceToHost, W.stream));
     W.sync();
   });
 }

@@ -1325,10 +1325,8 @@ void Instance::green_function(const cplx *z, int nz, bool spin_down, cplx *out, 
   }
 }
 
-void Instance::green_function_device(const cplx *z, int nz, bool spin_down, double *dG, Workspace &ws) {
-  if (spin_down && !(mix & mixing::up_down || mix == 0))
-    fail(QED_ERR_ARGUMENT, "spin_down=True impossible with Hilbert space mixing " + std::to_string(mix));
-  if (!gf_solved) green_solve(ws);
+void Instance::green_function_device(const cplx *z, const double *dz, int nz, bool spin_down, double *dG,
+                                     Workspace &ws) {
   const int n = model->n_sites;
   const int sd = (spin_down && (mix & mixing::up_down)) ? 1 : 0;
   const size_t nn = (size_t)n * n;
@@ -1340,14 +1338,17 @@ void Instance::green_function_device(const cplx *z, int nz, bool spin_down, doub
     ws.sync();
     return;
   }
-  DevBuf<double> dz(2 * (size_t)nz);
-  dz.upload(reinterpret_cast<const double *>(z), 2 * (size_t)nz, ws.stream);
   QED_CUDA(cudaMemsetAsync(dG, 0, 2 * nn * nz * sizeof(double), ws.stream));
   for (auto &st : states) {
     const QMat &q = st->q[sd];
-    launch_qmatrix_gf(n, q.M, q.de.p, q.dV.p, nz, dz.p, dG, ws.stream);
+    launch_qmatrix_gf(n, q.M, q.de.p, q.dV.p, nz, dz, dG, ws.stream);
   }
-  ws.sync();
+}
+
+void Instance::require_green_function(bool spin_down, Workspace &ws) {
+  if (spin_down && !(mix & mixing::up_down || mix == 0))
+    fail(QED_ERR_ARGUMENT, "spin_down=True impossible with Hilbert space mixing " + std::to_string(mix));
+  if (!gf_solved) green_solve(ws);
 }
 
 // hybridization_function (src_ed/model_instance.hpp:1004-1018)
