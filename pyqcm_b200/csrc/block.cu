@@ -166,6 +166,7 @@ template <int P>
 __global__ void __launch_bounds__(kPipeThreads) k_bl_pipe(size_t D, int p, double a, BlockOut Y, double s1,
                                                           BlockIn X1, const double *__restrict__ M1, int gram,
                                                           BlockIn L, double *partials) {
+  pdl_begin();
   constexpr int NT = P / 8;      // 8-vector tiles
   constexpr int KS = P / 4;      // k steps of the update
   constexpr int PANEL = P * kPanelLd;
@@ -331,9 +332,9 @@ int launch_bl_update(size_t D, int p, double a, const BlockOut &Y, double s1, co
     if (gram && g2 > max_blocks) g2 = max_blocks;
     g2 = std::max(g2, 1);
     if (p <= 8)
-      k_bl_pipe<8><<<g2, kPipeThreads, psmem(8), s>>>(D, p, a, Y, s1, X1, M1, gram, L, partials);
+      launch_pdl(D, k_bl_pipe<8>, g2, kPipeThreads, psmem(8), s, D, p, a, Y, s1, X1, M1, gram, L, partials);
     else
-      k_bl_pipe<16><<<g2, kPipeThreads, psmem(16), s>>>(D, p, a, Y, s1, X1, M1, gram, L, partials);
+      launch_pdl(D, k_bl_pipe<16>, g2, kPipeThreads, psmem(16), s, D, p, a, Y, s1, X1, M1, gram, L, partials);
     QED_LAUNCH();
     return g2;
   }

@@ -33,6 +33,37 @@ inline void cuda_check(cudaError_t e, const char *what, const char *file, int li
 #define QED_CUDA(x) ::qed::cuda_check((x), #x, __FILE__, __LINE__)
 #define QED_LAUNCH() ::qed::cuda_check(cudaGetLastError(), "kernel launch", __FILE__, __LINE__)
 
+// Launch that may begin while the stream's previous kernel ends (programmatic
+// dependent launch): the kernel's CTAs are scheduled once every CTA of the previous
+// kernel has started and, by pdl_begin() as their first statement, wait until it has
+// completed and its memory is visible. What a chain of dependent small kernels
+// saves is the gap between them, about a microsecond each (a solve of three sectors
+// of up to 124,000 states: 112 ms without, 86 ms with). D: the states the kernel
+// works on. Above kPdlStates a kernel's time hides its gap and the next kernel's CTAs
+// only stand in the way: the product with 41 million states took 1281 us without and
+// 1327 us with. A kernel launched without it passes through pdl_begin() at once.
+constexpr size_t kPdlStates = size_t(1) << 22;
+template <class... P, class... A>
+void launch_pdl(size_t D, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = D <= kPdlStates ? 1 : 0;
+  cuda_check(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...), "kernel launch", __FILE__, __LINE__);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 // Stream used for stream-ordered allocation by the calling host thread: the
 // stream of that thread's Workspace (legacy default stream before one exists).
 cudaStream_t alloc_stream();

@@ -70,6 +70,7 @@ __device__ __forceinline__ uint32_t colex_unrank(uint32_t I, int L, int N) {
 }
 
 __global__ void k_finalize(const double *partials, int nblocks, double *out) {
+  pdl_begin();
   // one block per slot, fixed-order tree sum
   __shared__ double sm[kThreads];
   const int slot = blockIdx.x;
@@ -388,6 +389,7 @@ __global__ void __launch_bounds__(kThreads) k_hv_cols(HvOperator op, const doubl
 template <int UNROLL>
 __global__ void __launch_bounds__(1024) k_hv_rows2(HvOperator op, const double *__restrict__ x,
                                                    double xs, double *y, SubList sub) {
+  pdl_begin();
   if (op.skip && *op.skip) return;
   extern __shared__ double2 xs2[];
   __shared__ double vals[256];
@@ -460,6 +462,7 @@ template <int VEC, bool CG>
 __global__ void __launch_bounds__(kThreads) k_hv_cols2(HvOperator op, const double *__restrict__ x,
                                                         double xs, double *y, int red_mask,
                                                         double *partials, uint32_t r0, uint32_t r1) {
+  pdl_begin();
   if (op.skip && *op.skip) return;
   __shared__ double cval[kColsR][kMaxHops];
   __shared__ uint32_t cidx[kColsR][kMaxHops];
@@ -1006,6 +1009,7 @@ __global__ void __launch_bounds__(256) k_mcf_eval(const McfDesc *desc, const dou
 // launch per pass for the whole block is what counts.
 template <int P>
 __global__ void __launch_bounds__(kThreads) k_blhv_rows(HvOperator op, int p, BlockIn X, BlockOut Y) {
+  pdl_begin();
   const uint32_t du = op.up.dim, dd = op.dn.dim;
   const size_t D = (size_t)du * dd;
   for (size_t I = blockIdx.x * (size_t)blockDim.x + threadIdx.x; I < D; I += (size_t)gridDim.x * blockDim.x) {
@@ -1032,6 +1036,7 @@ __global__ void __launch_bounds__(kThreads) k_blhv_rows(HvOperator op, int p, Bl
 
 template <int P>
 __global__ void __launch_bounds__(kThreads) k_blhv_cols(HvOperator op, int p, BlockIn X, BlockOut Y) {
+  pdl_begin();
   const uint32_t du = op.up.dim, dd = op.dn.dim;
   const size_t D = (size_t)du * dd;
   for (size_t I = blockIdx.x * (size_t)blockDim.x + threadIdx.x; I < D; I += (size_t)gridDim.x * blockDim.x) {
@@ -1059,6 +1064,7 @@ __global__ void __launch_bounds__(kThreads) k_blhv_cols(HvOperator op, int p, Bl
 template <int G>
 __global__ void k_dots(size_t D, double *x, double xs, int write_x, VecList ys, int first,
                        double *partials) {
+  pdl_begin();
   if (ys.skip && *ys.skip) return;
   if (ys.xsdev && first == 0) xs = *ys.xsdev;
   double acc[G];
@@ -1091,6 +1097,7 @@ __global__ void k_dots(size_t D, double *x, double xs, int write_x, VecList ys, 
 
 __global__ void k_multi_axpy(size_t D, const double *x, double xs, VecList ys, int norm_first,
                              double *partials) {
+  pdl_begin();
   if (ys.skip && *ys.skip) return;
   double nrm[1] = {0.0};
   for (size_t I = blockIdx.x * (size_t)blockDim.x + threadIdx.x; I < D; I += (size_t)gridDim.x * blockDim.x) {
@@ -1106,6 +1113,7 @@ __global__ void k_multi_axpy(size_t D, const double *x, double xs, VecList ys, i
 
 __global__ void k_axpby(size_t D, double a, double *y, double b, const double *x, int norm,
                         double *partials) {
+  pdl_begin();
   double nrm[1] = {0.0};
   for (size_t I = blockIdx.x * (size_t)blockDim.x + threadIdx.x; I < D; I += (size_t)gridDim.x * blockDim.x) {
     double v = (a != 0.0 ? a * y[I] : 0.0) + (x ? b * x[I] : 0.0);
@@ -1117,6 +1125,7 @@ __global__ void k_axpby(size_t D, double a, double *y, double b, const double *x
 
 __global__ void k_axpy_dev(size_t D, double *y, const double *x, const double *a_dev, double *partials,
                            const int *skip) {
+  pdl_begin();
   if (skip && *skip) return;
   const double b = -*a_dev;
   double nrm[1] = {0.0};
@@ -1129,6 +1138,7 @@ __global__ void k_axpy_dev(size_t D, double *y, const double *x, const double *a
 }
 
 __global__ void k_lanczos_advance(size_t D, double *y, LanczosScalars ls) {
+  pdl_begin();
   const double b = sqrt(*ls.b2_cur);
   const double z = (b > 0.0) ? 1.0 / b : 0.0;
   for (size_t I = blockIdx.x * (size_t)blockDim.x + threadIdx.x; I < D; I += (size_t)gridDim.x * blockDim.x)
@@ -1269,6 +1279,7 @@ __global__ void k_random(size_t D, uint64_t seed, double *y, double *partials) {
 }
 
 __global__ void k_scale_dev(size_t D, double *y, const double *a_dev, const int *skip) {
+  pdl_begin();
   if (skip && *skip) return;
   const double a = *a_dev;
   for (size_t I = blockIdx.x * (size_t)blockDim.x + threadIdx.x; I < D; I += (size_t)gridDim.x * blockDim.x)
@@ -1280,6 +1291,7 @@ __global__ void k_scale_dev(size_t D, double *y, const double *a_dev, const int 
 // otherwise it stores z and 1/z.
 __global__ void k_finalize_norm(const double *partials, int nblocks, double dtol, double *z_out,
                                 double *inv_out, int *flag, int step) {
+  pdl_begin();
   __shared__ double sm[kThreads];
   double s = 0.0;
   for (int b = threadIdx.x; b < nblocks; b += blockDim.x) s += partials[(size_t)b * Reducer::kMaxRed];
@@ -1301,6 +1313,7 @@ __global__ void k_finalize_norm(const double *partials, int nblocks, double dtol
 }
 
 __global__ void k_scale(size_t D, double *y, double a) {
+  pdl_begin();
   for (size_t I = blockIdx.x * (size_t)blockDim.x + threadIdx.x; I < D; I += (size_t)gridDim.x * blockDim.x)
     y[I] *= a;
 }
@@ -1312,6 +1325,7 @@ __global__ void k_scale(size_t D, double *y, double a) {
 
 // out[slot] = sum over blocks of partials[b * ld + slot], slot < n, fixed order.
 __global__ void k_finalize_ld(const double *partials, int nblocks, int ld, double *out) {
+  pdl_begin();
   __shared__ double sm[kThreads];
   const int slot = blockIdx.x;
   double s = 0.0;
@@ -1337,6 +1351,7 @@ __global__ void k_finalize_ld(const double *partials, int nblocks, int ld, doubl
 __global__ void __launch_bounds__(256) k_block_chol(int p, const double *G, double pivot_min, double *R,
                                                     double *Rinv, const double *Rprev, double *B_out,
                                                     double *Bt_out, double *fail_flag) {
+  pdl_begin();
   __shared__ double a[256], ri[256];
   __shared__ int bad;
   const int t = threadIdx.x, pp = p * p;
@@ -1671,9 +1686,9 @@ void launch_hv_rows(const HvOperator &op, const double *x, double xs, double *y,
     const int per_sm = smem2 > 110 * 1024 ? 1 : (smem2 > 72 * 1024 ? 2 : 3);
     int grid = (int)std::min<size_t>((dd + 1) / 2, (size_t)device_sms() * per_sm);
     if (hv_variant() & 2)
-      k_hv_rows2<4><<<grid, t2, smem2, s>>>(op, x, xs, y, sub);
+      launch_pdl((size_t)op.up.dim * op.dn.dim, k_hv_rows2<4>, grid, t2, smem2, s, op, x, xs, y, sub);
     else
-      k_hv_rows2<2><<<grid, t2, smem2, s>>>(op, x, xs, y, sub);
+      launch_pdl((size_t)op.up.dim * op.dn.dim, k_hv_rows2<2>, grid, t2, smem2, s, op, x, xs, y, sub);
   } else if (smem <= kRowSmemMax) {
     static const bool attr = [] {
       QED_CUDA(cudaFuncSetAttribute(k_hv_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1699,11 +1714,11 @@ int launch_hv_cols(const HvOperator &op, const double *x, double xs, double *y, 
   const bool cg = hv_variant() & 1;
   const uint32_t dd = op.dn.dim;
   if (vec2 && cg)
-    k_hv_cols2<2, true><<<grid, kThreads, 0, s>>>(op, x, xs, y, red_mask, r.partials, 0u, dd);
+    launch_pdl((size_t)op.up.dim * op.dn.dim, k_hv_cols2<2, true>, grid, kThreads, 0, s, op, x, xs, y, red_mask, r.partials, 0u, dd);
   else if (vec2)
-    k_hv_cols2<2, false><<<grid, kThreads, 0, s>>>(op, x, xs, y, red_mask, r.partials, 0u, dd);
+    launch_pdl((size_t)op.up.dim * op.dn.dim, k_hv_cols2<2, false>, grid, kThreads, 0, s, op, x, xs, y, red_mask, r.partials, 0u, dd);
   else
-    k_hv_cols2<1, false><<<grid, kThreads, 0, s>>>(op, x, xs, y, red_mask, r.partials, 0u, dd);
+    launch_pdl((size_t)op.up.dim * op.dn.dim, k_hv_cols2<1, false>, grid, kThreads, 0, s, op, x, xs, y, red_mask, r.partials, 0u, dd);
   QED_LAUNCH();
   return grid;
 }
@@ -1713,9 +1728,9 @@ void launch_hv_cols_rows(const HvOperator &op, const double *x, double xs, doubl
   if (r1 <= r0) return;
   const int grid = hv_cols_grid(op);
   if (op.up.dim % 2 == 0)
-    k_hv_cols2<2, false><<<grid, kThreads, 0, s>>>(op, x, xs, y, 0, nullptr, r0, r1);
+    launch_pdl((size_t)op.up.dim * op.dn.dim, k_hv_cols2<2, false>, grid, kThreads, 0, s, op, x, xs, y, 0, nullptr, r0, r1);
   else
-    k_hv_cols2<1, false><<<grid, kThreads, 0, s>>>(op, x, xs, y, 0, nullptr, r0, r1);
+    launch_pdl((size_t)op.up.dim * op.dn.dim, k_hv_cols2<1, false>, grid, kThreads, 0, s, op, x, xs, y, 0, nullptr, r0, r1);
   QED_LAUNCH();
 }
 
@@ -1905,17 +1920,17 @@ void launch_block_hv(const HvOperator &op, int p, const BlockIn &X, const BlockO
   }
   const int grid = grid_for(D, device_sms(), 8);
   if (p <= 4) {
-    k_blhv_rows<4><<<grid, kThreads, 0, s>>>(op, p, X, Y);
+    launch_pdl(D, k_blhv_rows<4>, grid, kThreads, 0, s, op, p, X, Y);
     QED_LAUNCH();
-    k_blhv_cols<4><<<grid, kThreads, 0, s>>>(op, p, X, Y);
+    launch_pdl(D, k_blhv_cols<4>, grid, kThreads, 0, s, op, p, X, Y);
   } else if (p <= 8) {
-    k_blhv_rows<8><<<grid, kThreads, 0, s>>>(op, p, X, Y);
+    launch_pdl(D, k_blhv_rows<8>, grid, kThreads, 0, s, op, p, X, Y);
     QED_LAUNCH();
-    k_blhv_cols<8><<<grid, kThreads, 0, s>>>(op, p, X, Y);
+    launch_pdl(D, k_blhv_cols<8>, grid, kThreads, 0, s, op, p, X, Y);
   } else {
-    k_blhv_rows<16><<<grid, kThreads, 0, s>>>(op, p, X, Y);
+    launch_pdl(D, k_blhv_rows<16>, grid, kThreads, 0, s, op, p, X, Y);
     QED_LAUNCH();
-    k_blhv_cols<16><<<grid, kThreads, 0, s>>>(op, p, X, Y);
+    launch_pdl(D, k_blhv_cols<16>, grid, kThreads, 0, s, op, p, X, Y);
   }
   QED_LAUNCH();
 }
@@ -1925,7 +1940,7 @@ int launch_dots(size_t D, double *x, double xs, int write_x, const VecList &ys, 
   int grid = std::min(grid_for(D, device_sms(), 4), r.max_blocks);
   constexpr int G = 8;
   if (ys.n == 0 && write_x) {
-    k_scale<<<grid, kThreads, 0, s>>>(D, x, xs);
+    launch_pdl(D, k_scale, grid, kThreads, 0, s, D, x, xs);
     QED_LAUNCH();
     return grid;
   }
@@ -1933,7 +1948,7 @@ int launch_dots(size_t D, double *x, double xs, int write_x, const VecList &ys, 
     // x is scaled in place only on the first sweep; later sweeps read the scaled x.
     const bool wx = write_x && first == 0;
     const double sc = (write_x && first > 0) ? 1.0 : xs;
-    k_dots<G><<<grid, kThreads, 0, s>>>(D, x, sc, wx, ys, first, r.partials);
+    launch_pdl(D, k_dots<G>, grid, kThreads, 0, s, D, x, sc, wx, ys, first, r.partials);
     QED_LAUNCH();
   }
   return grid;
@@ -1942,7 +1957,7 @@ int launch_dots(size_t D, double *x, double xs, int write_x, const VecList &ys, 
 int launch_multi_axpy(size_t D, const double *x, double xs, const VecList &ys, int norm_first,
                       Reducer &r, cudaStream_t s) {
   int grid = std::min(grid_for(D, device_sms(), 4), r.max_blocks);
-  k_multi_axpy<<<grid, kThreads, 0, s>>>(D, x, xs, ys, norm_first, r.partials);
+  launch_pdl(D, k_multi_axpy, grid, kThreads, 0, s, D, x, xs, ys, norm_first, r.partials);
   QED_LAUNCH();
   return grid;
 }
@@ -1950,7 +1965,7 @@ int launch_multi_axpy(size_t D, const double *x, double xs, const VecList &ys, i
 int launch_axpby(size_t D, double a, double *y, double b, const double *x, int norm, Reducer &r,
                  cudaStream_t s) {
   int grid = std::min(grid_for(D, device_sms(), 4), r.max_blocks);
-  k_axpby<<<grid, kThreads, 0, s>>>(D, a, y, b, x, norm, r.partials);
+  launch_pdl(D, k_axpby, grid, kThreads, 0, s, D, a, y, b, x, norm, r.partials);
   QED_LAUNCH();
   return grid;
 }
@@ -1958,13 +1973,13 @@ int launch_axpby(size_t D, double a, double *y, double b, const double *x, int n
 int launch_axpy_dev(size_t D, double *y, const double *x, const double *a_dev, Reducer &r, cudaStream_t s,
                     const int *skip) {
   int grid = std::min(grid_for(D, device_sms(), 4), r.max_blocks);
-  k_axpy_dev<<<grid, kThreads, 0, s>>>(D, y, x, a_dev, r.partials, skip);
+  launch_pdl(D, k_axpy_dev, grid, kThreads, 0, s, D, y, x, a_dev, r.partials, skip);
   QED_LAUNCH();
   return grid;
 }
 
 void launch_lanczos_advance(size_t D, double *y, const LanczosScalars &ls, cudaStream_t s) {
-  k_lanczos_advance<<<grid_for(D, device_sms(), 4), kThreads, 0, s>>>(D, y, ls);
+  launch_pdl(D, k_lanczos_advance, grid_for(D, device_sms(), 4), kThreads, 0, s, D, y, ls);
   QED_LAUNCH();
 }
 
@@ -1981,14 +1996,14 @@ void launch_lanczos_jobs(const LanczosJob *jobs, int njobs, cudaStream_t s) {
 }
 
 void launch_finalize_ld(const double *partials, int nblocks, int ld, int n, double *out, cudaStream_t s) {
-  k_finalize_ld<<<n, kThreads, 0, s>>>(partials, nblocks, ld, out);
+  launch_pdl(0, k_finalize_ld, n, kThreads, 0, s, partials, nblocks, ld, out);
   QED_LAUNCH();
 }
 
 void launch_block_chol(int p, const double *G, double pivot_min, double *R, double *Rinv, const double *Rprev,
                        double *B_out, double *Bt_out, double *fail_flag, cudaStream_t s) {
   if (p < 1 || p > 16) fail(QED_ERR_ARGUMENT, "launch_block_chol: block size outside [1, 16]");
-  k_block_chol<<<1, 256, 0, s>>>(p, G, pivot_min, R, Rinv, Rprev, B_out, Bt_out, fail_flag);
+  launch_pdl(0, k_block_chol, 1, 256, 0, s, p, G, pivot_min, R, Rinv, Rprev, B_out, Bt_out, fail_flag);
   QED_LAUNCH();
 }
 
@@ -2005,29 +2020,29 @@ int launch_random(size_t D, uint64_t seed, double *y, Reducer &r, cudaStream_t s
 }
 
 void launch_scale_dev(size_t D, double *y, const double *a_dev, const int *skip, cudaStream_t s) {
-  k_scale_dev<<<grid_for(D, device_sms(), 4), kThreads, 0, s>>>(D, y, a_dev, skip);
+  launch_pdl(D, k_scale_dev, grid_for(D, device_sms(), 4), kThreads, 0, s, D, y, a_dev, skip);
   QED_LAUNCH();
 }
 
 void launch_finalize_norm(const double *partials, int nblocks, double dtol, double *z_out, double *inv_out,
                           int *flag, int step, cudaStream_t s) {
-  k_finalize_norm<<<1, kThreads, 0, s>>>(partials, nblocks, dtol, z_out, inv_out, flag, step);
+  launch_pdl(0, k_finalize_norm, 1, kThreads, 0, s, partials, nblocks, dtol, z_out, inv_out, flag, step);
   QED_LAUNCH();
 }
 
 void launch_scale(size_t D, double *y, double a, cudaStream_t s) {
-  k_scale<<<grid_for(D, device_sms(), 4), kThreads, 0, s>>>(D, y, a);
+  launch_pdl(D, k_scale, grid_for(D, device_sms(), 4), kThreads, 0, s, D, y, a);
   QED_LAUNCH();
 }
 
 void finalize_sums(Reducer &r, int nblocks, int nred, cudaStream_t s) {
-  k_finalize<<<nred, kThreads, 0, s>>>(r.partials, nblocks, r.out);
+  launch_pdl(0, k_finalize, nred, kThreads, 0, s, r.partials, nblocks, r.out);
   QED_LAUNCH();
   QED_CUDA(cudaMemcpyAsync(r.host, r.out, nred * sizeof(double), cudaMemcpyDeviceToHost, s));
 }
 
 void launch_finalize(const double *partials, int nblocks, int nred, double *out, cudaStream_t s) {
-  k_finalize<<<nred, kThreads, 0, s>>>(partials, nblocks, out);
+  launch_pdl(0, k_finalize, nred, kThreads, 0, s, partials, nblocks, out);
   QED_LAUNCH();
 }
 

@@ -617,6 +617,7 @@ __device__ __forceinline__ void packed_part(const PackedView &P, const double *_
 template <int W, bool wide, class Epi>
 __global__ void __launch_bounds__(kPackedThreads) k_packed(const PackedView P, const double *__restrict__ x,
                                                            uint64_t D, uint64_t nslices, uint64_t nb, const Epi epi) {
+  pdl_begin();
   if (epi.off()) return;
   constexpr int kWarps = kPackedThreads / 32, kBlocks = kWarps / W, Q = 8 / W;
   __shared__ double values[256];
@@ -1007,9 +1008,9 @@ void launch_packed_w(const MixedHamiltonian &H, const double *x, const Epi &epi,
   const uint64_t nslices = (H.D + 31) / 32;
   const unsigned per = kPackedThreads / 32 / W, grid = (nb + per - 1) / per;
   if (H.code.p)
-    k_packed<W, true><<<grid, kPackedThreads, 0, s>>>(H.packed_view(), x, H.D, nslices, nb, epi);
+    launch_pdl(H.D, k_packed<W, true, Epi>, grid, kPackedThreads, 0, s, H.packed_view(), x, H.D, nslices, nb, epi);
   else
-    k_packed<W, false><<<grid, kPackedThreads, 0, s>>>(H.packed_view(), x, H.D, nslices, nb, epi);
+    launch_pdl(H.D, k_packed<W, false, Epi>, grid, kPackedThreads, 0, s, H.packed_view(), x, H.D, nslices, nb, epi);
   QED_LAUNCH();
 }
 template <class Epi>
