@@ -1004,11 +1004,12 @@ __global__ void __launch_bounds__(256) k_mcf_eval(const McfDesc *desc, const dou
 //
 // A block of p <= 16 vectors (pointer arrays) through the ELL tables: one
 // thread per state applies every hop to all p vectors, so each table entry is
-// read once per state for the whole block. Row pass: Y_c = (diag + up hops) X_c;
-// column pass: Y_c += (dn hops) X_c. Small sectors are launch-bound, where one
-// launch per pass for the whole block is what counts.
+// read once per state for the whole block. The up part (with the diagonal) and
+// the down part have accumulators of their own and are added at the end, as when
+// they were two passes through Y. Small sectors are launch-bound, where one launch
+// for the whole block is what counts.
 template <int P>
-__global__ void __launch_bounds__(kThreads) k_blhv_rows(HvOperator op, int p, BlockIn X, BlockOut Y) {
+__global__ void __launch_bounds__(kThreads) k_blhv(HvOperator op, int p, BlockIn X, BlockOut Y) {
   pdl_begin();
   const uint32_t du = op.up.dim, dd = op.dn.dim;
   const size_t D = (size_t)du * dd;
@@ -1016,46 +1017,32 @@ __global__ void __launch_bounds__(kThreads) k_blhv_rows(HvOperator op, int p, Bl
     const uint32_t u = (uint32_t)(I % du), d = (uint32_t)(I / du);
     const double dg = op.up.diag[u] + op.dn.diag[d] + inter_term(op.inter, op.up.bits[u], op.dn.bits[d]);
     const size_t row = (size_t)d * du;
-    double acc[P];
+    double up[P], dn[P];
 #pragma unroll
-    for (int c = 0; c < P; ++c) acc[c] = c < p ? dg * X.v[c][I] : 0.0;
-    const int cu = op.up.cnt[u];
+    for (int c = 0; c < P; ++c) {
+      up[c] = c < p ? dg * X.v[c][I] : 0.0;
+      dn[c] = 0.0;
+    }
+    const int cu = op.up.cnt[u], cd = op.dn.cnt[d];
     for (int k = 0; k < cu; ++k) {
       const uint32_t e = __ldg(op.up.ell + (size_t)k * du + u);
       const double v = op.up.vals[e & 255u];
       const size_t J = row + (e >> 8);
 #pragma unroll
       for (int c = 0; c < P; ++c)
-        if (c < p) acc[c] += v * X.v[c][J];
+        if (c < p) up[c] += v * X.v[c][J];
     }
-#pragma unroll
-    for (int c = 0; c < P; ++c)
-      if (c < p) Y.v[c][I] = acc[c];
-  }
-}
-
-template <int P>
-__global__ void __launch_bounds__(kThreads) k_blhv_cols(HvOperator op, int p, BlockIn X, BlockOut Y) {
-  pdl_begin();
-  const uint32_t du = op.up.dim, dd = op.dn.dim;
-  const size_t D = (size_t)du * dd;
-  for (size_t I = blockIdx.x * (size_t)blockDim.x + threadIdx.x; I < D; I += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t u = (uint32_t)(I % du), d = (uint32_t)(I / du);
-    double acc[P];
-#pragma unroll
-    for (int c = 0; c < P; ++c) acc[c] = 0.0;
-    const int cd = op.dn.cnt[d];
     for (int k = 0; k < cd; ++k) {
       const uint32_t e = __ldg(op.dn.ell + (size_t)k * dd + d);
       const double v = op.dn.vals[e & 255u];
       const size_t J = (size_t)(e >> 8) * du + u;
 #pragma unroll
       for (int c = 0; c < P; ++c)
-        if (c < p) acc[c] += v * X.v[c][J];
+        if (c < p) dn[c] += v * X.v[c][J];
     }
 #pragma unroll
     for (int c = 0; c < P; ++c)
-      if (c < p) Y.v[c][I] += acc[c];
+      if (c < p) Y.v[c][I] = __dadd_rn(up[c], dn[c]);
   }
 }
 
@@ -1121,6 +1108,21 @@ __global__ void k_axpby(size_t D, double a, double *y, double b, const double *x
     nrm[0] += v * v;
   }
   if (norm) block_reduce_store<1>(nrm, partials, 1);
+}
+
+// One step of a Krylov vector's replay: y = (y + c1 x1 + c2 x2) z (x1, x2 null: no
+// term), psi += w y, every product and sum rounded as by separate passes.
+__global__ void k_replay_step(size_t D, double *y, double c1, const double *x1, double c2, const double *x2, double z,
+                              double w, double *psi) {
+  pdl_begin();
+  for (size_t I = blockIdx.x * (size_t)blockDim.x + threadIdx.x; I < D; I += (size_t)gridDim.x * blockDim.x) {
+    double v = y[I];
+    if (x1) v = __dadd_rn(v, __dmul_rn(c1, x1[I]));
+    if (x2) v = __dadd_rn(v, __dmul_rn(c2, x2[I]));
+    v = v * z;
+    y[I] = v;
+    psi[I] = __dadd_rn(psi[I], __dmul_rn(w, v));
+  }
 }
 
 __global__ void k_axpy_dev(size_t D, double *y, const double *x, const double *a_dev, double *partials,
@@ -1339,61 +1341,67 @@ __global__ void k_finalize_ld(const double *partials, int nblocks, int ld, doubl
   if (threadIdx.x == 0) out[slot] = sm[0];
 }
 
-// Cholesky factor of a p x p Gram matrix (p <= 16, row-major): R upper
-// triangular with G = R^T R, and R^{-1}; the kernel exists so that the block
-// recurrence needs no host round trip for its QR. One CTA of 256 threads,
-// thread (r, c) owning entry r * p + c: p right-looking elimination steps in
-// shared memory (each entry receives the same subtractions, in the same order,
-// as the row-by-row host factorisation), then one back substitution per column
-// of R^{-1}. A diagonal that is not positive, or a pivot below pivot_min, sets
-// *fail_flag = 1 and zeroes R^{-1}. With Rprev given, also B = R Rprev (upper
-// triangular) into B_out and its transpose into Bt_out.
+// Cholesky factor of a p x p Gram matrix (p <= 16, row-major): R upper triangular
+// with G = R^T R, and R^{-1}; the kernel exists so that the block recurrence needs no
+// host round trip for its QR. One CTA, thread (r, c) owning entry r * p + c: p
+// right-looking elimination steps in shared memory (each entry receives the same
+// subtractions, in the same order, as the row-by-row host factorisation; a row's
+// scaling is repeated by its readers, which saves two of three barriers a step), then
+// one back substitution per column of R^{-1}. A diagonal that is not positive, or a pivot below pivot_min, sets *fail_flag = 1 and
+// zeroes R^{-1}. With Rprev given, also B = R Rprev (upper triangular) into B_out and
+// its transpose into Bt_out, and with `host` the step's record [A | B | failed] into
+// pinned host memory (A from `A`), which spares a copy (3.3 us). Bound by the chain of
+// square roots and quotients: 5 us for p = 4, 10 us for p = 8 to 10. Adding up the Gram matrix's partials here as well (one CTA
+// instead of one per entry) took longer than the launch it saves.
 __global__ void __launch_bounds__(256) k_block_chol(int p, const double *G, double pivot_min, double *R,
                                                     double *Rinv, const double *Rprev, double *B_out,
-                                                    double *Bt_out, double *fail_flag) {
+                                                    double *Bt_out, double *fail_flag, const double *A,
+                                                    double *host) {
   pdl_begin();
-  __shared__ double a[256], ri[256];
+  __shared__ double a[256], rs[256], ri[256];
   __shared__ int bad;
   const int t = threadIdx.x, pp = p * p;
-  const int r = t / p, c = t - (t / p) * p;  // valid for t < pp
-  if (t < pp) a[t] = G[t];
   if (t == 0) bad = 0;
+  if (t < pp) a[t] = G[t];
   __syncthreads();
+  const int r = t / p, c = t - (t / p) * p;  // valid for t < pp
   for (int i = 0; i < p; ++i) {
-    __syncthreads();                // the updates of step i - 1 are done
     const double d = a[i * p + i];  // fully updated by steps 0..i-1
     const bool ok = d > 0.0;
     const double rii = ok ? sqrt(d) : 1.0;
     if (t == 0 && (!ok || rii < pivot_min)) bad = 1;
-    __syncthreads();  // everyone has read a[i][i]
-    if (t < pp && r == i) a[t] = (c == i) ? rii : (c > i ? a[t] / rii : 0.0);
-    __syncthreads();  // row i of R is final
-    if (t < pp && r > i && c >= r) a[t] -= a[i * p + r] * a[i * p + c];
+    if (t < pp && r == i) rs[t] = (c == i) ? rii : (c > i ? a[t] / rii : 0.0);
+    if (t < pp && r > i && c >= r) a[t] -= (a[i * p + r] / rii) * (a[i * p + c] / rii);
+    __syncthreads();  // row i + 1 is complete, row i of R is final
   }
-  __syncthreads();
-  // R^{-1}: column c by back substitution from row c up (thread c)
-  if (t < p) {
+  if (t < p) {  // column t of R^{-1} by back substitution from row t up
     for (int i = t; i >= 0; --i) {
       double acc = 0.0;
-      for (int k = i + 1; k <= t; ++k) acc += a[i * p + k] * ri[k * p + t];
-      ri[i * p + t] = (i == t) ? 1.0 / a[i * p + i] : -acc / a[i * p + i];
+      for (int k = i + 1; k <= t; ++k) acc += rs[i * p + k] * ri[k * p + t];
+      ri[i * p + t] = (i == t ? 1.0 : -acc) / rs[i * p + i];
     }
     for (int i = t + 1; i < p; ++i) ri[i * p + t] = 0.0;
   }
   __syncthreads();
   if (t < pp) {
-    const double rv = (c >= r) ? a[t] : 0.0;
-    R[t] = rv;
+    R[t] = (c >= r) ? rs[t] : 0.0;
     Rinv[t] = bad ? 0.0 : ri[t];
     if (Rprev) {
       double acc = 0.0;
-      for (int k = r; k <= c; ++k) acc += a[r * p + k] * Rprev[k * p + c];
+      for (int k = r; k <= c; ++k) acc += rs[r * p + k] * Rprev[k * p + c];
       const double b = (c >= r) ? acc : 0.0;
       B_out[t] = b;
       Bt_out[c * p + r] = b;
+      if (host) {
+        host[t] = A[t];
+        host[pp + t] = b;
+      }
     }
   }
-  if (t == 0 && bad) *fail_flag = 1.0;
+  if (t == 0) {
+    if (bad) *fail_flag = 1.0;
+    if (host) host[2 * pp] = *fail_flag;
+  }
 }
 
 // -------------------------------------------------------- Green functions ----
@@ -1920,17 +1928,11 @@ void launch_block_hv(const HvOperator &op, int p, const BlockIn &X, const BlockO
   }
   const int grid = grid_for(D, device_sms(), 8);
   if (p <= 4) {
-    launch_pdl(D, k_blhv_rows<4>, grid, kThreads, 0, s, op, p, X, Y);
-    QED_LAUNCH();
-    launch_pdl(D, k_blhv_cols<4>, grid, kThreads, 0, s, op, p, X, Y);
+    launch_pdl(D, k_blhv<4>, grid, kThreads, 0, s, op, p, X, Y);
   } else if (p <= 8) {
-    launch_pdl(D, k_blhv_rows<8>, grid, kThreads, 0, s, op, p, X, Y);
-    QED_LAUNCH();
-    launch_pdl(D, k_blhv_cols<8>, grid, kThreads, 0, s, op, p, X, Y);
+    launch_pdl(D, k_blhv<8>, grid, kThreads, 0, s, op, p, X, Y);
   } else {
-    launch_pdl(D, k_blhv_rows<16>, grid, kThreads, 0, s, op, p, X, Y);
-    QED_LAUNCH();
-    launch_pdl(D, k_blhv_cols<16>, grid, kThreads, 0, s, op, p, X, Y);
+    launch_pdl(D, k_blhv<16>, grid, kThreads, 0, s, op, p, X, Y);
   }
   QED_LAUNCH();
 }
@@ -1970,6 +1972,11 @@ int launch_axpby(size_t D, double a, double *y, double b, const double *x, int n
   return grid;
 }
 
+void launch_replay_step(size_t D, double *y, double c1, const double *x1, double c2, const double *x2, double z,
+                        double w, double *psi, cudaStream_t s) {
+  launch_pdl(D, k_replay_step, grid_for(D, device_sms(), 4), kThreads, 0, s, D, y, c1, x1, c2, x2, z, w, psi);
+}
+
 int launch_axpy_dev(size_t D, double *y, const double *x, const double *a_dev, Reducer &r, cudaStream_t s,
                     const int *skip) {
   int grid = std::min(grid_for(D, device_sms(), 4), r.max_blocks);
@@ -2001,10 +2008,11 @@ void launch_finalize_ld(const double *partials, int nblocks, int ld, int n, doub
 }
 
 void launch_block_chol(int p, const double *G, double pivot_min, double *R, double *Rinv, const double *Rprev,
-                       double *B_out, double *Bt_out, double *fail_flag, cudaStream_t s) {
+                       double *B_out, double *Bt_out, double *fail_flag, const double *A, double *host,
+                       cudaStream_t s) {
   if (p < 1 || p > 16) fail(QED_ERR_ARGUMENT, "launch_block_chol: block size outside [1, 16]");
-  launch_pdl(0, k_block_chol, 1, 256, 0, s, p, G, pivot_min, R, Rinv, Rprev, B_out, Bt_out, fail_flag);
-  QED_LAUNCH();
+  launch_pdl(0, k_block_chol, 1, (p * p + 31) / 32 * 32, 0, s, p, G, pivot_min, R, Rinv, Rprev, B_out, Bt_out,
+             fail_flag, A, host);
 }
 
 void launch_swap_scale(size_t D, double *q, double *p, double beta, cudaStream_t s) {

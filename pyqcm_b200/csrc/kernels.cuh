@@ -147,6 +147,9 @@ struct LanczosScalars {
 // y -= (*a_dev) x, with |y|^2 block partials in r.partials; returns the grid size.
 int launch_axpy_dev(size_t D, double *y, const double *x, const double *a_dev, Reducer &r, cudaStream_t s,
                     const int *skip = nullptr);
+// y = (y + c1 x1 + c2 x2) z (x1, x2 may be null), psi += w y
+void launch_replay_step(size_t D, double *y, double c1, const double *x1, double c2, const double *x2, double z,
+                        double w, double *psi, cudaStream_t s);
 // y *= 1 / sqrt(*b2_cur) (0 if that is 0); records alpha_j, beta_j and advances *j.
 void launch_lanczos_advance(size_t D, double *y, const LanczosScalars &ls, cudaStream_t s);
 // Largest sector the one-CTA-per-sector job table takes (the option
@@ -186,12 +189,15 @@ struct BlockOut {
 };
 // Y = a Y + s1 X1 M1 (M1 p x p row-major, device; skipped when X1.v[0] is null;
 // Y is not read when a == 0); gram 1: per-CTA partials of Y^T Y of the result,
-// gram 2: of L^T Y; partials[b * p * p + i * p + c]. Returns the CTA count.
+// gram 2: of L^T Y; partials[b * p * p + i * p + c]. Returns the CTA count. M2 (a ==
+// 0, gram 0): Y = (s1 X1 M1) M2, the inner product as a kernel of its own would leave
+// it. keep false: Y is not written, only its Gram matrix (gram 1).
 int launch_bl_update(size_t D, int p, double a, const BlockOut &Y, double s1, const BlockIn &X1, const double *M1,
-                     int gram, const BlockIn &L, double *partials, int max_blocks, cudaStream_t s);
+                     int gram, const BlockIn &L, double *partials, int max_blocks, cudaStream_t s,
+                     const double *M2 = nullptr, bool keep = true);
 // Y_c = H X_c for the p vectors of a block: the staged single-vector H.v per
-// vector when the sector has packed tables, else one row and one column launch
-// for the whole block (ELL tables, every entry read once per state for all p).
+// vector when the sector has packed tables, else one launch for the whole block
+// (ELL tables, every entry read once per state for all p).
 void launch_block_hv(const HvOperator &op, int p, const BlockIn &X, const BlockOut &Y, Reducer &r, cudaStream_t s);
 
 // out[0..n) = fixed-order sums of partials with row stride ld
@@ -225,9 +231,11 @@ void launch_sef_logdet(int n, int nw, const double *G, const double *V0, const L
 // (one per frequency). partials: 2 n^2 nw lattice_blocks doubles.
 void launch_cpt_projected(int n, int nw, const double *G, const double *V0, const LatticeView &el, const int (&nk3)[3], double *partials, double *Gproj, cudaStream_t s);
 // G = R^T R on the device (p <= 16): R, R^{-1}; *fail = 1 if G is not positive
-// definite or a pivot is below pivot_min; with Rprev, B = R Rprev and B^T
+// definite or a pivot is below pivot_min; with Rprev, B = R Rprev and B^T, and with
+// host (pinned memory) the record [A | B | *fail] there
 void launch_block_chol(int p, const double *G, double pivot_min, double *R, double *Rinv, const double *Rprev,
-                       double *B_out, double *Bt_out, double *fail_flag, cudaStream_t s);
+                       double *B_out, double *Bt_out, double *fail_flag, const double *A, double *host,
+                       cudaStream_t s);
 
 // ---- H.v ------------------------------------------------------------------
 // Row pass: y = (diag + up hops) x - sum_k sub.c[k] sub.z[k]   (x scaled by xs)

@@ -873,8 +873,7 @@ void lanczos_eigenvector(const SectorOp &H, Workspace &ws, const LanczosResult &
       sub.z[1] = pa;
     }
     launch_hv(op, pb, 1.0, pc, sub, 0, ws.red, s);
-    launch_scale(D, pc, 1.0 / beta[j - 1], s);
-    launch_axpby(D, 1.0, psi.p, Z[j], pc, 0, ws.red, s);
+    launch_replay_step(D, pc, 0.0, nullptr, 0.0, nullptr, 1.0 / beta[j - 1], Z[j], psi.p, s);
     std::swap(pa, pb);
     std::swap(pb, pc);
   }
@@ -992,10 +991,9 @@ void lanczos_eigenvector_mixed(const MixedHamiltonian &H, Workspace &ws, const L
   double *pa = A.p, *pb = B.p, *pc = C.p;
   for (int j = 1; j < M; ++j) {
     H.apply_ordered(pb, pc, s);                                 // H v_{j-1}
-    launch_axpby(D, 1.0, pc, -alpha[j - 1], pb, 0, ws.red, s);  // - alpha_{j-1} v_{j-1}
-    if (j >= 2) launch_axpby(D, 1.0, pc, -beta[j - 2], pa, 0, ws.red, s);  // - beta_{j-2} v_{j-2}
-    launch_scale(D, pc, 1.0 / beta[j - 1], s);
-    launch_axpby(D, 1.0, psi.p, Z[j], pc, 0, ws.red, s);
+    // - alpha_{j-1} v_{j-1} - beta_{j-2} v_{j-2}, normalised, into psi
+    launch_replay_step(D, pc, -alpha[j - 1], pb, j >= 2 ? -beta[j - 2] : 0.0, j >= 2 ? pa : nullptr,
+                       1.0 / beta[j - 1], Z[j], psi.p, s);
     std::swap(pa, pb);
     std::swap(pb, pc);
   }
@@ -1225,18 +1223,20 @@ bool block_lanczos_qmatrix(const KrylovOp &H, Workspace &ws, std::vector<DevBuf<
     // W -= V_k A_k (with the gram of the result for the QR)
     nbk = launch_bl_update(D, p, 1.0, W, -1.0, in(Vk), rk, 1, none, part.p, max_blocks, s);
     if ((k + 1) * p < M0) {
-      // W = V_{k+1} B_{k+1}, Cholesky QR twice, through V_{k-1}'s buffer
+      // W = V_{k+1} B_{k+1}, Cholesky QR twice: W R1^{-1} is formed for its Gram
+      // matrix, and again for V_{k+1} = (W R1^{-1}) R2^{-1}, without being stored
       launch_finalize_ld(part.p, nbk, pp, pp, dG, s);
-      launch_block_chol(p, dG, kPivotMin, dR1, dR1i, nullptr, nullptr, nullptr, rk + 2 * pp, s);
-      nbk = launch_bl_update(D, p, 0.0, Vprev, 1.0, in(W), dR1i, 1, none, part.p, max_blocks, s);
+      launch_block_chol(p, dG, kPivotMin, dR1, dR1i, nullptr, nullptr, nullptr, rk + 2 * pp, nullptr, nullptr, s);
+      nbk = launch_bl_update(D, p, 0.0, Vprev, 1.0, in(W), dR1i, 1, none, part.p, max_blocks, s, nullptr, false);
       launch_finalize_ld(part.p, nbk, pp, pp, dG, s);
-      launch_block_chol(p, dG, 0.0, dR2, dR2i, dR1, rk + pp, dBt, rk + 2 * pp, s);
-      launch_bl_update(D, p, 0.0, W, 1.0, in(Vprev), dR2i, 0, none, part.p, max_blocks, s);
+      launch_block_chol(p, dG, 0.0, dR2, dR2i, dR1, rk + pp, dBt, rk + 2 * pp, rk,
+                        hrec + (size_t)ldr * (k & 1), s);
+      launch_bl_update(D, p, 0.0, Vprev, 1.0, in(W), dR1i, 0, none, part.p, max_blocks, s, dR2i);
+    } else {
+      QED_CUDA(cudaMemcpyAsync(hrec + (size_t)ldr * (k & 1), rk, ldr * sizeof(double), cudaMemcpyDeviceToHost, s));
     }
-    QED_CUDA(cudaMemcpyAsync(hrec + (size_t)ldr * (k & 1), rk, ldr * sizeof(double), cudaMemcpyDeviceToHost, s));
     QED_CUDA(cudaEventRecord(ev[k & 1], s));
-    const BlockOut nv = W;  // V_{k+1}
-    W = Vprev;
+    const BlockOut nv = Vprev;  // V_{k+1}, over V_{k-1}
     Vprev = Vk;
     Vk = nv;
   };
