@@ -1006,7 +1006,8 @@ __global__ void __launch_bounds__(256) k_mcf_eval(const McfDesc *desc, const dou
 // thread per state applies every hop to all p vectors, so each table entry is
 // read once per state for the whole block. The up part (with the diagonal) and
 // the down part have accumulators of their own and are added at the end, as when
-// they were two passes through Y. Small sectors are launch-bound, where one launch
+// they were two passes through Y (731,808 states, p = 4: 40 us, in two passes 52).
+// Small sectors are launch-bound, where one launch
 // for the whole block is what counts.
 template <int P>
 __global__ void __launch_bounds__(kThreads) k_blhv(HvOperator op, int p, BlockIn X, BlockOut Y) {
@@ -1198,55 +1199,130 @@ __global__ void __launch_bounds__(kLanczosJobThreads) k_lanczos_start_jobs(const
   if (threadIdx.x == 0) *J.beta_prev = 0.0;
 }
 
-__global__ void __launch_bounds__(kLanczosJobThreads) k_lanczos_jobs(const LanczosJob *__restrict__ jobs) {
+// acc plus one spin's hops of a state, in table order: four entries and their
+// gathers are in flight together
+__device__ __forceinline__ double add_hops(double acc, const uint32_t *ell, uint32_t ld, int cnt,
+                                           const double *vals, const double *x, uint32_t scale) {
+  for (int k = 0; k < cnt; k += 4) {
+    double v[4], g[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (k + j < cnt) {
+        const uint32_t e = ell[(k + j) * ld];
+        v[j] = vals[e & 255u];
+        g[j] = x[(e >> 8) * scale];
+      }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (k + j < cnt) acc += v[j] * g[j];
+  }
+  return acc;
+}
+
+// cta_sum over the CTA's first kLanczosJobThreads threads; every thread gets the total
+__device__ __forceinline__ double job_sum(double v, double *sm) {
+  constexpr int kWarps = kLanczosJobThreads / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < kWarps)
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  __syncthreads();  // previous use of sm is complete
+  if (warp < kWarps && lane == 0) sm[warp] = v;
+  __syncthreads();
+  double t = lane < kWarps ? sm[lane] : 0.0;  // every warp: spares a barrier
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  return __shfl_sync(0xffffffffu, t, 0);
+}
+
+// Lanczos steps of one sector per CTA of T threads. The sums alpha and beta run over
+// kLanczosJobThreads chains (state I belongs to chain I mod kLanczosJobThreads, in
+// increasing order) whatever T is, so that a sector's numbers do not depend on the form
+// that it takes: with T above that, H v is formed by all threads and the chains are
+// added up by the first kLanczosJobThreads in passes of their own, eight loads ahead.
+// Bound by the latency of the gathers, and the largest sectors set the end of a
+// launch: 2692 sectors of up to 63,504 states took 9.2 ms for 16 steps with 256 threads
+// each and one table entry after the other, now 4 to 5 ms (3.5 ms of it the 273 wide
+// sectors, which the narrow ones' launch overlaps). The limit kLanczosWideDim and T =
+// 1024 of the wide form: their whole eigenvalue phase takes 110 ms; with a limit of
+// 8192 139, of 4096 144, with T = 512 and a limit of 16384 120, of 4096 119.
+template <int T>
+__global__ void __launch_bounds__(T) k_lanczos_jobs(const LanczosJob *__restrict__ jobs) {
+  constexpr uint32_t C = kLanczosJobThreads;
   __shared__ LanczosJob J;
-  __shared__ double sm[33];
+  __shared__ double sm[C / 32], vals[2][256];
+  if (T > C) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) J = jobs[blockIdx.x];
   __syncthreads();
-  const uint32_t du = J.op.up.dim, dd = J.op.dn.dim;
-  const uint32_t D = du * dd;
+  const SpinTable up = J.op.up, dn = J.op.dn;
+  for (int i = threadIdx.x; i < min(up.nvals, 256); i += T) vals[0][i] = up.vals[i];
+  for (int i = threadIdx.x; i < min(dn.nvals, 256); i += T) vals[1][i] = dn.vals[i];
+  __syncthreads();
+  const uint32_t du = up.dim, dd = dn.dim;
+  const uint32_t D = du * dd, t0 = threadIdx.x;
+  const int nsteps = J.nsteps;
   double *vp = J.v[J.rot], *vc = J.v[(J.rot + 1) % 3], *w = J.v[(J.rot + 2) % 3];
-  for (int step = 0; step < J.nsteps; ++step) {
-    const double bprev = *J.beta_prev;
+  double bprev = *J.beta_prev;
+  for (int step = 0; step < nsteps; ++step) {
     double sa = 0.0;
-    for (uint32_t I = threadIdx.x; I < D; I += blockDim.x) {
-      const uint32_t u = I % du, d = I / du;
+    for (uint32_t I = t0; I < D; I += T) {
+      const uint32_t d = I / du, u = I - d * du;
       const double x = vc[I];
-      double acc = (J.op.up.diag[u] + J.op.dn.diag[d] + inter_term(J.op.inter, J.op.up.bits[u], J.op.dn.bits[d])) * x;
-      const double *row = vc + (size_t)d * du;
-      for (int k = 0; k < J.op.up.cnt[u]; ++k) {
-        const uint32_t e = J.op.up.ell[(size_t)k * du + u];
-        acc += J.op.up.vals[e & 255u] * row[e >> 8];
-      }
-      for (int k = 0; k < J.op.dn.cnt[d]; ++k) {
-        const uint32_t e = J.op.dn.ell[(size_t)k * dd + d];
-        acc += J.op.dn.vals[e & 255u] * vc[(size_t)(e >> 8) * du + u];
-      }
+      double acc = (up.diag[u] + dn.diag[d] + inter_term(J.op.inter, up.bits[u], dn.bits[d])) * x;
+      acc = add_hops(acc, up.ell + u, du, up.cnt[u], vals[0], vc + d * du, 1);
+      acc = add_hops(acc, dn.ell + d, dd, dn.cnt[d], vals[1], vc + u, du);
       acc -= bprev * vp[I];
       w[I] = acc;
-      sa += x * acc;
+      if (T == C) sa += x * acc;
     }
-    const double a = cta_sum(sa, sm);  // alpha_j = <v_j, w>
+    if (T > C) {
+      __syncthreads();
+      if (t0 < C)
+        for (uint32_t I = t0; I < D; I += 8 * C) {
+          double x[8], y[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const bool in = I + j * C < D;
+            x[j] = in ? vc[I + j * C] : 0.0;
+            y[j] = in ? w[I + j * C] : 0.0;
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) sa += x[j] * y[j];
+        }
+    }
+    const double a = job_sum(sa, sm);  // alpha_j = <v_j, w>
     double sb = 0.0;
-    for (uint32_t I = threadIdx.x; I < D; I += blockDim.x) {
-      const double t = w[I] - a * vc[I];
-      w[I] = t;
-      sb += t * t;
-    }
-    const double b = sqrt(cta_sum(sb, sm));  // beta_j = |w|
+    if (t0 < C)
+      for (uint32_t I = t0; I < D; I += 8 * C) {
+        double x[8], y[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const bool in = I + j * C < D;
+          x[j] = in ? vc[I + j * C] : 0.0;
+          y[j] = in ? w[I + j * C] : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const double t = y[j] - a * x[j];
+          if (I + j * C < D) w[I + j * C] = t;
+          sb += t * t;
+        }
+      }
+    const double b = sqrt(job_sum(sb, sm));  // beta_j = |w|
     const double z = (b > 0.0) ? 1.0 / b : 0.0;
-    for (uint32_t I = threadIdx.x; I < D; I += blockDim.x) w[I] *= z;
-    if (threadIdx.x == 0) {
+    for (uint32_t I = t0; I < D; I += T) w[I] *= z;
+    if (t0 == 0) {
       J.out[step] = a;
       J.out[kLanczosJobMaxSteps + step] = b;
-      *J.beta_prev = b;
     }
-    __syncthreads();  // v_{j+1} and beta_j visible to the whole CTA
+    bprev = b;
+    __syncthreads();  // v_{j+1} visible to the whole CTA
     double *t = vp;
     vp = vc;
     vc = w;
     w = t;
   }
+  if (t0 == 0) *J.beta_prev = bprev;
+  // the narrow sectors' launch overlaps the wide ones' and ends after them
+  if (T == C) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 __global__ void k_swap_scale(size_t D, double *q, double *p, double beta) {
@@ -1996,10 +2072,17 @@ void launch_lanczos_start_jobs(const LanczosJob *jobs, int njobs, cudaStream_t s
   QED_LAUNCH();
 }
 
-void launch_lanczos_jobs(const LanczosJob *jobs, int njobs, cudaStream_t s) {
-  if (njobs <= 0) return;
-  k_lanczos_jobs<<<njobs, kLanczosJobThreads, 0, s>>>(jobs);
-  QED_LAUNCH();
+void launch_lanczos_jobs(const LanczosJob *jobs, int njobs, int nwide, cudaStream_t s) {
+  if (nwide > 0) {
+    k_lanczos_jobs<kLanczosWideThreads><<<nwide, kLanczosWideThreads, 0, s>>>(jobs);
+    QED_LAUNCH();
+  }
+  if (njobs > nwide && nwide > 0) {
+    launch_pdl(0, k_lanczos_jobs<kLanczosJobThreads>, njobs - nwide, kLanczosJobThreads, 0, s, jobs + nwide);
+  } else if (njobs > 0 && nwide == 0) {
+    k_lanczos_jobs<kLanczosJobThreads><<<njobs, kLanczosJobThreads, 0, s>>>(jobs);
+    QED_LAUNCH();
+  }
 }
 
 void launch_finalize_ld(const double *partials, int nblocks, int ld, int n, double *out, cudaStream_t s) {

@@ -166,6 +166,8 @@ size_t lanczos_job_max_dim();
 // rotate once per step. out receives alpha then beta of the launch's steps
 // (2 * kLanczosJobMaxSteps doubles per job).
 constexpr int kLanczosJobThreads = 256;
+constexpr int kLanczosWideThreads = 1024;
+constexpr size_t kLanczosWideDim = 16384;
 constexpr int kLanczosJobMaxSteps = 16;
 struct LanczosJob {
   HvOperator op;
@@ -178,7 +180,9 @@ struct LanczosJob {
 // v_j = normalised random start vector (the values of launch_random for `seed`),
 // v_{j-1} = 0, beta_prev = 0, for every job
 void launch_lanczos_start_jobs(const LanczosJob *jobs, int njobs, cudaStream_t s);
-void launch_lanczos_jobs(const LanczosJob *jobs, int njobs, cudaStream_t s);
+// the first nwide jobs (sectors of at least kLanczosWideDim states, the largest first)
+// by kLanczosWideThreads threads each
+void launch_lanczos_jobs(const LanczosJob *jobs, int njobs, int nwide, cudaStream_t s);
 
 // ---- blocks of p separate vectors (block.cu) ---------------------------------
 struct BlockIn {

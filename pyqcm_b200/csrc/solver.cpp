@@ -616,33 +616,56 @@ void lanczos_energy_batch(std::vector<LanczosBatchItem> &items, Workspace &ws) {
   std::stable_sort(active.begin(), active.end(), [&](int a, int b) { return items[a].H->D > items[b].H->D; });
   std::vector<LanczosJob> batch;
   std::vector<double> hout;
-  while (!active.empty()) {
-    const int na = (int)active.size();
+  std::vector<char> finished(n, 0);
+  std::vector<int> table, steps;  // jobs and steps of the launch under way
+  auto launch = [&] {
+    std::vector<int> todo;
+    for (int i : active)
+      if (!finished[i]) todo.push_back(i);
+    table.swap(todo);
+    const int na = (int)table.size();
     batch.resize(na);
+    steps.resize(na);
+    int wide = 0;  // the table begins with the largest sectors
     for (int a = 0; a < na; ++a) {
-      const int i = active[a];
+      const int i = table[a];
       batch[a] = jobs[i];
-      batch[a].nsteps = run[i].chunk;
+      batch[a].nsteps = steps[a] = run[i].chunk;
       batch[a].rot = run[i].rot;
       batch[a].out = out.p + (size_t)a * 2 * kChunk;
+      run[i].rot = (run[i].rot + run[i].chunk) % 3;
+      run[i].chunk = kChunk;
+      if (items[i].H->D >= kLanczosWideDim) ++wide;
     }
     djobs.upload(batch.data(), na, s);
-    launch_lanczos_jobs(djobs.p, na, s);
+    launch_lanczos_jobs(djobs.p, na, wide, s);
+  };
+  // With many sectors the next chunk is launched before this one's tests, which
+  // then run beside it (64 clusters, 2692 sectors: tests of 4.6 ms beside launches of
+  // 4 to 5 ms); a sector that has finished runs one chunk too many. With few the tests
+  // are short against such a chunk.
+  constexpr int kAheadJobs = 256;
+  launch();
+  for (;;) {
+    const std::vector<int> tab(table), nstep(steps);
+    const int na = (int)tab.size();
     hout.resize((size_t)na * 2 * kChunk);
     out.download(hout.data(), hout.size(), s);
     ws.sync();
+    const bool ahead = na >= kAheadJobs;
+    if (ahead) launch();
     PhaseScope ps_ritz(kPhRitz);
-    std::vector<char> done(na, 0);
     std::vector<std::string> err(na);
     std::vector<int> code(na, 0);
     auto test = [&](int a) {  // the Ritz tests of one sector's chunk, in step order
-      const int i = active[a];
+      const int i = tab[a];
+      if (finished[i]) return;
       Run &R = run[i];
       LanczosResult &res = *items[i].out;
       const double *ha = hout.data() + (size_t)a * 2 * kChunk, *hb = ha + kChunk;
       bool stop = false;
       try {
-        for (int k = 0; k < R.chunk && !stop; ++k) {
+        for (int k = 0; k < nstep[a] && !stop; ++k) {
           res.alpha.push_back(ha[k]);
           res.beta.push_back(hb[k]);
           double last = 1.0;
@@ -668,12 +691,10 @@ void lanczos_energy_batch(std::vector<LanczosBatchItem> &items, Workspace &ws) {
         err[a] = e.what();
         return;
       }
-      R.rot = (R.rot + R.chunk) % 3;
-      R.chunk = kChunk;
       if (stop) {
         res.energy = R.lambda0;
         res.iterations = (int)res.alpha.size();
-        done[a] = 1;
+        finished[i] = 1;
       }
     };
     const ParallelFor &pf = parallel_for_hook();
@@ -681,12 +702,13 @@ void lanczos_energy_batch(std::vector<LanczosBatchItem> &items, Workspace &ws) {
       pf(na, test);
     else
       for (int a = 0; a < na; ++a) test(a);
-    std::vector<int> still;
+    bool more = false;
     for (int a = 0; a < na; ++a) {
       if (code[a]) fail(code[a], err[a]);
-      if (!done[a]) still.push_back(active[a]);
+      more = more || !finished[tab[a]];
     }
-    active.swap(still);
+    if (!more) break;
+    if (!ahead) launch();
   }
 }
 
