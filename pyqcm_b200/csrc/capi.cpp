@@ -195,6 +195,30 @@ const bool g_parallel_for_set = [] {
   return true;
 }();
 
+// The parts of a single solve run over a third pool. A thread that finds it taken by
+// another solve does its parts itself instead of waiting: callers with threads of
+// their own already overlap their solves.
+WorkerPool &part_pool() {
+  static WorkerPool *p = new WorkerPool;
+  return *p;
+}
+
+constexpr int kPartThreads = 8;
+
+const bool g_solve_parts_set = [] {
+  set_solve_parts([](const std::vector<std::function<void(Workspace &)>> &fns) {
+    const int n = (int)fns.size(), hw = (int)std::thread::hardware_concurrency();
+    std::atomic<int> next{0};
+    std::atomic<bool> ok{true};
+    auto work = [&] {
+      for (int i = next++; i < n && ok; i = next++)
+        if (guarded([&] { fns[i](ws()); }) != QED_OK) ok = false;
+    };
+    return part_pool().try_run(std::min({n, hw > 0 ? hw : 8, kPartThreads}) - 1, work) && ok;
+  });
+  return true;
+}();
+
 // The input of a lattice sum on the device: frequencies i w, the k-independent
 // parts of V and the inter-cluster elements (r, c, R, v) as LatticeView wants them
 // (ordered by row, the order of a row's elements kept; the grid's directions by

@@ -3,6 +3,7 @@
 #include "symmetry.hpp"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <iomanip>
 #include <limits>
@@ -931,73 +932,79 @@ void Instance::qmatrix_combine(State &st, bool spin_down, QPart (&parts)[2], Wor
 // symmetry-adapted Hamiltonian (or its full eigensystem below max_dim_full),
 // energy shift and sign, streamline in the irrep's orbital basis.
 void Instance::qmatrix_part_mixed(State &st, bool spin_down, int s, QPart &out, Workspace &ws) {
+  out.e.clear();
+  out.V.clear();
+  out.segs.clear();
+  std::unique_ptr<MixedHamiltonian> own;
+  for (int r = 0; r < model->group->g(); ++r) {
+    QPart::Seg seg;
+    if (qmatrix_irrep(st, spin_down, s, r, own, seg, ws)) out.segs.push_back(std::move(seg));
+  }
+}
+
+// The segment of irrep r, false if it has none. own: the state's own sector, for its
+// basis map, formed when it is first needed.
+bool Instance::qmatrix_irrep(State &st, bool spin_down, int s, int r, std::unique_ptr<MixedHamiltonian> &own,
+                             QPart::Seg &seg, Workspace &ws) {
   const SymmetryGroup &G = *model->group;
   const int pm = 2 * s - 1;
   const int spin = spin_down ? 1 : 0;
   const int ns = model->n_sites;
-  out.e.clear();
-  out.V.clear();
-  out.segs.clear();
-  std::unique_ptr<MixedHamiltonian> Hs;  // the state's own sector, for its basis map
-  int off = 0;
-  for (int r = 0; r < G.g(); ++r) {
-    const int nr = G.site_irrep_dim[r];
-    const int r_off = off;
-    off += nr;
-    if (nr == 0) continue;
-    Sector tsec = shift_sector(st.sec, pm, spin);
-    const int conj_r = sym_conjugate(G, r);
-    tsec.irrep = sym_tensor(G, st.sec.irrep, pm == 1 ? r : conj_r);
-    if (!sector_is_valid(tsec, model->n_orb, G.g())) continue;
-    auto Ht = mixed_sector(tsec, ws);
-    if (Ht->D == 0) continue;
-    if (!Hs) Hs = mixed_sector(st.sec, ws);
-    std::vector<DevBuf<double>> phi;
-    phi.reserve(nr);
-    {
-      PhaseScope ps_cdag(kPhCdag);
-      std::vector<double> coef(ns);
-      for (int i = 0; i < nr; ++i) {
-        for (int a = 0; a < ns; ++a) coef[a] = G.S[(size_t)(r_off + i) * ns + a].real();
-        phi.emplace_back(Ht->D);
-        mixed_cdag(*Hs, *Ht, pm, spin, ns, coef.data(), st.psi.p, phi.back().p, ws.stream);
-      }
-      ws.sync();
+  int r_off = 0;
+  for (int q = 0; q < r; ++q) r_off += G.site_irrep_dim[q];
+  const int nr = G.site_irrep_dim[r];
+  if (nr == 0) return false;
+  Sector tsec = shift_sector(st.sec, pm, spin);
+  const int conj_r = sym_conjugate(G, r);
+  tsec.irrep = sym_tensor(G, st.sec.irrep, pm == 1 ? r : conj_r);
+  if (!sector_is_valid(tsec, model->n_orb, G.g())) return false;
+  auto Ht = mixed_sector(tsec, ws);
+  if (Ht->D == 0) return false;
+  if (!own) own = mixed_sector(st.sec, ws);
+  std::vector<DevBuf<double>> phi;
+  phi.reserve(nr);
+  {
+    PhaseScope ps_cdag(kPhCdag);
+    std::vector<double> coef(ns);
+    for (int i = 0; i < nr; ++i) {
+      for (int a = 0; a < ns; ++a) coef[a] = G.S[(size_t)(r_off + i) * ns + a].real();
+      phi.emplace_back(Ht->D);
+      mixed_cdag(*own, *Ht, pm, spin, ns, coef.data(), st.psi.p, phi.back().p, ws.stream);
     }
-    std::vector<double> ev, Q;
-    int M = 0;
-    bool ok;
-    if ((long)Ht->D < opt_int("max_dim_full")) {
-      // Hamiltonian_Dense::build_Q_matrix: all D poles, Q(k, i) = <phi_i, u_k>
-      std::vector<double> A = Ht->dense(ws.stream), U, ph(Ht->D);
-      if (!sym_eig((int)Ht->D, A, ev, &U)) fail(QED_ERR_INTERNAL, "dense eigensolver did not converge");
-      M = (int)Ht->D;
-      Q.assign((size_t)M * nr, 0.0);
-      for (int i = 0; i < nr; ++i) {
-        phi[i].download(ph.data(), Ht->D, ws.stream);
-        ws.sync();
-        for (int k = 0; k < M; ++k) {
-          const double *uk = U.data() + (size_t)k * Ht->D;
-          double acc = 0.0;
-          for (size_t j = 0; j < Ht->D; ++j) acc += ph[j] * uk[j];
-          Q[(size_t)k * nr + i] = acc;
-        }
-      }
-      ok = true;
-    } else {
-      ok = band_lanczos_qmatrix(KrylovOp(*Ht), ws, phi, ev, Q, M);
-    }
-    if (!ok || M == 0) continue;
-    QPart::Seg seg;
-    seg.r = r;
-    seg.e = std::move(ev);
-    seg.V = std::move(Q);
-    for (auto &x : seg.e) x -= st.energy;
-    if (pm == -1)
-      for (auto &x : seg.e) x = -x;
-    streamline(seg.e, seg.V, nr);
-    out.segs.push_back(std::move(seg));
+    ws.sync();
   }
+  std::vector<double> ev, Q;
+  int M = 0;
+  bool ok;
+  if ((long)Ht->D < opt_int("max_dim_full")) {
+    // Hamiltonian_Dense::build_Q_matrix: all D poles, Q(k, i) = <phi_i, u_k>
+    std::vector<double> A = Ht->dense(ws.stream), U, ph(Ht->D);
+    if (!sym_eig((int)Ht->D, A, ev, &U)) fail(QED_ERR_INTERNAL, "dense eigensolver did not converge");
+    M = (int)Ht->D;
+    Q.assign((size_t)M * nr, 0.0);
+    for (int i = 0; i < nr; ++i) {
+      phi[i].download(ph.data(), Ht->D, ws.stream);
+      ws.sync();
+      for (int k = 0; k < M; ++k) {
+        const double *uk = U.data() + (size_t)k * Ht->D;
+        double acc = 0.0;
+        for (size_t j = 0; j < Ht->D; ++j) acc += ph[j] * uk[j];
+        Q[(size_t)k * nr + i] = acc;
+      }
+    }
+    ok = true;
+  } else {
+    ok = band_lanczos_qmatrix(KrylovOp(*Ht), ws, phi, ev, Q, M);
+  }
+  if (!ok || M == 0) return false;
+  seg.r = r;
+  seg.e = std::move(ev);
+  seg.V = std::move(Q);
+  for (auto &x : seg.e) x -= st.energy;
+  if (pm == -1)
+    for (auto &x : seg.e) x = -x;
+  streamline(seg.e, seg.V, nr);
+  return true;
 }
 
 // The rest of build_qmatrix with a point group: per irrep, hole then electron
@@ -1154,10 +1161,76 @@ void Instance::check_gf_solvable() const {
     fail(QED_ERR_UNSUPPORTED, "merge_states is not in this solver");
 }
 
+namespace {
+// constructed on first use: the library installs the hook from another translation
+// unit's static initialiser, which may run before this one's
+SolveParts &solve_parts_hook() {
+  static SolveParts f;
+  return f;
+}
+}  // namespace
+
+void set_solve_parts(SolveParts f) { solve_parts_hook() = std::move(f); }
+
+// The Q-matrices of all states by their parts (hole and electron, and each irrep of a
+// point group) at the same time, on streams and host threads of their own; false if
+// that is not done, or failed: the parts are then formed one after the other, with the
+// errors that this gives. A part of up to kPartStates states is a chain of kernels too
+// short to fill the GPU, with host work between them: eight parts of the 3x4 cluster
+// with both mirrors (37,000 states each) bring a solve from 88 to 51 ms, the two of the
+// plaquette with eight bath orbitals (731,808 states) from 40 to 36. Beyond, a part
+// fills the GPU by itself, and several would hold several times its memory.
+constexpr size_t kPartStates = 1u << 20;
+bool Instance::qmatrices_at_once(Workspace &ws) {
+  if (!solve_parts_hook()) return false;
+  for (auto &x : states)
+    if (sector_dim(x->sec) > kPartStates) return false;
+  struct Job {
+    State *st;
+    bool sd;
+    QPart parts[2];
+    std::vector<std::array<std::pair<bool, QPart::Seg>, 2>> irreps;
+  };
+  const int g = has_group() ? model->group->g() : 0;
+  std::vector<std::unique_ptr<Job>> jobs;
+  std::vector<std::unique_ptr<MixedHamiltonian>> own(states.size());
+  std::vector<std::function<void(Workspace &)>> fns;
+  for (size_t i = 0; i < states.size(); ++i) {
+    State *st = states[i].get();
+    if (g) own[i] = mixed_sector(st->sec, ws);
+    for (int sd = 0; sd < ((mix & mixing::up_down) ? 2 : 1); ++sd) {
+      jobs.emplace_back(new Job{st, sd != 0, {}, {}});
+      Job *j = jobs.back().get();
+      j->irreps.resize(g);
+      for (int s = 0; s < 2; ++s) {
+        if (!g) fns.push_back([this, j, s](Workspace &w) { qmatrix_part(*j->st, j->sd, s, j->parts[s], w); });
+        for (int r = 0; r < g; ++r)
+          fns.push_back([this, j, s, r, &own, i](Workspace &w) {
+            auto &out = j->irreps[r][s];
+            out.first = qmatrix_irrep(*j->st, j->sd, s, r, own[i], out.second, w);
+          });
+      }
+    }
+  }
+  ws.sync();  // the states and their bases are complete
+  if (fns.size() < 2 || !solve_parts_hook()(fns)) return false;
+  for (auto &j : jobs) {
+    for (int s = 0; s < 2; ++s)
+      for (int r = 0; r < g; ++r)
+        if (j->irreps[r][s].first) j->parts[s].segs.push_back(std::move(j->irreps[r][s].second));
+    qmatrix_combine(*j->st, j->sd, j->parts, ws);
+  }
+  return true;
+}
+
 void Instance::green_solve(Workspace &ws) {
   if (gf_solved) return;
   if (!gs_solved) low_energy_states(ws);
   check_gf_solvable();
+  if (!use_cf && !use_mcf && qmatrices_at_once(ws)) {
+    finish_gf();
+    return;
+  }
   for (auto &x : states) {
     for (int sd = 0; sd < ((mix & mixing::up_down) ? 2 : 1); ++sd) {
       if (use_cf) build_cf(*x, sd != 0, ws);

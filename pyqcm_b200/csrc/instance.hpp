@@ -91,6 +91,12 @@ struct QPart {
   std::vector<Seg> segs;
 };
 
+// Runs the functions, each with the Workspace of the thread that has it, and waits for
+// all of them; false if they could not run beside one another or one failed (the
+// library's worker pool; absent until it is installed).
+using SolveParts = std::function<bool(const std::vector<std::function<void(Workspace &)>> &)>;
+void set_solve_parts(SolveParts f);
+
 struct Instance {
   int label = 0;
   std::shared_ptr<Model> model;
@@ -194,6 +200,9 @@ struct Instance {
   // the symmetry-adapted Hamiltonian of a sector (models with a point group)
   std::unique_ptr<MixedHamiltonian> mixed_sector(const Sector &s, Workspace &ws) const;
   void qmatrix_part_mixed(State &st, bool spin_down, int s, QPart &out, Workspace &ws);
+  bool qmatrix_irrep(State &st, bool spin_down, int s, int r, std::unique_ptr<MixedHamiltonian> &own, QPart::Seg &seg,
+                     Workspace &ws);
+  bool qmatrices_at_once(Workspace &ws);
   void qmatrix_combine_mixed(State &st, bool spin_down, QPart (&parts)[2], Workspace &ws);
 };
 

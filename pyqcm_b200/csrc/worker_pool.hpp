@@ -19,6 +19,18 @@ class WorkerPool {
  public:
   void run(int extra, const std::function<void()> &work) {
     std::lock_guard<std::mutex> serial(run_mtx_);
+    run_locked(extra, work);
+  }
+  // the same unless another call has the pool: then nothing, and false
+  bool try_run(int extra, const std::function<void()> &work) {
+    std::unique_lock<std::mutex> serial(run_mtx_, std::try_to_lock);
+    if (!serial) return false;
+    run_locked(extra, work);
+    return true;
+  }
+
+ private:
+  void run_locked(int extra, const std::function<void()> &work) {
     {
       std::lock_guard<std::mutex> l(m_);
       while ((int)threads_ < extra) {
@@ -36,8 +48,6 @@ class WorkerPool {
     done_.wait(l, [&] { return active_ == 0; });
     job_ = nullptr;
   }
-
- private:
   void loop(int idx) {
     uint64_t seen = 0;
     std::unique_lock<std::mutex> l(m_);
