@@ -1177,7 +1177,7 @@ void set_solve_parts(SolveParts f) { solve_parts_hook() = std::move(f); }
 // that is not done, or failed: the parts are then formed one after the other, with the
 // errors that this gives. A part of up to kPartStates states is a chain of kernels too
 // short to fill the GPU, with host work between them: eight parts of the 3x4 cluster
-// with both mirrors (37,000 states each) bring a solve from 88 to 51 ms, the two of the
+// with both mirrors (183,000 states each) bring a solve from 88 to 51 ms, the two of the
 // plaquette with eight bath orbitals (731,808 states) from 40 to 36. Beyond, a part
 // fills the GPU by itself, and several would hold several times its memory.
 constexpr size_t kPartStates = 1u << 20;
