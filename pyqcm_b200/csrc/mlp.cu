@@ -54,7 +54,8 @@ inline int pad16(int x) { return (x + 15) / 16 * 16; }
 // back - is all there is: a training step was 32 launches with four-CTA products
 // whose rounds waited for one another, 210 us for a batch of 256; with the rounds
 // in flight, 32-column tiles, no transposes and the elementwise work in the
-// epilogues it is eight launches and 61 us. Every sum keeps its
+// epilogues it is eight launches and 61 us, 54 with each launch beginning as its
+// predecessor ends. Every sum keeps its
 // order, so that both train to the same bits.
 
 constexpr int kUmmaM = 128;       // rows of a tile = TMEM lanes (cta_group::1)
@@ -184,7 +185,6 @@ __device__ void umma_tile(const GemmJob &j, int tile, unsigned char *sm) {
     umma_stage(sb + st * b_bytes, j.B, j.ldb, j.b_mn, n0, j.bn, j.N, k0, kc);
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  for (int r = 0; r < min(kUmmaStages, rounds); ++r) fill(r);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tslot)),
                  "r"(ncols)
@@ -196,6 +196,10 @@ __device__ void umma_tile(const GemmJob &j, int tile, unsigned char *sm) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar[st])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // the previous launch's results from here on (tensor memory is taken before the
+  // next launch may begin, so no two launches' tiles wait for one another's)
+  pdl_begin();
+  for (int r = 0; r < min(kUmmaStages, rounds); ++r) fill(r);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -299,6 +303,7 @@ struct ColJob {
 constexpr int kColRows = 256;
 
 __device__ void column_sums(const ColJob &j, int cta, float *sm) {
+  pdl_begin();
   const int f0 = cta * 32, lane = threadIdx.x & 31, f = f0 + lane;
   float *wr = sm + kColRows * 32;
   float s = 0.0f;
@@ -413,8 +418,7 @@ void run_stage(const StageJobs &jobs, cudaStream_t s) {
     grid += j.tiles;
   }
   for (const ColJob &j : jobs.c) grid += j.ctas;
-  k_mlp_stage<<<grid, kUmmaThreads, smem, s>>>(jobs);
-  QED_LAUNCH();
+  launch_pdl(0, k_mlp_stage, grid, kUmmaThreads, smem, s, jobs);
 }
 
 // The output layer, one warp per row b: y = sum_k H[b][k] w[k] + b0 (fp32
@@ -423,6 +427,7 @@ void run_stage(const StageJobs &jobs, cudaStream_t s) {
 // the optimiser's step count, advanced here once per training step.
 __global__ void k_head(int rows, int F, const bf16 *H, const bf16 *w, const float *b0, float *y, const float *t,
                        float *dy, float *loss_terms, const float *Z, float *dZ, bf16 *dZh, int *step) {
+  pdl_begin();
   if (step && blockIdx.x == 0 && threadIdx.x == 0) *step += 1;
   const int b = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x % 32;
   if (b >= rows) return;
@@ -450,6 +455,7 @@ __global__ void k_head(int rows, int F, const bf16 *H, const bf16 *w, const floa
 // lives on the device so that a captured step can be replayed.
 __global__ void k_adam(int n, float *w, const float *g, float *m, float *v, bf16 *wh, const int *step, float lr,
                        float b1, float b2, float eps, const unsigned char *mask) {
+  pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   if (mask && !mask[i]) return;  // padding stays zero
@@ -624,7 +630,7 @@ struct MLP {
   // y = network output
   void forward(int rows) {
     hidden(rows);
-    k_head<<<(rows * 32 + 255) / 256, 256, 0, s>>>(rows, W, H[2].p, Ph(6), P(7), y.p, nullptr, nullptr, nullptr,
+    launch_pdl(0, k_head, (rows * 32 + 255) / 256, 256, 0, s, rows, W, H[2].p, Ph(6), P(7), y.p, nullptr, nullptr, nullptr,
                                                   nullptr, nullptr, nullptr, nullptr);
     QED_LAUNCH();
   }
@@ -634,7 +640,7 @@ struct MLP {
   // dZ_l^T prev, db_l and dZ_{l-1} = dZ_l W_l GELU'(Z_{l-1}) all read dZ_l only.
   void gradients(int rows, bool training) {
     hidden(rows);
-    k_head<<<(rows * 32 + 255) / 256, 256, 0, s>>>(rows, W, H[2].p, Ph(6), P(7), y.p, T.p, dy.p, lt.p, Z[2].p,
+    launch_pdl(0, k_head, (rows * 32 + 255) / 256, 256, 0, s, rows, W, H[2].p, Ph(6), P(7), y.p, T.p, dy.p, lt.p, Z[2].p,
                                                   dZ[2].p, dZh[2].p, training ? step.p : nullptr);
     QED_LAUNCH();
     for (int l = 2; l >= 0; --l) {
@@ -658,7 +664,7 @@ struct MLP {
   }
 
   void adam(float lr) {
-    k_adam<<<blocks_for(n_par), 256, 0, s>>>((int)n_par, p.p, g.p, m.p, v.p, ph.p, step.p, lr, 0.9f, 0.999f,
+    launch_pdl(0, k_adam, blocks_for(n_par), 256, 0, s, (int)n_par, p.p, g.p, m.p, v.p, ph.p, step.p, lr, 0.9f, 0.999f,
                                               1e-8f, mask.p);
     QED_LAUNCH();
   }
