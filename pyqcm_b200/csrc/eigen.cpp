@@ -73,6 +73,29 @@ bool ql_implicit(int n, double *d, double *e, Rot &&rot) {
   return true;
 }
 
+// QL on (d, e) with the rotations accumulated on the m rows of Q; sorted eigenvalues
+// into w, the rows into Z (column-major m x n)
+bool ql_rows(int n, int m, std::vector<double> &d, std::vector<double> &e, std::vector<double> &Q,
+             std::vector<double> &w, std::vector<double> &Z) {
+  bool ok = ql_implicit(n, d.data(), e.data(), [&](int i, double c, double s) {
+    double *ci = Q.data() + (size_t)m * i, *cj = ci + m;
+    for (int r = 0; r < m; ++r) {
+      const double f = cj[r];
+      cj[r] = s * ci[r] + c * f;
+      ci[r] = c * ci[r] - s * f;
+    }
+  });
+  if (!ok) return false;
+  std::vector<int> idx(n);
+  std::iota(idx.begin(), idx.end(), 0);
+  std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return d[x] < d[y]; });
+  for (int k = 0; k < n; ++k) {
+    w[k] = d[idx[k]];
+    std::copy(Q.data() + (size_t)m * idx[k], Q.data() + (size_t)m * (idx[k] + 1), Z.data() + (size_t)m * k);
+  }
+  return true;
+}
+
 }  // namespace
 
 bool tridiag_eig(int n, std::vector<double> &d, std::vector<double> e, std::vector<double> *z) {
@@ -257,20 +280,21 @@ void tridiag_lowest_track(int n, const double *alpha, const double *beta, RitzTr
   fallback();
 }
 
-bool sym_eig(int n, const std::vector<double> &A, std::vector<double> &w, std::vector<double> *V) {
-  w.assign(n, 0.0);
-  if (n == 0) return true;
+namespace {
+
+// Householder reduction of the symmetric A to tridiagonal (d, e); reflect(k, v, beta2) is
+// called for every reflection I - beta2 v v^T (v zero up to k), so that a caller can
+// accumulate all of Q or some of its rows.
+template <class Reflect>
+void tridiagonalise(int n, const std::vector<double> &A, std::vector<double> &d, std::vector<double> &e,
+                    Reflect &&reflect) {
   // Householder reduction A = Q T Q^T, working on a full copy; column-major a(i,j) = a[i + n*j].
   std::vector<double> a(A);
   auto at = [&](int i, int j) -> double & { return a[i + (size_t)n * j]; };
   for (int j = 0; j < n; ++j)
     for (int i = 0; i < j; ++i) at(i, j) = at(j, i);  // symmetrise from the lower triangle
-  std::vector<double> d(n), e(n, 0.0);
-  std::vector<double> Q;
-  if (V) {
-    Q.assign((size_t)n * n, 0.0);
-    for (int i = 0; i < n; ++i) Q[i + (size_t)n * i] = 1.0;
-  }
+  d.assign(n, 0.0);
+  e.assign(n, 0.0);
   std::vector<double> v(n), p(n), q(n);
   for (int k = 0; k < n - 2; ++k) {
     // Householder vector annihilating a(k+2:n, k)
@@ -289,12 +313,14 @@ bool sym_eig(int n, const std::vector<double> &A, std::vector<double> &w, std::v
     if (vv == 0.0) { e[k] = at(k + 1, k); continue; }
     double beta2 = 2.0 / vv;
     // p = beta2 * A v (trailing block), K = beta2/2 * v^T p, q = p - K v
-    for (int i = k; i < n; ++i) {  // A symmetric: row i of A == column i
-      double s = 0.0;
-      const double *ci = a.data() + (size_t)n * i;
-      for (int j = k + 1; j < n; ++j) s += ci[j] * v[j];
-      p[i] = beta2 * s;
+    // (A is exactly symmetric: column by column, each sum still in order of j)
+    std::fill(p.begin() + k, p.end(), 0.0);
+    for (int j = k + 1; j < n; ++j) {
+      const double *cj = a.data() + (size_t)n * j;
+      const double vj = v[j];
+      for (int i = k; i < n; ++i) p[i] += cj[i] * vj;
     }
+    for (int i = k; i < n; ++i) p[i] *= beta2;
     double K = 0.0;
     for (int i = k + 1; i < n; ++i) K += v[i] * p[i];
     K *= 0.5 * beta2;
@@ -302,21 +328,36 @@ bool sym_eig(int n, const std::vector<double> &A, std::vector<double> &w, std::v
     // A <- A - v q^T - q v^T on rows/cols k..n-1 (v[k] = 0)
     for (int j = k; j < n; ++j)
       for (int i = k; i < n; ++i) at(i, j) -= v[i] * q[j] + q[i] * v[j];
-    if (V) {  // Q <- Q H = Q - beta2 (Q v) v^T
-      std::fill(q.begin(), q.end(), 0.0);
-      for (int j = k + 1; j < n; ++j) {
-        const double *cj = Q.data() + (size_t)n * j;
-        for (int i = 0; i < n; ++i) q[i] += cj[i] * v[j];
-      }
-      for (int j = k + 1; j < n; ++j) {
-        double *cj = Q.data() + (size_t)n * j;
-        double f = beta2 * v[j];
-        for (int i = 0; i < n; ++i) cj[i] -= q[i] * f;
-      }
-    }
+    reflect(k, v, beta2);
   }
   for (int i = 0; i < n; ++i) d[i] = at(i, i);
   for (int i = 0; i < n - 1; ++i) e[i] = at(i + 1, i);
+}
+
+}  // namespace
+
+bool sym_eig(int n, const std::vector<double> &A, std::vector<double> &w, std::vector<double> *V) {
+  w.assign(n, 0.0);
+  if (n == 0) return true;
+  std::vector<double> d, e, Q, q(n);
+  if (V) {
+    Q.assign((size_t)n * n, 0.0);
+    for (int i = 0; i < n; ++i) Q[i + (size_t)n * i] = 1.0;
+  }
+  tridiagonalise(n, A, d, e, [&](int k, const std::vector<double> &v, double beta2) {
+    if (!V) return;
+    // Q <- Q H = Q - beta2 (Q v) v^T
+    std::fill(q.begin(), q.end(), 0.0);
+    for (int j = k + 1; j < n; ++j) {
+      const double *cj = Q.data() + (size_t)n * j;
+      for (int i = 0; i < n; ++i) q[i] += cj[i] * v[j];
+    }
+    for (int j = k + 1; j < n; ++j) {
+      double *cj = Q.data() + (size_t)n * j;
+      double f = beta2 * v[j];
+      for (int i = 0; i < n; ++i) cj[i] -= q[i] * f;
+    }
+  });
   std::vector<double> Z;
   if (!tridiag_eig(n, d, e, V ? &Z : nullptr)) return false;
   w = d;
@@ -332,6 +373,25 @@ bool sym_eig(int n, const std::vector<double> &A, std::vector<double> &w, std::v
       }
   }
   return true;
+}
+
+bool sym_eig_rows(int n, const std::vector<double> &A, int m, std::vector<double> &w, std::vector<double> &Z) {
+  m = std::min(m, n);
+  w.assign(n, 0.0);
+  Z.assign((size_t)m * n, 0.0);
+  if (n == 0) return true;
+  std::vector<double> d, e, Q((size_t)m * n, 0.0), q(m);
+  for (int r = 0; r < m; ++r) Q[r + (size_t)m * r] = 1.0;
+  tridiagonalise(n, A, d, e, [&](int k, const std::vector<double> &v, double beta2) {
+    std::fill(q.begin(), q.end(), 0.0);
+    for (int j = k + 1; j < n; ++j)
+      for (int r = 0; r < m; ++r) q[r] += Q[r + (size_t)m * j] * v[j];
+    for (int j = k + 1; j < n; ++j) {
+      const double f = beta2 * v[j];
+      for (int r = 0; r < m; ++r) Q[r + (size_t)m * j] -= q[r] * f;
+    }
+  });
+  return ql_rows(n, m, d, e, Q, w, Z);
 }
 
 namespace {
@@ -540,23 +600,7 @@ bool band_eig_rows(int n, int b, std::vector<double> A, int m, std::vector<doubl
   };
   std::vector<double> d, e;
   band_to_tridiagonal(n, b, A, d, e, rot_cols);
-  bool ok = ql_implicit(n, d.data(), e.data(), [&](int i, double c, double s) {
-    double *ci = Q.data() + (size_t)m * i, *cj = ci + m;
-    for (int r = 0; r < m; ++r) {
-      const double f = cj[r];
-      cj[r] = s * ci[r] + c * f;
-      ci[r] = c * ci[r] - s * f;
-    }
-  });
-  if (!ok) return false;
-  std::vector<int> idx(n);
-  std::iota(idx.begin(), idx.end(), 0);
-  std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return d[x] < d[y]; });
-  for (int k = 0; k < n; ++k) {
-    w[k] = d[idx[k]];
-    std::copy(Q.data() + (size_t)m * idx[k], Q.data() + (size_t)m * (idx[k] + 1), Z.data() + (size_t)m * k);
-  }
-  return true;
+  return ql_rows(n, m, d, e, Q, w, Z);
 }
 
 bool complex_inverse(int n, std::complex<double> *a) {

@@ -89,6 +89,9 @@ bool band_lowest(int n, int b, const std::vector<double> &B, BandLowest &st, dou
 // only the first p rows (Q = P U with P zero beyond the p start vectors).
 bool band_eig_rows(int n, int b, std::vector<double> A, int m, std::vector<double> &w, std::vector<double> &Z);
 
+// The same of a symmetric matrix (full column-major array, lower triangle read).
+bool sym_eig_rows(int n, const std::vector<double> &A, int m, std::vector<double> &w, std::vector<double> &Z);
+
 // In-place inverse of a complex n x n column-major matrix (Gauss-Jordan with
 // partial pivoting). Returns false if singular.
 bool complex_inverse(int n, std::complex<double> *a);
