@@ -5,7 +5,7 @@ TEST INFRASTRUCTURE ONLY: used by the oracle's build recipe callers
 
 The reference checkout is named by the environment variable PYQCM_REFERENCE_ROOT.
 When it is unset, the checkout location of this build container is used if it
-exists (that is where the oracle is compiled; the GPU box only loads the prebuilt
+holds the sources (that is where the oracle is compiled; the GPU box only loads the prebuilt
 oracle/_ref library). `reference_root(required=True)` raises with a clear message
 when neither is there.
 """
@@ -25,7 +25,7 @@ def reference_root(required: bool = False) -> str | None:
         if not os.path.isdir(root):
             raise RuntimeError(f"{ENV}={root} is not a directory")
         return root
-    if os.path.isdir(_CONTAINER_DEFAULT):
+    if os.path.isdir(os.path.join(_CONTAINER_DEFAULT, "src_ed")):
         return _CONTAINER_DEFAULT
     if required:
         raise RuntimeError(f"the reference checkout is needed here: set {ENV} to its directory")
