@@ -4,9 +4,8 @@ TEST INFRASTRUCTURE ONLY: used by the oracle's build recipe callers
 (__graft_entry__.build, tests/conftest.py) and the golden-fixture generators.
 
 The reference checkout is named by the environment variable PYQCM_REFERENCE_ROOT.
-When it is unset, the checkout location of this build container is used if it
-holds the sources (that is where the oracle is compiled; the GPU box only loads the prebuilt
-oracle/_ref library). `reference_root(required=True)` raises with a clear message
+When it is unset, a default location is used if it holds the sources (that is
+where the oracle is compiled; elsewhere the prebuilt oracle/_ref library is loaded). `reference_root(required=True)` raises with a clear message
 when neither is there.
 """
 from __future__ import annotations
