@@ -578,6 +578,13 @@ void lanczos_energy_batch(std::vector<LanczosBatchItem> &items, Workspace &ws) {
   const long max_iter = opt_int("max_iter_lanczos");
   cudaStream_t s = ws.stream;
   constexpr int kChunk = kLanczosJobMaxSteps;
+  // A chunk launched ahead of its tests (below) may still run when these end the
+  // loop, or throw. It reads the sectors' tables, which callers free on streams of
+  // their own: nothing may be in flight once this function is left.
+  struct Drain {
+    cudaStream_t s;
+    ~Drain() { cudaStreamSynchronize(s); }
+  };
   // one arena for the three vectors of every sector (32-byte aligned blocks)
   std::vector<size_t> off(n);
   size_t tot = 0;
@@ -588,6 +595,7 @@ void lanczos_energy_batch(std::vector<LanczosBatchItem> &items, Workspace &ws) {
   }
   DevBuf<double> arena(std::max<size_t>(tot, 1)), bprev(n), out((size_t)n * 2 * kChunk);
   DevBuf<LanczosJob> djobs(n);
+  const Drain drain{s};
   std::vector<LanczosJob> jobs(n);
   struct Run {
     RitzTracker tracker;
