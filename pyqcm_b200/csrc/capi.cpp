@@ -134,6 +134,12 @@ template <class F> int guarded(F &&f) {
   }
 }
 
+// Waits for the calling thread's stream, after a task that failed on it: what the
+// task's caller frees next is freed on another stream.
+void drain_thread() {
+  if (cudaStream_t s = alloc_stream()) cudaStreamSynchronize(s);
+}
+
 std::shared_ptr<Instance> instance(int label) {
   std::lock_guard<std::mutex> l(g_reg);
   auto it = g_instances.find(label);
@@ -162,6 +168,7 @@ template <class F> int run_batch(int n, int threads, F &&fn) {
     for (int i = next++; i < n; i = next++) {
       int rc = guarded([&] { fn(i); });
       if (rc != QED_OK) {
+        drain_thread();
         int expected = QED_OK;
         if (first_code.compare_exchange_strong(expected, rc)) {
           std::lock_guard<std::mutex> l(emtx);
@@ -207,14 +214,10 @@ constexpr int kPartThreads = 8;
 
 const bool g_solve_parts_set = [] {
   set_solve_parts([](const std::vector<std::function<void(Workspace &)>> &fns) {
-    const int n = (int)fns.size(), hw = (int)std::thread::hardware_concurrency();
-    std::atomic<int> next{0};
-    std::atomic<bool> ok{true};
-    auto work = [&] {
-      for (int i = next++; i < n && ok; i = next++)
-        if (guarded([&] { fns[i](ws()); }) != QED_OK) ok = false;
-    };
-    return part_pool().try_run(std::min({n, hw > 0 ? hw : 8, kPartThreads}) - 1, work) && ok;
+    const int hw = (int)std::thread::hardware_concurrency();
+    return run_parts(
+        part_pool(), std::min(hw > 0 ? hw : 8, kPartThreads), (int)fns.size(),
+        [&](int i) { return guarded([&] { fns[i](ws()); }) == QED_OK; }, drain_thread);
   });
   return true;
 }();

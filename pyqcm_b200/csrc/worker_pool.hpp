@@ -1,5 +1,7 @@
 // A pool of host threads that live for the whole process (host code).
 #pragma once
+#include <algorithm>
+#include <atomic>
 #include <condition_variable>
 #include <cstdint>
 #include <functional>
@@ -69,5 +71,24 @@ class WorkerPool {
   int wanted_ = 0, active_ = 0;
   uint64_t gen_ = 0;
 };
+
+// Runs call(0) .. call(n - 1) on up to `threads` threads of the pool and waits for
+// them; false if the pool was taken (then none ran) or a call returned false (then no
+// further one is started). After a failed call its thread runs drain() before the
+// caller goes on: a call that was left by an exception may have work on its thread's
+// stream that reads what the caller frees next.
+template <class Call, class Drain>
+bool run_parts(WorkerPool &pool, int threads, int n, Call &&call, Drain &&drain) {
+  std::atomic<int> next{0};
+  std::atomic<bool> ok{true};
+  auto work = [&] {
+    for (int i = next++; i < n && ok; i = next++)
+      if (!call(i)) {
+        ok = false;
+        drain();
+      }
+  };
+  return pool.try_run(std::max(1, std::min(threads, n)) - 1, work) && ok;
+}
 
 }  // namespace qed
