@@ -397,12 +397,22 @@ __global__ void k_cpt_reduce(int n, int nblk, double nk, const double *__restric
   }
 }
 
-// Wavevector batches per warp: as many as leave about eight CTAs per SM over
-// all frequencies (forming V0 G costs a CTA about N batches' work), at most 16.
+// Wavevector batches per warp: as many as leave about eight CTAs per SM over all
+// frequencies (forming V0 G costs a CTA about N batches' work), at most 8, where the
+// CTAs' start is a few per cent of their work. Beyond that the grid has CTAs enough,
+// and more batches only bound their number: at most kLatMaxBlocks per frequency, or
+// 32 per SM over all of them, since each leaves a partial sum of n^2 entries in memory
+// (100 frequencies of dimension 16 on 128^3 wavevectors: 27 MB; at 8 batches 13 GB).
+// The time is the same: 64 frequencies, 128^2 wavevectors, dimension 10, whole calls:
+// 971 and 1769 us (log det, inverse), at 8 batches 983 and 1798; dimension 16: 2430
+// and 6865, 2505 and 6815.
+constexpr unsigned long long kLatCtas = 148 * 8, kLatMaxBlocks = 64;
 int batches_per_warp(int n, int nw, unsigned long long nk) {
-  const unsigned long long per = (unsigned long long)kLatWarps * (32 / n);
-  const unsigned long long all = (nk + per - 1) / per * (unsigned long long)std::max(nw, 1);
-  return (int)std::min<unsigned long long>(8, std::max<unsigned long long>(1, all / (148 * 8)));
+  const unsigned long long per = (unsigned long long)kLatWarps * (32 / n), w = (unsigned long long)std::max(nw, 1);
+  const unsigned long long one = (nk + per - 1) / per;  // CTAs per frequency at one batch per warp
+  const unsigned long long few = std::min<unsigned long long>(8, std::max<unsigned long long>(1, one * w / kLatCtas));
+  const unsigned long long most = std::max(kLatMaxBlocks, 4 * kLatCtas / w);
+  return (int)std::max(few, (one + most - 1) / most);
 }
 
 using LatticeFn = void (*)(const double *, const double *, LatticeTerms, unsigned long long, int, double *);
