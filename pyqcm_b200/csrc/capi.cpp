@@ -227,9 +227,14 @@ const bool g_solve_parts_set = [] {
 // (ordered by row, the order of a row's elements kept; the grid's directions by
 // size, R reduced to the grid; the phase of the grid's offset, the same along every
 // direction in units of a grid step, in v). One pinned copy and one allocation
-// instead of five each: the sums themselves take some ten microseconds.
+// instead of five each: the sums themselves take some ten microseconds. The pinned
+// buffer stays with the thread, so inputs above kPinnedDoubles (1 MB) are staged in
+// memory of the call's own: 1200 frequencies of dimension 8, 788 us a call through
+// pinned memory, 804 so.
 struct LatticeInput {
+  static constexpr size_t kPinnedDoubles = size_t(1) << 17;
   DevBuf<double> buf;
+  std::vector<double> own;
   std::vector<cplx> z;
   const double *dz, *V0;
   LatticeView el;
@@ -244,7 +249,8 @@ struct LatticeInput {
     // [elements | z | V0 | first element of each row], in doubles
     const size_t ne = std::max(nel, 1) * (sizeof(LatticeElement) / sizeof(double)), nz = 2 * (size_t)nw;
     const size_t total = ne + nz + nV0 + (dim + 2) / 2 + 1;
-    double *h = W.pinned(total);
+    if (total > kPinnedDoubles) own.resize(total);
+    double *h = own.empty() ? W.pinned(total) : own.data();
     LatticeElement *he = reinterpret_cast<LatticeElement *>(h);
     int *first = reinterpret_cast<int *>(h + ne + nz + nV0);
     std::fill(first, first + dim + 1, 0);
