@@ -261,7 +261,9 @@ std::vector<Instance::SusQ> Instance::susceptibility_qmatrices(const std::string
       std::vector<DevBuf<double>> b(1);
       b[0].alloc(H.D);
       SubList none;
-      launch_hv(O.op, st->psi.p, 1.0, b[0].p, none, 0, ws.red, ws.stream);  // b = O psi
+      HvOperator op = O.op;
+      op.keep_order = true;  // b starts a recurrence
+      launch_hv(op, st->psi.p, 1.0, b[0].p, none, 0, ws.red, ws.stream);  // b = O psi
       SusQ q;
       q.st = st.get();
       int M = 0;
