@@ -1724,7 +1724,13 @@ int hv_cols_grid(const HvOperator &op) {
   const int g = (int)std::max<size_t>(1, std::min<size_t>(nitems, (size_t)device_sms() * 8));
   // the staged pass runs one CTA per column pair, at most one per SM
   const int g16 = (int)std::max<size_t>(1, std::min<size_t>(du / 2, (size_t)device_sms()));
-  return std::max({g, g16, fused_applies(op) ? fused_grid(op) : 1, tile_applies(op) ? tile_grid(op) : 1});
+  return std::max(g, g16);
+}
+
+// The most rows of partial sums that a product of this operator writes, whichever
+// form it takes.
+int hv_partial_rows(const HvOperator &op) {
+  return std::max({hv_cols_grid(op), fused_applies(op) ? fused_grid(op) : 1, tile_applies(op) ? tile_grid(op) : 1});
 }
 
 std::atomic<bool> g_staged_used{false};  // set by the first staged H.v launch
@@ -2175,9 +2181,9 @@ double *noalloc_partials_address() {
 
 void launch_hv_dots_noalloc(const HvOperator &op, const double *x, double *y, double *dots,
                             cudaStream_t s) {
-  // The grid the column pass launches (grid-stride, at most 8 CTAs per SM);
-  // each CTA needs one row of the scratch.
-  const size_t want = (size_t)hv_cols_grid(op);
+  // Each CTA of the launch that takes the sums (grid-stride, at most 8 CTAs per SM)
+  // needs one row of the scratch.
+  const size_t want = (size_t)hv_partial_rows(op);
   if (want > (size_t)kHvColsMaxBlocks)
     fail(QED_ERR_MEMORY, "H.v without allocation: the column pass needs " + std::to_string(want) +
                              " partial-sum rows, the fixed scratch holds " +
