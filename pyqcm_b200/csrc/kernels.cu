@@ -1798,7 +1798,9 @@ void launch_hv_rows(const HvOperator &op, const double *x, double xs, double *y,
 
 int launch_hv_cols(const HvOperator &op, const double *x, double xs, double *y, int red_mask,
                    Reducer &r, cudaStream_t s) {
-  const bool vec2 = (op.up.dim % 2 == 0);
+  // the two-column form reads and writes 16 bytes at a time: rows of even length and
+  // vectors that start on such a boundary (a caller's may be a view at an odd offset)
+  const bool vec2 = op.up.dim % 2 == 0 && aligned16(x) && aligned16(y);
   int grid = hv_cols_grid(op);
   if (red_mask && grid > r.max_blocks) grid = r.max_blocks;
   const bool cg = hv_variant() & 1;
