@@ -486,10 +486,8 @@ __global__ void k_gather(int rows, int n_in, int ld, const float *X, const float
   if (T) Tp[b] = T[src];
 }
 
-inline int blocks_for(size_t n, int threads = 256) {
-  size_t g = (n + threads - 1) / threads;
-  return (int)std::min<size_t>(std::max<size_t>(g, 1), 148 * 16);
-}
+// CTAs of a kernel with a thread per element
+inline int blocks_for(size_t n, int threads = 256) { return (int)std::max<size_t>((n + threads - 1) / threads, 1); }
 
 }  // namespace
 
