@@ -3,6 +3,7 @@
 #include "mixed.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -12,6 +13,7 @@
 #include <limits>
 #include <map>
 #include <system_error>
+#include <thread>
 
 #include "bank_order.hpp"
 #include "eigen.hpp"
@@ -1616,7 +1618,8 @@ bool band_lanczos_qmatrix(const KrylovOp &H, Workspace &ws, std::vector<DevBuf<d
   // threads of their own, up to kAheadTests behind the recurrence, and are read in
   // order: the result is that of the first that stops, as if none had run ahead. Four
   // such halves, alone at the end, were 330 of the 465 ms that the Green functions of
-  // 64 clusters took; these now take 180 to 215.
+  // 64 clusters took; these now take 180 to 215. All recurrences together have as many
+  // such threads as the host has cores: a test beyond them runs when it is read.
   constexpr int kAheadDim = 96, kAheadTests = 8;
   struct Ahead {
     int j;
@@ -1646,11 +1649,24 @@ bool band_lanczos_qmatrix(const KrylovOp &H, Workspace &ws, std::vector<DevBuf<d
       if (!sym_eig(jc, Hpr, ev, nullptr)) fail(QED_ERR_INTERNAL, "projected eigensolver failed");
       return ev[0];
     };
-    try {
-      pending.push_back({jc, std::async(std::launch::async, lowest_of)});
-    } catch (const std::system_error &) {  // no thread to be had: when it is read
-      pending.push_back({jc, std::async(std::launch::deferred, lowest_of)});
+    static const int cores = std::max(1, (int)std::thread::hardware_concurrency());
+    static std::atomic<int> running{0};
+    struct Slot {  // one of the threads, kept until its future is read and the thread has ended
+      bool on = ++running <= cores;
+      Slot() { if (!on) --running; }
+      Slot(Slot &&o) : on(o.on) { o.on = false; }
+      ~Slot() { if (on) --running; }
+    };
+    Slot slot;
+    if (slot.on) {
+      try {
+        pending.push_back(
+            {jc, std::async(std::launch::async, [lowest_of, slot = std::move(slot)] { return lowest_of(); })});
+        return settle(kAheadTests - 1);
+      } catch (const std::system_error &) {  // no thread to be had
+      }
     }
+    pending.push_back({jc, std::async(std::launch::deferred, std::move(lowest_of))});
     return settle(kAheadTests - 1);
   };
   // Device-resident steps: while nothing has been deflated (nd == 0) and the
