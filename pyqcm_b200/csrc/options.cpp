@@ -77,8 +77,9 @@ struct Table {
     // sectors): 44.7 solves/s at 65536, 24.8 at 2^20 (one CTA is too little there).
     i["lanczos_job_max_dim"] = 65536;
     // solver options: the symmetry-adapted (mixed-basis) Hamiltonian of a sector
-    // is stored unless that takes more than mixed_csr_max_gb gigabytes at 12 B an entry;
-    // then (or always, with mixed_on_the_fly) every product recomputes its entries.
+    // is stored unless that takes more than mixed_csr_max_gb gigabytes (the packed form
+    // 4 B a slot, padding included, 5 above 2^24 states; CSR 12 B an entry); then (or
+    // always, with mixed_on_the_fly) every product recomputes its entries.
     b["mixed_on_the_fly"] = false;
     d["mixed_csr_max_gb"] = 32.0;
     i["lanczos_graphs_min_dim"] = 131072;
