@@ -922,7 +922,7 @@ MixedHamiltonian::MixedHamiltonian(const SymmetryGroup &G, const MixedTerms &t, 
 // Builds the packed form where it applies (see mixed.hpp); false: nothing done.
 bool MixedHamiltonian::pack(const MixedTerms &t, const uint32_t *ustr, const uint32_t *dstr, cudaStream_t s) {
   const int g = group.g, N = group.N;
-  if ((long)D < opt_int("max_dim_full") || opt_bool("mixed_on_the_fly")) return false;
+  if ((long)D < opt_int("max_dim_full") || opt_bool("mixed_on_the_fly") || (opt_int("mixed_variant") & 1)) return false;
   if ((g & (g - 1)) || du >= (1u << 24) || dd >= (1u << 24) || t.r.empty()) return false;
   int nlog = 0;
   while ((1 << nlog) < g) ++nlog;
@@ -965,7 +965,7 @@ bool MixedHamiltonian::pack(const MixedTerms &t, const uint32_t *ustr, const uin
   uint64_t slots = 0;
   QED_CUDA(cudaMemcpyAsync(&slots, slice_off.p + nslices, sizeof(slots), cudaMemcpyDeviceToHost, s));
   QED_CUDA(cudaStreamSynchronize(s));
-  const bool wide = D > (1u << 24);
+  const bool wide = D > (1u << 24) || (opt_int("mixed_variant") & 2);
   if ((wide ? 5.0 : 4.0) * 32.0 * (double)slots > opt_double("mixed_csr_max_gb") * 1e9) {
     slice_off.release();
     slice_up.release();

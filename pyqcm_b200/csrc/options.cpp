@@ -82,6 +82,10 @@ struct Table {
     // always, with mixed_on_the_fly) every product recomputes its entries.
     b["mixed_on_the_fly"] = false;
     d["mixed_csr_max_gb"] = 32.0;
+    // solver option: form of the stored matrix (bits: 1 CSR instead of packed, 2 the
+    // packed form's codes apart from its columns, as above 2^24 states). The recurrences
+    // give the same bits in every form; for checks of that.
+    i["mixed_variant"] = 0;
     i["lanczos_graphs_min_dim"] = 131072;
     // solver option: launch variant of the H.v kernels of sectors without the
     // staged kernels (bits: 1 L2-only column gathers, 2 row pass with four
