@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <array>
+#include <chrono>
 #include <cmath>
 #include <iomanip>
 #include <limits>
@@ -1215,7 +1216,11 @@ bool Instance::qmatrices_at_once(Workspace &ws) {
     }
   }
   ws.sync();  // the states and their bases are complete
-  if (fns.size() < 2 || !solve_parts_hook()(fns)) return false;
+  if (fns.size() < 2) return false;
+  const auto t0 = std::chrono::steady_clock::now();
+  if (!solve_parts_hook()(fns)) return false;
+  if (profiling())
+    profile_add(kPhPartsAtOnce, std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count());
   for (auto &j : jobs) {
     for (int s = 0; s < 2; ++s)
       for (int r = 0; r < g; ++r)

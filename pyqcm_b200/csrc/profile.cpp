@@ -13,7 +13,7 @@ const char *kNames[kPhCount] = {"sector setup",       "GS Lanczos (eigenvalue)",
                                 "band Lanczos checks", "band projected eigensystem", "continued fractions",
                                 "GS Ritz tests (in GS eigenvalue)", "block Lanczos recurrence",
                                 "block Lanczos fallbacks", "ground-state operator averages",
-                                "GS batched small sectors"};
+                                "GS batched small sectors", "Q-matrix parts at the same time"};
 
 struct Totals {
   std::atomic<long long> ns[kPhCount];

@@ -21,6 +21,7 @@ enum Phase {
   kPhBlockFallback, // block recurrence abandoned for the band one (count)
   kPhAverages,      // operator averages of the ground state (cluster_averages)
   kPhGsBatch,       // batched eigenvalue pass of small sectors (inside kPhGsLanczos)
+  kPhPartsAtOnce,   // Q-matrices of a solve by their parts at the same time
   kPhCount
 };
 
