@@ -32,6 +32,7 @@
 
 #include "common.hpp"
 #include "kernels.cuh"
+#include "reciprocal.cuh"
 
 namespace qed {
 
@@ -67,17 +68,6 @@ __device__ __forceinline__ Cplx cmul(Cplx a, Cplx b) {
 __device__ __forceinline__ void csub(Cplx &a, Cplx l, Cplx q) {
   a.x = fma(-l.x, q.x, fma(l.y, q.y, a.x));
   a.y = fma(-l.x, q.y, fma(-l.y, q.x, a.y));
-}
-// 1 / d for d > 0 to about an ulp: the hardware's approximation (rcp.approx, at
-// least 20 bits) and two Newton-Raphson steps r += r (1 - d r), each doubling
-// the number of correct bits. A division instead costs a call with its checks
-// per elimination step. Zero, infinite and subnormal d take the division.
-__device__ __forceinline__ double reciprocal(double d) {
-  if (!(d > 1e-290 && d < 1e290)) return 1.0 / d;
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  r = fma(r, fma(-d, r, 1.0), r);
-  return fma(r, fma(-d, r, 1.0), r);
 }
 __device__ __forceinline__ Cplx shfl(Cplx a, int src) {
   return {__shfl_sync(0xffffffffu, a.x, src), __shfl_sync(0xffffffffu, a.y, src)};
