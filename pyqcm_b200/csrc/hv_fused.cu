@@ -1,7 +1,7 @@
 // One-launch H.v for small sectors (see launch_hv_fused).
 //
 // The two-pass kernels (kernels.cu) read and write y twice and launch twice; on a
-// sector of 10^3 to 10^5 states the launches, the serial chain count -> entry ->
+// sector of up to 10^5 states the launches, the serial chain count -> entry ->
 // value -> gather of each pass, and a grid of one or two rows per CTA are what
 // they cost, not bytes. Here a work item is NV rows by a chunk of up strings. The
 // item's rows are staged in shared memory (NV values side by side, so that an up
@@ -31,7 +31,6 @@ namespace {
 constexpr int kFusedThreads = 512;
 constexpr int kFusedHops = 256;  // at most 255 hops per string
 constexpr int kAhead = 4;        // up-hop entries loaded ahead
-constexpr int kDeep = 4;         // down-hop gathers in flight
 
 struct DnHop {
   double v;
@@ -202,8 +201,8 @@ int fused_sms() {
   return n;
 }
 
-constexpr size_t kFusedSmemMax = 200 * 1024;
 constexpr uint32_t kFusedMaxRow = 4096;  // up strings: every chunk stages whole rows
+constexpr size_t kFusedSmemMax = 2 * kFusedMaxRow * sizeof(double);
 
 struct FusedPlan {
   int nv;  // rows per work item
@@ -222,24 +221,22 @@ void plan_chunks(const HvOperator &op, int rows, FusedPlan &p) {
   p.threads = std::min<uint32_t>(kFusedThreads, ((p.chunk + turns - 1) / turns + 31) / 32 * 32);
 }
 
-// Rows per work item: more of them share table entries, fewer keep the SMs full
-// (sectors of 213444 states: 11.9, 10.3 and 11.7 us for 1, 2 and 4 rows).
+// Rows per work item: two share table entries, one keeps the SMs full (sectors of
+// 213444 states: 11.9 and 10.3 us for 1 and 2 rows, 11.7 for 4). With rows of at most
+// kFusedMaxRow strings both fit shared memory.
 FusedPlan plan_fused(const HvOperator &op) {
   const uint64_t D = (uint64_t)op.up.dim * op.dn.dim;
   FusedPlan p;
-  p.nv = D >= 600000 ? 4 : (D >= 150000 ? 2 : 1);
-  while (p.nv > 1 && ((uint32_t)p.nv > op.dn.dim || (size_t)op.up.dim * p.nv * 8 > kFusedSmemMax / 2)) p.nv /= 2;
+  p.nv = D >= 150000 && op.dn.dim >= 2 ? 2 : 1;
   plan_chunks(op, p.nv, p);
   return p;
 }
 
-FusedFn fused_fn(int nv) {
-  return nv == 4 ? k_hv_fused<4> : (nv == 2 ? k_hv_fused<2> : k_hv_fused<1>);
-}
+FusedFn fused_fn(int nv) { return nv == 2 ? k_hv_fused<2> : k_hv_fused<1>; }
 
 void set_fused_attributes() {
   static const bool once = [] {
-    for (int nv : {1, 2, 4})
+    for (int nv : {1, 2})
       QED_CUDA(cudaFuncSetAttribute(fused_fn(nv), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmemMax));
     return true;
   }();
@@ -252,7 +249,7 @@ int grid_of(const FusedPlan &p) { return (int)std::min<uint32_t>(p.items, 8u * (
 
 bool fused_applies(const HvOperator &op) {
   const uint64_t D = (uint64_t)op.up.dim * op.dn.dim;
-  return D >= kFusedMinStates && D <= kFusedMaxStates && op.up.dim <= kFusedMaxRow;
+  return D <= kFusedMaxStates && op.up.dim <= kFusedMaxRow;
 }
 
 int fused_grid(const HvOperator &op) { return grid_of(plan_fused(op)); }
