@@ -213,8 +213,22 @@ def cpu_baseline_sample():
     return H
 
 
+def reference_unavailable():
+    """Why the reference's code cannot be timed here (one line), or None if it can."""
+    from oracle import ref, refpath
+    if ref.available():
+        return None
+    if refpath.reference_root() is None:
+        return f"the reference's library is not built ({ref.LIB_PATH}) and its sources are not here"
+    return f"the reference's library is not built: {ref.LIB_PATH} (make -C oracle/ref_build)"
+
+
 def run_reference(args, world, rank):
     if rank != 0:
+        return
+    why = reference_unavailable()
+    if why:
+        print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
         return
     H = cpu_baseline_sample()
     D = H.dim
@@ -417,6 +431,9 @@ def batch_line(workload, batch, threads, steps, warmup, impl, world=1, rank=0, l
     if impl == "reference":
         if rank != 0:
             return None
+        why = reference_unavailable()
+        if why:
+            return {"impl": "reference", "unavailable": why}
         import multiprocessing as mp
         cores = os.cpu_count() or 8
         n = min(len(probs), cores)
@@ -541,7 +558,9 @@ VCA_REF_POINT = (7.0, 0.15, 0.0)  # (U, M', dmu) of the reference's timed Omega 
 def vca_reference_sample():
     """One Potthoff-functional evaluation of the 2x5 VCA workload by the reference's
     own lattice layer (the compiled oracle; ED ground state + Green function + the
-    fixed grid) on one host core: (seconds, Omega)."""
+    fixed grid) on one host core: (seconds, Omega), or None without that library."""
+    if reference_unavailable():
+        return None
     from oracle import ref
     from pyqcm_b200 import vca
     from pyqcm_b200 import workloads as W
@@ -604,12 +623,21 @@ def vca_line(n_points, epochs, threads, Us=(5.0, 7.0, 9.0), local=0):
     t_sur = sum(r["surrogate_s"] for r in runs)
     t_ed = sum(r["ed_only_s"] for r in runs)
     om_here = float(ev(np.array([VCA_REF_POINT]))[0])
-    t_ref, om_ref = vca_reference_sample()
+    sample = vca_reference_sample()
     n_ed = sum(r["ed_only_omega_evals"] for r in runs)
     # what the surrogate costs in full, and after how many searches it pays for itself
     t_fixed = t_data + t_train
     gain = (t_ed - t_sur) / len(Us)
     breakeven = (t_fixed / gain) if gain > 0 else None
+    cpu = None
+    if sample:
+        t_ref, om_ref = sample
+        cpu = {"value": t_ref * n_ed, "unit": "s", "cores": 1, "kind": "reference",
+               "sample": f"one Potthoff-functional evaluation by the reference's compiled lattice "
+                         f"layer at (U, M', dmu) = {VCA_REF_POINT} took {t_ref:.2f} s on one host "
+                         f"core; value = that x the {n_ed} evaluations of the ED-only searches",
+               "omega_reference": om_ref, "omega_this_solver": om_here,
+               "omega_abs_diff": abs(om_ref - om_here)}
     return {"metric": "VCA wall time, surrogate-guided (same stationary point as ED-only within 1e-8)",
             "value": t_sur, "unit": "s", "n_gpus": 1, "steps": len(Us), "warmup": 0,
             "ms_per_step": 1e3 * t_sur / len(Us), "higher_is_better": False, "scaling": "replicas",
@@ -623,12 +651,7 @@ def vca_line(n_points, epochs, threads, Us=(5.0, 7.0, 9.0), local=0):
             "speedup_including_training": t_ed / (t_fixed + t_sur),
             "breakeven_searches": breakeven,
             "max_grad_norm": max(max(r["grad_norm_ed_only"], r["grad_norm_surrogate"]) for r in runs),
-            "cpu_baseline": {"value": t_ref * n_ed, "unit": "s", "cores": 1, "kind": "reference",
-                             "sample": f"one Potthoff-functional evaluation by the reference's compiled lattice "
-                                       f"layer at (U, M', dmu) = {VCA_REF_POINT} took {t_ref:.2f} s on one host "
-                                       f"core; value = that x the {n_ed} evaluations of the ED-only searches",
-                             "omega_reference": om_ref, "omega_this_solver": om_here,
-                             "omega_abs_diff": abs(om_ref - om_here)},
+            "cpu_baseline": cpu,
             "max_omega_abs_diff": max(r["omega_abs_diff"] for r in runs),
             "training": {"data_seconds": t_data, "omega_per_second": n_points / t_data,
                          "train_seconds": t_train, "first_loss": float(losses[0]), "last_loss": float(losses[-1])},
