@@ -3,7 +3,6 @@
 #include "mixed.hpp"
 
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -12,11 +11,11 @@
 #include <future>
 #include <limits>
 #include <map>
-#include <system_error>
 #include <thread>
 
 #include "bank_order.hpp"
 #include "eigen.hpp"
+#include "worker_pool.hpp"
 #include "options.hpp"
 #include "profile.hpp"
 
@@ -1537,6 +1536,14 @@ void block_lanczos_mcf(const KrylovOp &H, Workspace &ws, const double *Q0, int p
   ws.sync();
 }
 
+namespace {
+// the dense convergence tests of all band recurrences
+TaskQueue<double> &test_queue() {
+  static TaskQueue<double> *q = new TaskQueue<double>(std::max(1, (int)std::thread::hardware_concurrency()));
+  return *q;
+}
+}  // namespace
+
 bool band_lanczos_qmatrix(const KrylovOp &H, Workspace &ws, std::vector<DevBuf<double>> &phi,
                           std::vector<double> &evals, std::vector<double> &Q, int &Mout) {
   const size_t D = H.D;
@@ -1615,11 +1622,11 @@ bool band_lanczos_qmatrix(const KrylovOp &H, Workspace &ws, std::vector<DevBuf<d
   // After a deflation in a small sector the recurrence can go on for hundreds of
   // steps (a space of 90 states, 372 steps) with a dense test of milliseconds every p
   // of them, where p steps take half of one. Such tests (from kAheadDim on) run on
-  // threads of their own, up to kAheadTests behind the recurrence, and are read in
+  // other threads, up to kAheadTests behind the recurrence, and are read in
   // order: the result is that of the first that stops, as if none had run ahead. Four
   // such halves, alone at the end, were 330 of the 465 ms that the Green functions of
-  // 64 clusters took; these now take 180 to 215. All recurrences together have as many
-  // such threads as the host has cores: a test beyond them runs when it is read.
+  // 64 clusters took; these now take 180 to 215. All recurrences together share one
+  // thread per core of the host.
   constexpr int kAheadDim = 96, kAheadTests = 8;
   struct Ahead {
     int j;
@@ -1644,29 +1651,11 @@ bool band_lanczos_qmatrix(const KrylovOp &H, Workspace &ws, std::vector<DevBuf<d
     std::vector<double> Hpr((size_t)jc * jc);
     for (int c = 0; c < jc; ++c)
       for (int r = 0; r < jc; ++r) Hpr[(size_t)r + (size_t)jc * c] = T(r, c);
-    auto lowest_of = [jc, Hpr = std::move(Hpr)] {
-      std::vector<double> ev;
-      if (!sym_eig(jc, Hpr, ev, nullptr)) fail(QED_ERR_INTERNAL, "projected eigensolver failed");
-      return ev[0];
-    };
-    static const int cores = std::max(1, (int)std::thread::hardware_concurrency());
-    static std::atomic<int> running{0};
-    struct Slot {  // one of the threads, kept until its future is read and the thread has ended
-      bool on = ++running <= cores;
-      Slot() { if (!on) --running; }
-      Slot(Slot &&o) : on(o.on) { o.on = false; }
-      ~Slot() { if (on) --running; }
-    };
-    Slot slot;
-    if (slot.on) {
-      try {
-        pending.push_back(
-            {jc, std::async(std::launch::async, [lowest_of, slot = std::move(slot)] { return lowest_of(); })});
-        return settle(kAheadTests - 1);
-      } catch (const std::system_error &) {  // no thread to be had
-      }
-    }
-    pending.push_back({jc, std::async(std::launch::deferred, std::move(lowest_of))});
+    pending.push_back({jc, test_queue().submit([jc, Hpr = std::move(Hpr)] {
+                         std::vector<double> ev;
+                         if (!sym_eig(jc, Hpr, ev, nullptr)) fail(QED_ERR_INTERNAL, "projected eigensolver failed");
+                         return ev[0];
+                       })});
     return settle(kAheadTests - 1);
   };
   // Device-resident steps: while nothing has been deflated (nd == 0) and the

@@ -4,8 +4,11 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstdint>
+#include <deque>
 #include <functional>
+#include <future>
 #include <mutex>
+#include <system_error>
 #include <thread>
 
 namespace qed {
@@ -70,6 +73,55 @@ class WorkerPool {
   size_t threads_ = 0;
   int wanted_ = 0, active_ = 0;
   uint64_t gen_ = 0;
+};
+
+// A queue of independent tasks, taken in order by threads that are started as they are
+// needed, up to `most`, and live for the rest of the process (like a WorkerPool, it is
+// never destroyed). Without any thread a task runs where it is submitted.
+template <class T> class TaskQueue {
+ public:
+  explicit TaskQueue(int most) : most_(most) {}
+  std::future<T> submit(std::function<T()> f) {
+    std::packaged_task<T()> t(std::move(f));
+    std::future<T> r = t.get_future();
+    std::unique_lock<std::mutex> l(m_);
+    if (idle_ <= (int)q_.size() && threads_ < most_) {
+      try {
+        std::thread([this] { loop(); }).detach();
+        ++threads_;
+      } catch (const std::system_error &) {  // no thread to be had
+      }
+    }
+    if (!threads_) {
+      l.unlock();
+      t();
+      return r;
+    }
+    q_.push_back(std::move(t));
+    cv_.notify_one();
+    return r;
+  }
+
+ private:
+  void loop() {
+    std::unique_lock<std::mutex> l(m_);
+    for (;;) {
+      ++idle_;
+      cv_.wait(l, [&] { return !q_.empty(); });
+      --idle_;
+      std::packaged_task<T()> t = std::move(q_.front());
+      q_.pop_front();
+      l.unlock();
+      t();
+      t = std::packaged_task<T()>();  // what it holds goes with it
+      l.lock();
+    }
+  }
+  const int most_;
+  std::mutex m_;
+  std::condition_variable cv_;
+  std::deque<std::packaged_task<T()>> q_;
+  int threads_ = 0, idle_ = 0;
 };
 
 // Runs call(0) .. call(n - 1) on up to `threads` threads of the pool and waits for
