@@ -8,10 +8,12 @@
 
 namespace qed {
 
-// Inter-spin density-density terms of one state (see InterSpin).
+// Inter-spin density-density terms of one state (see InterSpin). MASKED false: without
+// mode 4, for kernels whose operator has it as mode 2.
+template <bool MASKED = true>
 __device__ __forceinline__ double inter_term(const InterSpin &it, uint32_t up, uint32_t dn) {
   if (it.mode == 1) return it.u * (double)__popc(up & dn);
-  if (it.mode == 4) return it.sum[__popc(up & dn & it.mask)];
+  if (MASKED && it.mode == 4) return it.sum[__popc(up & dn & it.mask)];
   double s = 0.0;
   if (it.mode == 2) {
     uint32_t w = up & dn;
