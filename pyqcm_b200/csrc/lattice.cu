@@ -6,11 +6,15 @@
 //   V(k) = V0 + sum_e v_e exp(2 pi i k.R_e) at (r_e, c_e)   (set_V, src_qcm/CPT.cpp:22-64).
 // A matrix of dimension N (a template argument, 1..16) belongs to N lanes of a
 // warp, lane r holding row r in registers; a warp works on 32 / N matrices at
-// once and a CTA on one frequency. V0 G - 1 does not depend on k: the CTA forms
+// once and a CTA on one frequency. V0 G does not depend on k: the CTA forms
 // it once in shared memory, and a lane only adds its own elements' rows,
 //   row r += sum_{e: r_e = r} v_e exp(2 pi i k.R_e) G[c_e, :],
 // N multiplications per element instead of the N^3 of the whole product (the
-// elements couple neighbouring super cells: two or three per boundary site).
+// elements couple neighbouring super cells: two or three per boundary site). The 1 is
+// subtracted last, per wavevector: V0 G is small against it, and the rounding of
+// V0 G - 1, formed once, would be the same for all wavevectors and stay in their mean
+// (30 cases of dimension 2 to 12 against 80-bit values: 1.5e-15 so, 4.5e-16 now, 1.2e-15
+// with V(k) G - 1 formed per wavevector; 221 us a kernel so, 234 now).
 // Gaussian elimination with partial pivoting then needs no row exchanges: the
 // pivot lane is the largest |re| + |im| among the lanes not used yet (a
 // maximum passed round the matrix's lanes) and its row goes round by shuffles.
@@ -18,13 +22,13 @@
 // What bounds it: the shuffles (4 per broadcast complex entry; the pipe they
 // share with shared memory is busy 53 % of the time) and the latency of the
 // elimination's serial chain (22 warps per SM, two instructions per cycle).
-// On a B200, 64 x 4096 matrices of dimension 10: 216 us, and 1537 us with one
+// On a B200, 64 x 4096 matrices of dimension 10: 234 us, and 1537 us with one
 // thread per matrix holding V, V G and the factors in local memory; the averages
-// of 64 x 1024 matrices of dimension 4: 17 us, and 354 us in 64 CTAs of 64
+// of 64 x 1024 matrices of dimension 4: 19 us, and 354 us in 64 CTAs of 64
 // threads. On the way: a sincospi per element and wavevector, divisions and a
 // redux.sync per elimination step 293 us; the phase table and fewer registers
 // 272 us; Newton-Raphson reciprocals and fused multiply-adds 254 us; the pivot
-// search by shuffles 216 us.
+// search by shuffles 216 to 221 us; the 1 per wavevector 234 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -94,20 +98,20 @@ struct GridPoint {
   }
 };
 
-// G of one frequency and +-(V0 G - 1) in shared memory, rows padded to N + 1
+// G of one frequency and +-V0 G in shared memory, rows padded to N + 1
 // entries so that lanes reading different rows hit different banks.
 template <int N> struct LatticeTile {
   static constexpr int kLd = N + 1;
   double2 g[N * kLd], w[N * kLd];
 
-  // sign = 1: V0 G - 1, sign = -1: 1 - V0 G; G and V0 column-major
+  // w = sign V0 G; G and V0 column-major
   __device__ void load(const double *__restrict__ G, const double *__restrict__ V0, double sign) {
     for (int t = threadIdx.x; t < N * N; t += blockDim.x)
       g[(t % N) * kLd + t / N] = make_double2(G[2 * t], G[2 * t + 1]);
     __syncthreads();
     for (int t = threadIdx.x; t < N * N; t += blockDim.x) {
       const int r = t % N, b = t / N;
-      double sr = (r == b) ? -1.0 : 0.0, si = 0.0;
+      double sr = 0.0, si = 0.0;
       for (int c = 0; c < N; ++c) {
         const double xr = V0[2 * (r + N * c)], xi = V0[2 * (r + N * c) + 1];
         const double2 y = g[c * kLd + b];
@@ -155,6 +159,9 @@ template <int N> struct LatticeTile {
         csub(a[b], p, Cplx{y.x, y.y});
       }
     }
+#pragma unroll
+    for (int b = 0; b < N; ++b)
+      if (b == r) a[b].x -= sign;
   }
 };
 
