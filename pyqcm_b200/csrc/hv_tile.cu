@@ -253,8 +253,29 @@ void set_tile_attributes() {
 
 }  // namespace
 
+// Work of a pass's fullest SM over an even share of it.
+double tile_unevenness(uint32_t n, uint32_t m) {
+  const TilePlan p = plan_tiles(n, m);
+  const uint32_t sms = (uint32_t)tile_sms(), items = p.ntile * p.nchunk;
+  return (double)((items + sms - 1) / sms) * sms * kTile / ((double)m * p.nchunk);
+}
+
+// Where the tiled form is the faster one, from 812 sectors of 11 to 28 sites against the
+// two-pass and staged kernels. Below kTileAlwaysStates they gain 1.0 to 2.0x (but for
+// 0.93x at 2925 x 351 with six hops a string at most). Above, tiles that leave most SMs idle in a last wave lose: 171 tiles on 148 SMs at 1365 x
+// 1365 states 49 to 68 us against 46 to 62, 1365 x 3003 110 to 151 against 101 to 139.
+// For rows of even length that takes an almost empty wave in both passes (mean
+// unevenness 1.78 0.94x, 1.61 1.01x). For odd ones, whose columns are read and written 8
+// bytes at a time, an unevenness of 1.3 (1.18 gains up to 1.4x, 1.34 0.95x), and vectors
+// that leave L2 (3003 x 2002 states 1.15x, 3003 x 3432 0.88x).
 bool tile_applies(const HvOperator &op) {
-  return op.up.tile_max && op.dn.tile_max && (uint64_t)op.up.dim * op.dn.dim >= kTileMinStates;
+  constexpr uint64_t kTileAlwaysStates = 1700000, kTileOddStates = 8000000;
+  const uint32_t du = op.up.dim, dd = op.dn.dim;
+  const uint64_t D = (uint64_t)du * dd;
+  if (!op.up.tile_max || !op.dn.tile_max || D < kTileMinStates) return false;
+  if (D < kTileAlwaysStates) return true;
+  const double uneven = 0.5 * (tile_unevenness(du, dd) + tile_unevenness(dd, du));
+  return du % 2 == 0 ? uneven < 1.7 : uneven < 1.25 && D < kTileOddStates;
 }
 
 int tile_grid(const HvOperator &op) { return (int)plan_tiles(op.up.dim, op.dn.dim).grid; }
