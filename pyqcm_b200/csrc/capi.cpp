@@ -222,18 +222,31 @@ const bool g_solve_parts_set = [] {
   return true;
 }();
 
+// Whether V(k) is stored for every wavevector before a lattice sum (LatticeView). Each of
+// the sum's frequencies then reads an entry of V(k) where it would otherwise form the
+// phases of all its elements. With long-range hops the elements are many: 64 frequencies,
+// 64 x 64 wavevectors, dimension 4, whole calls: 16 elements a row 131 us, 276 without
+// (216 with one thread per matrix, which shared the phases of a wavevector's elements
+// between its rows); 64 a row 209, 856 and 472. At three elements a row the two forms
+// break even (dimension 2 to 12: 76 to 457 us stored, 79 to 473 not; on 16 x 16
+// wavevectors 61 to 107, 59 to 108).
+bool stored_entries(int dim, int nel, int entries, double nk) {
+  constexpr double kMostBytes = 512e6;
+  return nel > 3 * dim && 16.0 * nk * entries <= kMostBytes;
+}
+
 // The input of a lattice sum on the device: frequencies i w, the k-independent
 // parts of V and the inter-cluster elements (r, c, R, v) as LatticeView wants them
-// (ordered by row, the order of a row's elements kept; the grid's directions by
-// size, R reduced to the grid; the phase of the grid's offset, the same along every
-// direction in units of a grid step, in v). One pinned copy and one allocation
-// instead of five each: the sums themselves take some ten microseconds. The pinned
-// buffer stays with the thread, so inputs above kPinnedDoubles (1 MB) are staged in
-// memory of the call's own: 1200 frequencies of dimension 8, 788 us a call through
-// pinned memory, 804 so.
+// (ordered by row, the order of a row's elements kept, or that of an entry's in the
+// stored form; the grid's directions by size, R reduced to the grid; the phase of the
+// grid's offset, the same along every direction in units of a grid step, in v). One
+// pinned copy and one allocation instead of five each: the sums themselves take some ten
+// microseconds. The pinned buffer stays with the thread, so inputs above kPinnedDoubles
+// (1 MB) are staged in memory of the call's own: 1200 frequencies of dimension 8, 788 us
+// a call through pinned memory, 804 so.
 struct LatticeInput {
   static constexpr size_t kPinnedDoubles = size_t(1) << 17;
-  DevBuf<double> buf;
+  DevBuf<double> buf, vk;
   std::vector<double> own;
   std::vector<cplx> z;
   const double *dz, *V0;
@@ -246,18 +259,38 @@ struct LatticeInput {
     int dir[3] = {0, 1, 2};
     std::stable_sort(dir, dir + 3, [&](int a, int b) { return given[a] < given[b]; });
     for (int i = 0; i < 3; ++i) nk[i] = given[dir[i]];
-    // [elements | z | V0 | first element of each row], in doubles
+    std::vector<int> at(nel), lead((size_t)dim * dim, -1);
+    int entries = 0;
+    for (int e = 0; e < nel; ++e) {
+      at[e] = e;
+      int &f = lead[(size_t)r[e] * dim + c[e]];
+      if (f < 0) {
+        f = e;
+        ++entries;
+      }
+    }
+    if (!stored_entries(dim, nel, entries, (double)nkx * nky * nkz)) entries = 0;
+    auto entry = [&](int e) { return entries ? lead[(size_t)r[e] * dim + c[e]] : 0; };
+    std::stable_sort(at.begin(), at.end(), [&](int x, int y) {
+      return r[x] != r[y] ? r[x] < r[y] : entry(x) < entry(y);
+    });
+    // [elements | z | V0 | row | start | col], in doubles
     const size_t ne = std::max(nel, 1) * (sizeof(LatticeElement) / sizeof(double)), nz = 2 * (size_t)nw;
-    const size_t total = ne + nz + nV0 + (dim + 2) / 2 + 1;
+    const size_t total = ne + nz + nV0 + (dim + 2 * (size_t)entries + 3) / 2 + 1;
     if (total > kPinnedDoubles) own.resize(total);
     double *h = own.empty() ? W.pinned(total) : own.data();
     LatticeElement *he = reinterpret_cast<LatticeElement *>(h);
-    int *first = reinterpret_cast<int *>(h + ne + nz + nV0);
+    int *first = reinterpret_cast<int *>(h + ne + nz + nV0), *start = first + dim + 1, *col = start + entries + 1;
     std::fill(first, first + dim + 1, 0);
-    for (int e = 0; e < nel; ++e) ++first[r[e] + 1];
-    for (int a = 0; a < dim; ++a) first[a + 1] += first[a];
-    std::vector<int> next(first, first + dim);
-    for (int e = 0; e < nel; ++e) {
+    int group = 0;
+    for (int a = 0; a < nel; ++a) {
+      const int e = at[a];
+      const bool opens = entries && (a == 0 || entry(at[a - 1]) != entry(e));
+      if (opens) {
+        start[group] = a;
+        col[group++] = c[e];
+      }
+      if (opens || !entries) ++first[r[e] + 1];
       int q[3];
       double turn = 0.0;
       for (int i = 0; i < 3; ++i) {
@@ -267,15 +300,25 @@ struct LatticeInput {
       }
       std::complex<double> x(vv[2 * e], vv[2 * e + 1]);
       if (off != 0.0) x *= std::polar(1.0, 2.0 * M_PI * turn);
-      he[next[r[e]]++] = LatticeElement{{x.real(), x.imag()}, {c[e], q[0], q[1], q[2]}};
+      he[a] = LatticeElement{{x.real(), x.imag()}, {c[e], q[0], q[1], q[2]}};
     }
+    if (entries) start[entries] = nel;
+    for (int a = 0; a < dim; ++a) first[a + 1] += first[a];
     for (int i = 0; i < nw; ++i) z[i] = cplx(0.0, w[i]);
     std::memcpy(h + ne, z.data(), nz * sizeof(double));
     std::memcpy(h + ne + nz, hV0, nV0 * sizeof(double));
     buf.upload(h, total, W.stream);
     dz = buf.p + ne;
     V0 = dz + nz;
-    el = {reinterpret_cast<const int *>(V0 + nV0), reinterpret_cast<const LatticeElement *>(buf.p)};
+    const int *row = reinterpret_cast<const int *>(V0 + nV0);
+    el = {row, reinterpret_cast<const LatticeElement *>(buf.p)};
+    if (entries) {
+      vk.alloc(2 * (size_t)nkx * nky * nkz * entries);
+      el.entries = entries;
+      el.start = row + dim + 1;
+      el.col = el.start + entries + 1;
+      el.vk = vk.p;
+    }
   }
 };
 

@@ -216,9 +216,15 @@ struct alignas(16) LatticeElement {
   double2 v;
   int4 where;  // column, then R reduced to [0, nk) of each direction
 };
+// Stored form: the `entries` (r, c) that have elements, ordered by row, and their
+// values at every wavevector in vk (2 entries nk doubles, formed by the launch). Then
+// row counts entries, entry i has column col[i] and the elements start[i] .. start[i + 1].
 struct LatticeView {
   const int *row;
   const LatticeElement *el;
+  int entries = 0;  // 0: the elements of a row one by one
+  const int *start = nullptr, *col = nullptr;
+  double *vk = nullptr;
 };
 // CTAs per frequency, for the sizes of the partial sums below
 int lattice_blocks(int n, int nw, long nk);

@@ -10,7 +10,9 @@
 // it once in shared memory, and a lane only adds its own elements' rows,
 //   row r += sum_{e: r_e = r} v_e exp(2 pi i k.R_e) G[c_e, :],
 // N multiplications per element instead of the N^3 of the whole product (the
-// elements couple neighbouring super cells: two or three per boundary site). The 1 is
+// elements couple neighbouring super cells: two or three per boundary site). Many
+// elements in a row (long-range hops) are summed per entry of V(k) beforehand, once
+// for all frequencies (STORED; the rule and both sides stand at stored_entries). The 1 is
 // subtracted last, per wavevector: V0 G is small against it, and the rounding of
 // V0 G - 1, formed once, would be the same for all wavevectors and stay in their mean
 // (30 cases of dimension 2 to 12 against 80-bit values: 1.5e-15 so, 4.5e-16 now, 1.2e-15
@@ -54,8 +56,11 @@ constexpr int lattice_ctas(int n) { return n <= 6 ? 8 : (n <= 10 ? 6 : (n <= 13 
 constexpr int kPhaseTable = 384;
 
 struct LatticeTerms {
-  const int *row;               // elements of matrix row r: row[r] .. row[r + 1]
+  const int *row;               // elements (or stored entries) of matrix row r: row[r] .. row[r + 1]
   const LatticeElement *el;
+  const double2 *vk;            // stored entries of V(k), k slowest, entries' columns
+  const int *col;
+  int entries;
   int nk0, nk1, nk2;            // grid, the largest direction last
   unsigned magic0, magic1, magic2;  // ceil(2^32 / nk): j mod nk by a multiplication, for j < nk^2
   bool table;
@@ -124,6 +129,7 @@ template <int N> struct LatticeTile {
   }
 
   // row r of +-(V(k) G - 1) at grid point (i0, i1, i2); ph: the phase table, or unused
+  template <bool STORED>
   __device__ __forceinline__ void row(const LatticeTerms &t, const double2 *ph, const GridPoint &k, int e, int e1,
                                       int r, double sign, Cplx (&a)[N]) const {
 #pragma unroll
@@ -131,32 +137,47 @@ template <int N> struct LatticeTile {
       const double2 v = w[r * kLd + b];
       a[b] = {v.x, v.y};
     }
-    for (; e < e1; ++e) {
-      const double2 v = __ldg(&t.el[e].v);
-      const int4 m = __ldg(&t.el[e].where);  // column, R
-      Cplx p = {sign * v.x, sign * v.y};
-      if (t.table) {
-        auto turn = [&](unsigned j, int nk, unsigned magic, const double2 *tab) {
-          const double2 f = tab[j - (unsigned)nk * __umulhi(j, magic)];
-          p = cmul(p, Cplx{f.x, f.y});
-        };
-        if (t.nk0 > 1) turn(k.i0 * (unsigned)m.y, t.nk0, t.magic0, ph);
-        if (t.nk1 > 1) turn(k.i1 * (unsigned)m.z, t.nk1, t.magic1, ph + t.nk0);
-        turn(k.i2 * (unsigned)m.w, t.nk2, t.magic2, ph + t.nk0 + t.nk1);
-      } else {
-        auto part = [](unsigned i, int R, int nk) {
-          return (double)((unsigned long long)i * (unsigned)R % (unsigned)nk) / nk;
-        };
-        double s, c;
-        sincospi(2.0 * (part(k.i0, m.y, t.nk0) + part(k.i1, m.z, t.nk1) + part(k.i2, m.w, t.nk2)), &s, &c);
-        p = cmul(p, Cplx{c, s});
-      }
-      const double2 *gr = g + m.x * kLd;
-      p = {-p.x, -p.y};
+    if (STORED) {
+      const double2 *vk = t.vk + (((size_t)k.i0 * t.nk1 + k.i1) * t.nk2 + k.i2) * t.entries;
+#pragma unroll 2
+      for (; e < e1; ++e) {
+        const double2 v = __ldg(vk + e);
+        const double2 *gr = g + __ldg(t.col + e) * kLd;
+        const Cplx p = {-sign * v.x, -sign * v.y};
 #pragma unroll
-      for (int b = 0; b < N; ++b) {
-        const double2 y = gr[b];
-        csub(a[b], p, Cplx{y.x, y.y});
+        for (int b = 0; b < N; ++b) {
+          const double2 y = gr[b];
+          csub(a[b], p, Cplx{y.x, y.y});
+        }
+      }
+    } else {
+      for (; e < e1; ++e) {
+        const double2 v = __ldg(&t.el[e].v);
+        const int4 m = __ldg(&t.el[e].where);  // column, R
+        Cplx p = {sign * v.x, sign * v.y};
+        if (t.table) {
+          auto turn = [&](unsigned j, int nk, unsigned magic, const double2 *tab) {
+            const double2 f = tab[j - (unsigned)nk * __umulhi(j, magic)];
+            p = cmul(p, Cplx{f.x, f.y});
+          };
+          if (t.nk0 > 1) turn(k.i0 * (unsigned)m.y, t.nk0, t.magic0, ph);
+          if (t.nk1 > 1) turn(k.i1 * (unsigned)m.z, t.nk1, t.magic1, ph + t.nk0);
+          turn(k.i2 * (unsigned)m.w, t.nk2, t.magic2, ph + t.nk0 + t.nk1);
+        } else {
+          auto part = [](unsigned i, int R, int nk) {
+            return (double)((unsigned long long)i * (unsigned)R % (unsigned)nk) / nk;
+          };
+          double s, c;
+          sincospi(2.0 * (part(k.i0, m.y, t.nk0) + part(k.i1, m.z, t.nk1) + part(k.i2, m.w, t.nk2)), &s, &c);
+          p = cmul(p, Cplx{c, s});
+        }
+        const double2 *gr = g + m.x * kLd;
+        p = {-p.x, -p.y};
+#pragma unroll
+        for (int b = 0; b < N; ++b) {
+          const double2 y = gr[b];
+          csub(a[b], p, Cplx{y.x, y.y});
+        }
       }
     }
 #pragma unroll
@@ -164,6 +185,39 @@ template <int N> struct LatticeTile {
       if (b == r) a[b].x -= sign;
   }
 };
+
+// The entries of V(k) that have elements, for every wavevector: out[k * entries + i], by
+// L lanes each (a grid of few entries has too few threads otherwise, each with a chain
+// of sincospi: one entry of 64 elements on 256 wavevectors 100 us with one lane).
+template <int L>
+__global__ void __launch_bounds__(128) k_lattice_entries(LatticeTerms t, const int *__restrict__ start,
+                                                         unsigned long long n, double2 *out) {
+  const unsigned lane = threadIdx.x % L;
+  const unsigned long long all = (n + 128 / L - 1) / (128 / L) * (128 / L);  // whole CTAs, for the shuffles
+  for (unsigned long long q = blockIdx.x * (128ull / L) + threadIdx.x / L; q < all; q += gridDim.x * (128ull / L)) {
+    const unsigned long long kid = min(q, n - 1) / (unsigned)t.entries;
+    const int i = (int)(min(q, n - 1) - kid * (unsigned)t.entries);
+    const GridPoint k(t, kid);
+    auto part = [](unsigned j, int R, int nk) {
+      return (double)((unsigned long long)j * (unsigned)R % (unsigned)nk) / nk;
+    };
+    double sr = 0.0, si = 0.0;
+    for (int e = start[i] + lane; e < start[i + 1]; e += L) {
+      const double2 v = __ldg(&t.el[e].v);
+      const int4 m = __ldg(&t.el[e].where);
+      double s, c;
+      sincospi(2.0 * (part(k.i0, m.y, t.nk0) + part(k.i1, m.z, t.nk1) + part(k.i2, m.w, t.nk2)), &s, &c);
+      sr += v.x * c - v.y * s;
+      si += v.x * s + v.y * c;
+    }
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) {
+      sr += __shfl_xor_sync(0xffffffffu, sr, o);
+      si += __shfl_xor_sync(0xffffffffu, si, o);
+    }
+    if (lane == 0 && q < n) out[q] = make_double2(sr, si);
+  }
+}
 
 // The CTA's phase table (visible after the next barrier).
 __device__ __forceinline__ void fill_phases(const LatticeTerms &t, double2 *ph) {
@@ -201,7 +255,7 @@ template <int N> struct PivotRing {
 
 // Per frequency (blockIdx.y) and CTA: the sum over its wavevectors of
 // log |det(V(k) G - 1)|. per_warp: wavevector batches of one warp.
-template <int N>
+template <int N, bool STORED>
 __global__ void __launch_bounds__(kLatThreads, lattice_ctas(N)) k_sef_logdet(const double *__restrict__ G,
                                                             const double *__restrict__ V0, LatticeTerms terms,
                                                             unsigned long long nk, int per_warp, double *partials) {
@@ -210,7 +264,7 @@ __global__ void __launch_bounds__(kLatThreads, lattice_ctas(N)) k_sef_logdet(con
   __shared__ double2 ph[kPhaseTable];
   __shared__ double red[kLatWarps];
   const int iw = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  fill_phases(terms, ph);
+  if (!STORED) fill_phases(terms, ph);
   tile.load(G + 2 * (size_t)iw * N * N, V0, 1.0);
   const int grp = min(lane / N, GW - 1);  // lanes past the last whole matrix repeat it, without a say in the pivots
   const bool mine = lane < GW * N;
@@ -228,7 +282,7 @@ __global__ void __launch_bounds__(kLatThreads, lattice_ctas(N)) k_sef_logdet(con
     const bool valid = kid < nk;
     if (!__any_sync(0xffffffffu, valid)) break;
     Cplx a[N];
-    tile.row(terms, ph, k, e0, e1, r, 1.0, a);
+    tile.template row<STORED>(terms, ph, k, e0, e1, r, 1.0, a);
     bool open = true;
     Cplx piv = {1.0, 0.0};
 #pragma unroll
@@ -278,7 +332,7 @@ __global__ void __launch_bounds__(kLatThreads, lattice_ctas(N)) k_sef_logdet(con
 // left where they are, lane p_j ends with row j of the inverse, its column c
 // holding the inverse's column p_c; every matrix slot of the CTA adds into its
 // own N x N accumulator in shared memory, and the slots are added in order.
-template <int N>
+template <int N, bool STORED>
 __global__ void __launch_bounds__(kLatThreads, lattice_ctas(N)) k_cpt_partial(const double *__restrict__ G,
                                                              const double *__restrict__ V0, LatticeTerms terms,
                                                              unsigned long long nk, int per_warp, double *partials) {
@@ -287,7 +341,7 @@ __global__ void __launch_bounds__(kLatThreads, lattice_ctas(N)) k_cpt_partial(co
   __shared__ double2 ph[kPhaseTable];
   __shared__ double2 acc[kLatWarps * GW][N * N];
   const int iw = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  fill_phases(terms, ph);
+  if (!STORED) fill_phases(terms, ph);
   double2 *flat = &acc[0][0];
   for (int t = threadIdx.x; t < kLatWarps * GW * N * N; t += blockDim.x) flat[t] = make_double2(0.0, 0.0);
   tile.load(G + 2 * (size_t)iw * N * N, V0 + 2 * (size_t)iw * N * N, -1.0);
@@ -304,7 +358,7 @@ __global__ void __launch_bounds__(kLatThreads, lattice_ctas(N)) k_cpt_partial(co
     const bool valid = kid < nk;
     if (!__any_sync(0xffffffffu, valid)) break;
     Cplx a[N];
-    tile.row(terms, ph, k, e0, e1, r, -1.0, a);
+    tile.template row<STORED>(terms, ph, k, e0, e1, r, -1.0, a);
     int row = -1;                  // the inverse's row this lane ends with
     unsigned long long perm = 0;   // p_c in bits 4 c ..
 #pragma unroll
@@ -413,19 +467,34 @@ int batches_per_warp(int n, int nw, unsigned long long nk) {
 }
 
 using LatticeFn = void (*)(const double *, const double *, LatticeTerms, unsigned long long, int, double *);
-LatticeTerms lattice_terms(const LatticeView &el, int nk0, int nk1, int nk2) {
+// The terms of a sum, with the stored entries formed on s where the view has them.
+LatticeTerms lattice_terms(const LatticeView &el, const int (&nk)[3], cudaStream_t s) {
   auto magic = [](int nk) { return nk > 1 ? (unsigned)((0x100000000ull + nk - 1) / (unsigned)nk) : 0u; };
-  return {el.row, el.el, nk0, nk1, nk2, magic(nk0), magic(nk1), magic(nk2), (long)nk0 + nk1 + nk2 <= kPhaseTable};
+  const LatticeTerms t = {el.row, el.el, reinterpret_cast<const double2 *>(el.vk), el.col, el.entries, nk[0], nk[1],
+                          nk[2], magic(nk[0]), magic(nk[1]), magic(nk[2]), (long)nk[0] + nk[1] + nk[2] <= kPhaseTable};
+  if (el.entries) {
+    const unsigned long long n = (unsigned long long)nk[0] * nk[1] * nk[2] * (unsigned)el.entries;
+    const int lanes = n < 65536 ? 16 : 1;
+    const unsigned grid = (unsigned)std::min<unsigned long long>((n * lanes + 127) / 128, 148 * 32);
+    (lanes == 16 ? k_lattice_entries<16> : k_lattice_entries<1>)<<<grid, 128, 0, s>>>(
+        t, el.start, n, reinterpret_cast<double2 *>(el.vk));
+    QED_LAUNCH();
+  }
+  return t;
 }
 
-const LatticeFn kLogdet[kLatMaxN] = {k_sef_logdet<1>,  k_sef_logdet<2>,  k_sef_logdet<3>,  k_sef_logdet<4>,
-                                     k_sef_logdet<5>,  k_sef_logdet<6>,  k_sef_logdet<7>,  k_sef_logdet<8>,
-                                     k_sef_logdet<9>,  k_sef_logdet<10>, k_sef_logdet<11>, k_sef_logdet<12>,
-                                     k_sef_logdet<13>, k_sef_logdet<14>, k_sef_logdet<15>, k_sef_logdet<16>};
-const LatticeFn kCpt[kLatMaxN] = {k_cpt_partial<1>,  k_cpt_partial<2>,  k_cpt_partial<3>,  k_cpt_partial<4>,
-                                  k_cpt_partial<5>,  k_cpt_partial<6>,  k_cpt_partial<7>,  k_cpt_partial<8>,
-                                  k_cpt_partial<9>,  k_cpt_partial<10>, k_cpt_partial<11>, k_cpt_partial<12>,
-                                  k_cpt_partial<13>, k_cpt_partial<14>, k_cpt_partial<15>, k_cpt_partial<16>};
+template <bool STORED> struct LatticeFns {
+  static constexpr LatticeFn logdet[kLatMaxN] = {
+      k_sef_logdet<1, STORED>,  k_sef_logdet<2, STORED>,  k_sef_logdet<3, STORED>,  k_sef_logdet<4, STORED>,
+      k_sef_logdet<5, STORED>,  k_sef_logdet<6, STORED>,  k_sef_logdet<7, STORED>,  k_sef_logdet<8, STORED>,
+      k_sef_logdet<9, STORED>,  k_sef_logdet<10, STORED>, k_sef_logdet<11, STORED>, k_sef_logdet<12, STORED>,
+      k_sef_logdet<13, STORED>, k_sef_logdet<14, STORED>, k_sef_logdet<15, STORED>, k_sef_logdet<16, STORED>};
+  static constexpr LatticeFn cpt[kLatMaxN] = {
+      k_cpt_partial<1, STORED>,  k_cpt_partial<2, STORED>,  k_cpt_partial<3, STORED>,  k_cpt_partial<4, STORED>,
+      k_cpt_partial<5, STORED>,  k_cpt_partial<6, STORED>,  k_cpt_partial<7, STORED>,  k_cpt_partial<8, STORED>,
+      k_cpt_partial<9, STORED>,  k_cpt_partial<10, STORED>, k_cpt_partial<11, STORED>, k_cpt_partial<12, STORED>,
+      k_cpt_partial<13, STORED>, k_cpt_partial<14, STORED>, k_cpt_partial<15, STORED>, k_cpt_partial<16, STORED>};
+};
 
 }  // namespace
 
@@ -442,8 +511,8 @@ void launch_sef_logdet(int n, int nw, const double *G, const double *V0, const L
   const int nblk = lattice_blocks(n, nw, nk);
   if (nw <= 0 || nk <= 0) return;
   if (nw > 65535) fail(QED_ERR_ARGUMENT, "SEF grid integrand: more than 65535 frequencies");
-  const LatticeTerms t = lattice_terms(el, nk3[0], nk3[1], nk3[2]);
-  kLogdet[n - 1]<<<dim3(nblk, nw), kLatThreads, 0, s>>>(G, V0, t, (unsigned long long)nk,
+  const LatticeTerms t = lattice_terms(el, nk3, s);
+  (el.entries ? LatticeFns<true>::logdet : LatticeFns<false>::logdet)[n - 1]<<<dim3(nblk, nw), kLatThreads, 0, s>>>(G, V0, t, (unsigned long long)nk,
                                                          batches_per_warp(n, nw, nk), partials);
   QED_LAUNCH();
 }
@@ -452,11 +521,11 @@ void launch_cpt_projected(int n, int nw, const double *G, const double *V0, cons
   const long nk = (long)nk3[0] * nk3[1] * nk3[2];
   const int nblk = lattice_blocks(n, std::min(nw, 65535), nk);
   if (nw <= 0 || nk <= 0) return;
-  const LatticeTerms t = lattice_terms(el, nk3[0], nk3[1], nk3[2]);
+  const LatticeTerms t = lattice_terms(el, nk3, s);
   for (int w0 = 0; w0 < nw; w0 += 65535) {  // the grid's second dimension ends there
     const int m = std::min(nw - w0, 65535);
     const size_t o = 2 * (size_t)w0 * n * n;
-    kCpt[n - 1]<<<dim3(nblk, m), kLatThreads, 0, s>>>(G + o, V0 + o, t, (unsigned long long)nk,
+    (el.entries ? LatticeFns<true>::cpt : LatticeFns<false>::cpt)[n - 1]<<<dim3(nblk, m), kLatThreads, 0, s>>>(G + o, V0 + o, t, (unsigned long long)nk,
                                                        batches_per_warp(n, std::min(nw, 65535), nk),
                                                        partials + o * nblk);
     QED_LAUNCH();
