@@ -1486,32 +1486,36 @@ __global__ void __launch_bounds__(256) k_block_chol(int p, const double *G, doub
 // frequency. (Q_matrix::Green_function + VDVH kernel, src_ed/Q_matrix.hpp:133-151,
 // src_util/VDVH_kernel.cpp:28-36.) A thread owns one pair a <= b (G is symmetric)
 // and every `slices`-th pole, so that a small G still fills the CTA; the slices
-// are added in order. Poles are staged in shared memory, as many as fit
-// (kGfStage doubles), because each refill costs a round trip to L2. Bound by that
-// latency (the measured times stand at the launcher).
+// are added in order. Poles are staged in shared memory, `chunk` at a time, as many as
+// fit (kGfStage doubles), because each refill costs a round trip to L2. Bound by that
+// latency, and with many frequencies by the CTAs' own (sizes and times at the launcher).
 constexpr int kGfThreads = 512;
 constexpr int kGfStage = 5120;  // 40 KB
-__global__ void __launch_bounds__(kGfThreads) k_qmatrix_gf(int L, int M, const double *__restrict__ e,
-                                                           const double *__restrict__ V, const double *z, double *G) {
-  __shared__ double stage[kGfStage];
-  __shared__ double2 part[kGfThreads];
-  const int chunk = min(M, kGfStage / (L + 2));
-  double *vs = stage, *ur = stage + (size_t)chunk * L, *ui = ur + chunk;
+__global__ void __launch_bounds__(kGfThreads) k_qmatrix_gf(int L, int M, int slices, int chunk,
+                                                           const double *__restrict__ e, const double *__restrict__ V,
+                                                           const double *z, double *G) {
+  extern __shared__ __align__(16) double stage[];
+  double2 *tile = reinterpret_cast<double2 *>(stage);  // L x L
+  double2 *part = tile + L * L;                        // one per thread (slices > 1)
+  double *vs = reinterpret_cast<double *>(part + (slices > 1 ? blockDim.x : 0)), *ur = vs + (size_t)chunk * L,
+         *ui = ur + chunk;
   const int k = blockIdx.x, t = threadIdx.x;
   const double zr = z[2 * k], zi = z[2 * k + 1];
-  const int npair = L * (L + 1) / 2, slices = max(1, kGfThreads / npair);
-  for (int p0 = 0; p0 < npair; p0 += kGfThreads) {
+  const int npair = L * (L + 1) / 2, T = blockDim.x;
+  for (int p0 = 0; p0 < npair; p0 += T) {  // more than one round only without slices
     const int slice = t / npair, pidx = slices > 1 ? t % npair : p0 + t;
     const bool on = pidx < npair && (slices == 1 || slice < slices);
-    int b = 0;
-    while ((b + 1) * (b + 2) / 2 <= pidx) ++b;  // pairs (a, b), a <= b, column by column
+    // pairs (a, b), a <= b, column by column: b from the root, put right where it is off by one
+    int b = (int)(0.5f * (sqrtf(8.0f * pidx + 1.0f) - 1.0f));
+    if ((b + 1) * (b + 2) / 2 <= pidx) ++b;
+    if (b * (b + 1) / 2 > pidx) --b;
     const int a = pidx - b * (b + 1) / 2;
     double gr = 0.0, gi = 0.0;
     for (int i0 = 0; i0 < M; i0 += chunk) {
       const int nc = min(chunk, M - i0);
       __syncthreads();
-      for (int i = t; i < nc * L; i += kGfThreads) vs[i] = V[(size_t)i0 * L + i];
-      for (int i = t; i < nc; i += kGfThreads) {
+      for (int i = t; i < nc * L; i += T) vs[i] = V[(size_t)i0 * L + i];
+      for (int i = t; i < nc; i += T) {
         const double dr = zr - e[i0 + i], di = zi;
         const double den = dr * dr + di * di;
         ur[i] = dr / den;
@@ -1536,15 +1540,13 @@ __global__ void __launch_bounds__(kGfThreads) k_qmatrix_gf(int L, int M, const d
           gi += part[s * npair + t].y;
         }
     }
-    if (on && (slices == 1 || slice == 0)) {
-      double *g = G + 2 * (size_t)k * L * L;
-      g[2 * (b + a * L)] += gr;
-      g[2 * (b + a * L) + 1] += gi;
-      if (a != b) {
-        g[2 * (a + b * L)] += gr;
-        g[2 * (a + b * L) + 1] += gi;
-      }
-    }
+    if (on && (slices == 1 || slice == 0)) tile[b + a * L] = tile[a + b * L] = make_double2(gr, gi);
+  }
+  __syncthreads();
+  double2 *g = reinterpret_cast<double2 *>(G) + (size_t)k * L * L;
+  for (int i = t; i < L * L; i += T) {  // both triangles together: contiguous
+    const double2 x = g[i];
+    g[i] = make_double2(x.x + tile[i].x, x.y + tile[i].y);
   }
 }
 
@@ -2212,8 +2214,27 @@ void launch_qmatrix_gf(int L, int M, const double *e, const double *V, int nz, c
                        double *G, cudaStream_t s) {
   if (nz <= 0 || M <= 0) return;
   if (L > 64) fail(QED_ERR_UNSUPPORTED, "Green function dimension above 64");
-  // 64 frequencies, 480 poles, L = 10: 8.5 us (18 us with chunks of 64 poles and one thread per matrix entry)
-  k_qmatrix_gf<<<nz, kGfThreads, 0, s>>>(L, M, e, V, z, G);
+  // Slices of 16 poles or more, 64 at most (their sum is one thread's chain), and CTAs of
+  // as many threads as keep the SMs full: 64 frequencies, 480 poles, L = 10: 8.5 us (18
+  // with chunks of 64 poles and one thread per matrix entry). The smaller CTAs are for
+  // many frequencies, and the matrices are read and written row by row: 20,000, 50 poles,
+  // L = 1 32 us (62 with one thread per entry), L = 8 61 (77). With 512 threads and as
+  // many slices whatever the sizes, whole calls of L = 1 took 573 us; with one thread per
+  // entry 192, now 161.
+  const int npair = L * (L + 1) / 2;
+  const int most = nz <= 2 * device_sms() ? kGfThreads : (nz <= 8 * device_sms() || npair > 32 ? 256 : 128);
+  const int slices = std::max(1, std::min({most / npair, M / 16, 64}));
+  // few frequencies: threads beyond the pairs' still stage poles
+  const int threads = std::min(kGfThreads, std::max(nz <= 2 * device_sms() ? 256 : 64, (npair * slices + 31) / 32 * 32));
+  const int chunk = std::min(M, kGfStage / (L + 2));
+  const size_t smem = ((size_t)chunk * (L + 2) + 2 * L * L + (slices > 1 ? 2 * (size_t)threads : 0)) * sizeof(double);
+  static const bool attr = [] {
+    QED_CUDA(cudaFuncSetAttribute(k_qmatrix_gf, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (kGfStage + 2 * 64 * 64 + 2 * kGfThreads) * (int)sizeof(double)));
+    return true;
+  }();
+  (void)attr;
+  k_qmatrix_gf<<<nz, threads, smem, s>>>(L, M, slices, chunk, e, V, z, G);
   QED_LAUNCH();
 }
 
