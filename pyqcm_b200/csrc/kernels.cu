@@ -1243,7 +1243,10 @@ __device__ __forceinline__ double job_sum(double v, double *sm) {
 // each and one table entry after the other, now 4 to 5 ms (3.5 ms of it the 273 wide
 // sectors, which the narrow ones' launch overlaps). The limit kLanczosWideDim and T =
 // 1024 of the wide form: their whole eigenvalue phase takes 110 ms; with a limit of
-// 8192 139, of 4096 144, with T = 512 and a limit of 16384 120, of 4096 119.
+// 8192 139, of 4096 144, with T = 512 and a limit of 16384 120, of 4096 119. Few jobs
+// leave an SM to each, and the wide form gains from kLanczosWideDimFew on (whole ground
+// states, narrow and wide: 1225 states 2.21 and 2.06 ms, 4900 4.99 and 3.71, 15,876 of
+// the 3x3 cluster 25.9 and 14.4, where the former kernel took 23.3).
 template <int T>
 __global__ void __launch_bounds__(T) k_lanczos_jobs(const LanczosJob *__restrict__ jobs) {
   constexpr uint32_t C = kLanczosJobThreads;

@@ -167,7 +167,9 @@ size_t lanczos_job_max_dim();
 // (2 * kLanczosJobMaxSteps doubles per job).
 constexpr int kLanczosJobThreads = 256;
 constexpr int kLanczosWideThreads = 1024;
-constexpr size_t kLanczosWideDim = 16384;
+// with at most a job per SM the wide form is the faster one from here on
+constexpr size_t kLanczosWideDim = 16384, kLanczosWideDimFew = 1024;
+constexpr int kLanczosFewJobs = 148;
 constexpr int kLanczosJobMaxSteps = 16;
 struct LanczosJob {
   HvOperator op;
@@ -180,7 +182,8 @@ struct LanczosJob {
 // v_j = normalised random start vector (the values of launch_random for `seed`),
 // v_{j-1} = 0, beta_prev = 0, for every job
 void launch_lanczos_start_jobs(const LanczosJob *jobs, int njobs, cudaStream_t s);
-// the first nwide jobs (sectors of at least kLanczosWideDim states, the largest first)
+// the first nwide jobs (sectors of at least kLanczosWideDim states, or
+// kLanczosWideDimFew in a table of at most kLanczosFewJobs; the largest first)
 // by kLanczosWideThreads threads each
 void launch_lanczos_jobs(const LanczosJob *jobs, int njobs, int nwide, cudaStream_t s);
 

@@ -648,7 +648,7 @@ void lanczos_energy_batch(std::vector<LanczosBatchItem> &items, Workspace &ws) {
       batch[a].out = out.p + (size_t)a * 2 * kChunk;
       run[i].rot = (run[i].rot + run[i].chunk) % 3;
       run[i].chunk = kChunk;
-      if (items[i].H->D >= kLanczosWideDim) ++wide;
+      if (items[i].H->D >= (na <= kLanczosFewJobs ? kLanczosWideDimFew : kLanczosWideDim)) ++wide;
     }
     djobs.upload(batch.data(), na, s);
     launch_lanczos_jobs(djobs.p, na, wide, s);
