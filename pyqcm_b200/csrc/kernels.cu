@@ -2217,16 +2217,16 @@ void launch_qmatrix_gf(int L, int M, const double *e, const double *V, int nz, c
                        double *G, cudaStream_t s) {
   if (nz <= 0 || M <= 0) return;
   if (L > 64) fail(QED_ERR_UNSUPPORTED, "Green function dimension above 64");
-  // Slices of 16 poles or more, 64 at most (their sum is one thread's chain), and CTAs of
-  // as many threads as keep the SMs full: 64 frequencies, 480 poles, L = 10: 8.5 us (18
-  // with chunks of 64 poles and one thread per matrix entry). The smaller CTAs are for
-  // many frequencies, and the matrices are read and written row by row: 20,000, 50 poles,
-  // L = 1 32 us (62 with one thread per entry), L = 8 61 (77). With 512 threads and as
-  // many slices whatever the sizes, whole calls of L = 1 took 573 us; with one thread per
-  // entry 192, now 161.
+  // Slices of 16 poles or more (64 where the pairs alone fill two warps), 64 at most: their
+  // sum is one thread's chain. They depend on the matrix only, so that G at a frequency is
+  // the same bits in any call. 64 frequencies, 480 poles, L = 10: 8.5 us (18 with chunks of
+  // 64 poles and one thread per matrix entry). CTAs have the threads that they use, and the
+  // matrices are read and written row by row, for calls of many frequencies: 20,000, 50
+  // poles, L = 1 32 us (62 with one thread per entry), L = 8 61 (77). With 512 threads and
+  // as many slices whatever the sizes, whole calls of L = 1 took 573 us; with one thread
+  // per entry 192, now 161.
   const int npair = L * (L + 1) / 2;
-  const int most = nz <= 2 * device_sms() ? kGfThreads : (nz <= 8 * device_sms() || npair > 32 ? 256 : 128);
-  const int slices = std::max(1, std::min({most / npair, M / 16, 64}));
+  const int slices = std::max(1, std::min({kGfThreads / npair, M / (npair < 64 ? 16 : 64), 64}));
   // few frequencies: threads beyond the pairs' still stage poles
   const int threads = std::min(kGfThreads, std::max(nz <= 2 * device_sms() ? 256 : 64, (npair * slices + 31) / 32 * 32));
   const int chunk = std::min(M, kGfStage / (L + 2));

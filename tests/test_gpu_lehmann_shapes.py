@@ -33,3 +33,13 @@ def test_green_function_of_poles_over_shapes(qed, fresh, n, M, nz):
     got = qed.Green_function(z, label=label)
     ref = 2 * np.einsum("am,zm,bm->zab", v, 1.0 / (z[:, None] - e[None, :]), v, optimize=True)
     assert np.max(np.abs(got - ref)) < 1e-11 * max(1.0, np.max(np.abs(ref)))
+
+
+@pytest.mark.parametrize("n,M", [(1, 40), (4, 360), (10, 480), (16, 130)])
+def test_a_frequency_is_the_same_in_any_call(qed, fresh, n, M):
+    from tests.test_gpu_lattice_sums import _loaded_instance
+    label, _ = _loaded_instance(qed, fresh, n, np.random.default_rng(n), M=M)
+    z = 1j * np.linspace(0.1, 30.0, 3000)
+    G = qed.Green_function(z, label=label)
+    for m in (1, 70, 500):
+        assert np.array_equal(qed.Green_function(z[:m], label=label), G[:m]), m
