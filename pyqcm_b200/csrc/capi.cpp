@@ -270,6 +270,14 @@ struct LatticeInput {
       }
     }
     if (!stored_entries(dim, nel, entries, (double)nkx * nky * nkz)) entries = 0;
+    if (entries) {
+      try {
+        vk.alloc(2 * (size_t)nkx * nky * nkz * entries);
+      } catch (const Error &) {  // no memory for it: the elements one by one
+        cudaGetLastError();
+        entries = 0;
+      }
+    }
     auto entry = [&](int e) { return entries ? lead[(size_t)r[e] * dim + c[e]] : 0; };
     std::stable_sort(at.begin(), at.end(), [&](int x, int y) {
       return r[x] != r[y] ? r[x] < r[y] : entry(x) < entry(y);
@@ -313,7 +321,6 @@ struct LatticeInput {
     const int *row = reinterpret_cast<const int *>(V0 + nV0);
     el = {row, reinterpret_cast<const LatticeElement *>(buf.p)};
     if (entries) {
-      vk.alloc(2 * (size_t)nkx * nky * nkz * entries);
       el.entries = entries;
       el.start = row + dim + 1;
       el.col = el.start + entries + 1;
