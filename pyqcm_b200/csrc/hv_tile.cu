@@ -268,14 +268,17 @@ double tile_unevenness(uint32_t n, uint32_t m) {
 // unevenness 1.78 0.94x, 1.61 1.01x). For odd ones, whose columns are read and written 8
 // bytes at a time, an unevenness of 1.3 (1.18 gains up to 1.4x, 1.34 0.95x), and vectors
 // that leave L2 (3003 x 2002 states 1.15x, 3003 x 3432 0.88x).
-bool tile_applies(const HvOperator &op) {
+bool tile_sizes(uint32_t du, uint32_t dd) {
   constexpr uint64_t kTileAlwaysStates = 1700000, kTileOddStates = 8000000;
-  const uint32_t du = op.up.dim, dd = op.dn.dim;
   const uint64_t D = (uint64_t)du * dd;
-  if (!op.up.tile_max || !op.dn.tile_max || D < kTileMinStates) return false;
+  if (std::min(du, dd) < kTileMinDim || std::max(du, dd) > kTileMaxDim || D < kTileMinStates) return false;
   if (D < kTileAlwaysStates) return true;
   const double uneven = 0.5 * (tile_unevenness(du, dd) + tile_unevenness(dd, du));
   return du % 2 == 0 ? uneven < 1.7 : uneven < 1.25 && D < kTileOddStates;
+}
+
+bool tile_applies(const HvOperator &op) {
+  return op.up.tile_max && op.dn.tile_max && tile_sizes(op.up.dim, op.dn.dim);
 }
 
 int tile_grid(const HvOperator &op) { return (int)plan_tiles(op.up.dim, op.dn.dim).grid; }

@@ -280,8 +280,9 @@ int launch_hv_fused(const HvOperator &op, const double *x, double xs, double *y,
                     Reducer &r, cudaStream_t s);
 // The tiled two-pass form (hv_tile.cu) of half bases that fit shared memory eight
 // vectors wide. From kTileMinStates on (213444 states: 10.5 us, the one-launch form
-// 10.3-14), where tile_applies finds its tiles to fill the SMs.
+// 10.3-14), where its tiles fill the SMs (tile_sizes: half bases of an up and a down spin).
 constexpr uint64_t kTileMinStates = 180000;
+bool tile_sizes(uint32_t du, uint32_t dd);
 bool tile_applies(const HvOperator &op);
 int tile_grid(const HvOperator &op);
 int launch_hv_tile(const HvOperator &op, const double *x, double xs, double *y, const SubList &sub, int red_mask,

@@ -381,12 +381,15 @@ SectorOp::SectorOp(const SpinData &t, const Sector &s, Workspace &ws, HalfCache 
     fail(QED_ERR_UNSUPPORTED, "sector " + s.name() + " does not conserve N and S");
   if ((s.N + s.S) % 2) fail(QED_ERR_ARGUMENT, "sector " + s.name() + " is not valid");
   if (L > 32) fail(QED_ERR_UNSUPPORTED, "more than 32 orbitals per spin");
+  auto strings = [&](int N) -> uint32_t { return N < 0 || N > L ? 0 : (uint32_t)std::min<uint64_t>(binom(L, N), 1u << 24); };
+  const bool tiles = !cache && tile_sizes(strings(s.Nup()), strings(s.Ndw()));
   auto table = [&](int spin, int N) -> std::shared_ptr<const HalfTables> {
     auto make = [&] {
       auto h = std::make_shared<HalfTables>();
-      // tables shared by an instance's sectors serve the recurrences, which keep the
-      // two-pass and staged kernels (HvOperator::keep_order): no grouped copy
-      build_half(*h, L, N, spin ? t.t_dn : t.t_up, spin ? t.v_dd : t.v_uu, ws, spin == 0, !cache);
+      // no grouped copy where the tiled kernels do not run: in sectors of other sizes, and
+      // in tables that an instance's sectors share for the recurrences, which keep the
+      // two-pass and staged kernels (HvOperator::keep_order)
+      build_half(*h, L, N, spin ? t.t_dn : t.t_up, spin ? t.v_dd : t.v_uu, ws, spin == 0, tiles);
       return std::shared_ptr<const HalfTables>(h);
     };
     if (!cache) return make();
